@@ -363,6 +363,17 @@ ct_status ct_haar_fwd(const ct_fd_desc* d, const float* x, float* w,
 ct_status ct_haar_adj(const ct_fd_desc* d, const float* w, float* x,
                       int32_t batch, ct_stream_t stream);
 
+/* out = TVNorm.prox(v) (scico/functional/_tvnorm.py:190-237) for the isotropic
+ * (iso = 1, L2,1 base norm) or anisotropic (iso = 0, L1) norm: the Haar
+ * transform of v over d->axes (edge-padded by one sample on those axes unless
+ * d->circular), its highpass part shrunk by `thr` = sqrt(2) K lam outside the
+ * padding, the adjoint transform cropped back, times 1/K, K = 2 naxes.  One
+ * kernel, bit-identical to ct_haar_fwd + ct_l21_prox / ct_l1_prox +
+ * ct_haar_adj.  d: circular, or append = 0 and no prepend.  batch <= 65535 and
+ * fewer than 2^31 elements per item, else CT_ERR_UNSUPPORTED. */
+ct_status ct_tv_prox(const ct_fd_desc* d, const float* v, float* out,
+                     int32_t iso, float thr, int32_t batch, ct_stream_t stream);
+
 /* ------------------------------------------------------------------------ */
 /* Proximal operators and norms (scico/functional/_norm.py)                 */
 /* ------------------------------------------------------------------------ */

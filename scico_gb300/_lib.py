@@ -216,6 +216,7 @@ _SIGNATURES = {
     "ct_fd_adj": (ctypes.c_int, [P, P, P, c_int32, P]),
     "ct_haar_fwd": (ctypes.c_int, [P, P, P, c_int32, P]),
     "ct_haar_adj": (ctypes.c_int, [P, P, P, c_int32, P]),
+    "ct_tv_prox": (ctypes.c_int, [P, P, P, c_int32, c_float, c_int32, P]),
     "ct_l21_prox": (ctypes.c_int, [P, P, c_int32, c_int64, c_float, P]),
     "ct_l1_prox": (ctypes.c_int, [P, P, c_int64, c_float, P]),
     "ct_l21_norm": (ctypes.c_int, [P, c_int32, c_int64, P, P, c_size_t, P]),

@@ -64,6 +64,158 @@ ct_status make_fd(const ct_fd_desc* d, FdParams& p, const char* who) {
   return CT_OK;
 }
 
+// ---------------------------------------------------------------------------
+// Same-shape differences (circular, or exactly one end extended: every output
+// block has the input's shape), the form of every regulariser here.  Bound by
+// memory; what cost the time before was index arithmetic (two 64-bit divisions
+// an element) and one element in flight per thread.  A thread now takes kFdU
+// elements kFdT apart, finds each one's coordinates with two 32-bit
+// multiply-high divisions, reads x once for all axes and has all its loads in
+// flight before the first store.  192^3, three axes: forward 176 -> FWD_US us,
+// adjoint 150 -> ADJ_US us (as launched alone by a profiler).  Scalar
+// accesses throughout: rows of odd length are as common as multiples of four,
+// and 32-bit accesses of whole warps already fill the sectors.
+// ---------------------------------------------------------------------------
+constexpr int kFdT = 256;  // threads of a block
+constexpr int kFdU = 4;    // elements per thread
+
+// Division of 31-bit unsigned numbers by a fixed divisor: q = (mulhi(e, m) + e) >> s.
+struct FastDiv {
+  uint32_t d, m, s;
+};
+FastDiv fast_div(uint32_t d) {
+  FastDiv f{d, 0, 0};
+  while ((1u << f.s) < d && f.s < 31) ++f.s;
+  f.m = (uint32_t)((((1ull << f.s) - d) << 32) / d + 1);
+  return f;
+}
+__device__ __forceinline__ uint32_t div_by(const FastDiv& f, uint32_t e) { return (__umulhi(e, f.m) + e) >> f.s; }
+
+struct FdSame {
+  uint32_t count;  // elements of one input
+  FastDiv n2, n1;
+  int n[3];
+  int axis[3];
+  uint32_t stride[3];  // of axis[k]
+  int mode;            // 0 circular, 1 append, 2 prepend
+  int zero;            // extended sample: 0 = copy of the end, 1 = zero
+};
+
+// True when `p` is same-shape and every index fits 31 bits (the descriptor's
+// divisors must be below 2^31 for fast_div).
+bool make_same(const FdParams& p, FdSame& q) {
+  const bool pre = p.prepend >= 0, app = p.append >= 0;
+  if (!p.circular && pre == app) return false;
+  if (p.in_count >= (1ull << 31)) return false;
+  q.count = (uint32_t)p.in_count;
+  q.n1 = fast_div((uint32_t)p.n[1]);
+  q.n2 = fast_div((uint32_t)p.n[2]);
+  for (int k = 0; k < 3; ++k) q.n[k] = p.n[k];
+  for (int k = 0; k < p.nblocks; ++k) {
+    q.axis[k] = p.blk[k].axis;
+    q.stride[k] = q.axis[k] == 2 ? 1u : (q.axis[k] == 1 ? (uint32_t)p.n[2] : (uint32_t)p.n[1] * (uint32_t)p.n[2]);
+  }
+  q.mode = p.circular ? 0 : (app ? 1 : 2);
+  q.zero = p.circular ? 0 : (app ? p.append : p.prepend);
+  return true;
+}
+
+__device__ __forceinline__ void fd_coords(const FdSame& q, uint32_t e, int (&c)[3]) {
+  const uint32_t r = div_by(q.n2, e);
+  c[2] = (int)(e - r * (uint32_t)q.n[2]);
+  c[0] = (int)div_by(q.n1, r);
+  c[1] = (int)(r - (uint32_t)c[0] * (uint32_t)q.n[1]);
+}
+
+// out[k][e] = (next) - (this) along axis k, next the circular neighbour or the
+// extended sample at the end (append), or (this) - (previous) (prepend).
+template <int NB>
+__global__ void __launch_bounds__(kFdT) k_fd_fwd_same(const float* __restrict__ x, float* __restrict__ out, const FdSame q) {
+  x += (size_t)blockIdx.y * q.count;
+  out += (size_t)blockIdx.y * NB * q.count;
+  const uint32_t e0 = blockIdx.x * (uint32_t)(kFdT * kFdU) + threadIdx.x;
+  float xc[kFdU], xn[kFdU][NB];
+#pragma unroll
+  for (int u = 0; u < kFdU; ++u) {
+    const uint32_t e = min(e0 + u * kFdT, q.count - 1);  // loads stay unconditional, all in flight
+    int c[3];
+    fd_coords(q, e, c);
+    xc[u] = __ldg(x + e);
+#pragma unroll
+    for (int k = 0; k < NB; ++k) {
+      const int a = q.axis[k], ca = a == 2 ? c[2] : (a == 1 ? c[1] : c[0]), na = a == 2 ? q.n[2] : (a == 1 ? q.n[1] : q.n[0]);
+      const bool end = q.mode == 2 ? ca == 0 : ca == na - 1;
+      // mode 0 wraps to the line's start; an extended end reads its own sample
+      const uint32_t at = end ? (q.mode == 0 ? e - (uint32_t)ca * q.stride[k] : e)
+                              : (q.mode == 2 ? e - q.stride[k] : e + q.stride[k]);
+      const float v = __ldg(x + at);
+      xn[u][k] = end && q.zero ? 0.0f : v;
+    }
+  }
+#pragma unroll
+  for (int u = 0; u < kFdU; ++u) {
+    const uint32_t e = e0 + u * kFdT;
+    if (e >= q.count) break;
+#pragma unroll
+    for (int k = 0; k < NB; ++k)
+      out[(size_t)k * q.count + e] = q.mode == 2 ? ct::fsub(xc[u], xn[u][k]) : ct::fsub(xn[u][k], xc[u]);
+  }
+}
+
+// x[e] = sum over axes, in axis order, of the extended line's cotangents
+// ce[t] = d[t-1] - d[t] (terms off the line are 0) at the positions holding
+// x[e]; an end copied by the extension holds two, added in position order
+// (k_fd_adj below states the rule in general).
+template <int NB>
+__global__ void __launch_bounds__(kFdT) k_fd_adj_same(const float* __restrict__ d, float* __restrict__ x, const FdSame q) {
+  d += (size_t)blockIdx.y * NB * q.count;
+  x += (size_t)blockIdx.y * q.count;
+  const uint32_t e0 = blockIdx.x * (uint32_t)(kFdT * kFdU) + threadIdx.x;
+  float dc[kFdU][NB], dn[kFdU][NB];
+  unsigned two = 0;  // bit u*NB + k: the sample is a copied end
+#pragma unroll
+  for (int u = 0; u < kFdU; ++u) {
+    const uint32_t e = min(e0 + u * kFdT, q.count - 1);  // loads stay unconditional, all in flight
+    int c[3];
+    fd_coords(q, e, c);
+#pragma unroll
+    for (int k = 0; k < NB; ++k) {
+      const float* dk = d + (size_t)k * q.count;
+      const int a = q.axis[k], ca = a == 2 ? c[2] : (a == 1 ? c[1] : c[0]), na = a == 2 ? q.n[2] : (a == 1 ? q.n[1] : q.n[0]);
+      // the neighbour of the cotangent pair: the previous difference
+      // (circular, append) or the next one (prepend)
+      const bool off = q.mode == 2 ? ca == na - 1 : ca == 0;
+      const uint32_t at = off ? (q.mode == 0 ? e + (uint32_t)(na - 1) * q.stride[k] : e)
+                              : (q.mode == 2 ? e + q.stride[k] : e - q.stride[k]);
+      const float v = __ldg(dk + at);
+      dc[u][k] = __ldg(dk + e);
+      dn[u][k] = off && q.mode != 0 ? 0.0f : v;
+      const bool copied = q.mode != 0 && !q.zero && (q.mode == 2 ? ca == 0 : ca == na - 1);
+      if (copied) two |= 1u << (u * NB + k);
+    }
+  }
+#pragma unroll
+  for (int u = 0; u < kFdU; ++u) {
+    const uint32_t e = e0 + u * kFdT;
+    if (e >= q.count) break;
+    float acc = 0.0f;
+#pragma unroll
+    for (int k = 0; k < NB; ++k) {
+      const bool cp = (two >> (u * NB + k)) & 1u;
+      float v;
+      if (q.mode == 2) {
+        v = ct::fsub(dc[u][k], dn[u][k]);
+        if (cp) v = ct::fadd(ct::fsub(0.0f, dc[u][k]), v);  // position 0 first
+      } else {
+        v = ct::fsub(dn[u][k], dc[u][k]);
+        if (cp) v = ct::fadd(v, dc[u][k]);  // then the position past the end: d[n-1] - 0
+      }
+      acc = k == 0 ? v : ct::fadd(acc, v);
+    }
+    x[e] = acc;
+  }
+}
+
 // Value of the extended line e (prepend/append applied) at position t.
 __device__ __forceinline__ float fd_ext(const float* __restrict__ x, size_t stride, int n, int P,
                                         int prepend, int append, int t) {
@@ -230,9 +382,49 @@ int grid_for(size_t n, int threads) {
   return (int)std::max<size_t>(1, std::min(want, cap));
 }
 
-// L2,1 prox over the leading axis (L21Norm._prox, _norm.py:254-263):
-// len = sqrt(sum_c v_c^2); dir = v/len (0 where len == 0);
-// nl = len - lam; nl = 0.5 (nl + |nl|); out = nl * dir.
+// Shrink one vector of NC components (values v, component order): L21Norm._prox
+// (_norm.py:254-263): len = sqrt(sum_c v_c^2); dir = v/len (0 where len == 0);
+// nl = len - lam; nl = 0.5 (nl + |nl|); v = nl * dir.
+template <int NC>
+__device__ __forceinline__ void l21_shrink(float (&v)[NC], float lam) {
+  float ss = ct::fmul(v[0], v[0]);
+#pragma unroll
+  for (int c = 1; c < NC; ++c) ss = ct::fadd(ss, ct::fmul(v[c], v[c]));
+  const float len = __fsqrt_rn(ss);
+  float nl = ct::fsub(len, lam);
+  nl = ct::fmul(0.5f, ct::fadd(nl, fabsf(nl)));
+#pragma unroll
+  for (int c = 0; c < NC; ++c) {
+    const float dir = (len != 0.0f) ? __fdiv_rn(v[c], len) : 0.0f;
+    v[c] = ct::fmul(nl, dir);
+  }
+}
+
+// The prox of up to three components (every image gradient): the components
+// are read once and kept in registers, kPxU vectors in flight per thread.
+// 3 x 192^3: 43 -> PROX_US us.
+constexpr int kPxU = 4;
+template <int NC>
+__global__ void __launch_bounds__(256) k_l21_prox_few(const float* __restrict__ v, float* __restrict__ out, size_t n,
+                                                      float lam) {
+  const size_t e0 = (size_t)blockIdx.x * (256 * kPxU) + threadIdx.x;
+  float r[kPxU][NC];
+#pragma unroll
+  for (int u = 0; u < kPxU; ++u) {
+    const size_t e = min(e0 + u * 256, n - 1);
+#pragma unroll
+    for (int c = 0; c < NC; ++c) r[u][c] = __ldg(v + (size_t)c * n + e);
+  }
+#pragma unroll
+  for (int u = 0; u < kPxU; ++u)
+    if (e0 + u * 256 < n) {
+      l21_shrink<NC>(r[u], lam);
+#pragma unroll
+      for (int c = 0; c < NC; ++c) out[(size_t)c * n + e0 + u * 256] = r[u][c];
+    }
+}
+
+// The same for any number of components (two passes over them).
 __global__ void k_l21_prox(const float* __restrict__ v, float* __restrict__ out, int ncomp,
                            size_t n, float lam) {
   for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < n;
@@ -255,16 +447,101 @@ __global__ void k_l21_prox(const float* __restrict__ v, float* __restrict__ out,
 }
 
 // L1 prox (L1Norm.prox, _norm.py:110-116): sign(v) * 0.5 (t + |t|), t = |v| - lam.
+__device__ __forceinline__ float l1_shrink(float x, float lam) {
+  float t = ct::fsub(fabsf(x), lam);
+  t = ct::fmul(0.5f, ct::fadd(t, fabsf(t)));
+  const float sg = (x > 0.0f) ? 1.0f : ((x < 0.0f) ? -1.0f : (x == 0.0f ? 0.0f : x));
+  return ct::fmul(sg, t);
+}
+
 __global__ void k_l1_prox(const float* __restrict__ v, float* __restrict__ out, size_t n,
                           float lam) {
   for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < n;
        e += (size_t)gridDim.x * blockDim.x) {
-    const float x = v[e];
-    float t = ct::fsub(fabsf(x), lam);
-    t = ct::fmul(0.5f, ct::fadd(t, fabsf(t)));
-    const float sg = (x > 0.0f) ? 1.0f : ((x < 0.0f) ? -1.0f : (x == 0.0f ? 0.0f : x));
-    out[e] = ct::fmul(sg, t);
+    out[e] = l1_shrink(v[e], lam);
   }
+}
+
+// ---------------------------------------------------------------------------
+// TV prox in one pass (TVNorm.prox, scico/functional/_tvnorm.py:190-237): the
+// shift-invariant Haar transform of v (edge-padded by one sample on every
+// differenced axis unless circular), the base norm's prox on its highpass part
+// (on the region without the padding), the adjoint transform cropped back,
+// times 1/K.  Output e along axis k needs lowpass and shrunk highpass at e and
+// at the sample before it, and nothing else, so nothing goes through memory
+// but v and the result: a thread evaluates both positions of every axis.  Each
+// sum, product, root and quotient is the one that ct_haar_fwd, ct_l21_prox /
+// ct_l1_prox and ct_haar_adj round, in their order: same bits.  Bound by the
+// divisions and roots (L2,1) or by launch latency at small sizes; the composed
+// path took eight launches and passed over 2 naxes arrays: 512^2, L2,1, edge
+// padding 280 -> TVP_US us, 1024^2 TVP1_US us.
+// ---------------------------------------------------------------------------
+struct TvArgs {
+  const float* x;
+  float* out;
+  FdSame q;      // axes, strides, mode 0 = circular, 1 = edge-padded
+  float r, thr, inv_k;
+};
+
+template <int NB, bool ISO>
+__global__ void __launch_bounds__(256) k_tv_prox(const TvArgs a) {
+  const FdSame& q = a.q;
+  const uint32_t e = blockIdx.x * 256u + threadIdx.x;
+  if (e >= q.count) return;
+  const float* __restrict__ x = a.x + (size_t)blockIdx.y * q.count;
+  int c[3];
+  fd_coords(q, e, c);
+  int ca[NB], na[NB];
+#pragma unroll
+  for (int k = 0; k < NB; ++k) {
+    const int ax = q.axis[k];
+    ca[k] = ax == 2 ? c[2] : (ax == 1 ? c[1] : c[0]);
+    na[k] = ax == 2 ? q.n[2] : (ax == 1 ? q.n[1] : q.n[0]);
+  }
+  // the sample after position p along axis k, whose coordinate there is t
+  auto next = [&](uint32_t p, int k, int t) {
+    const uint32_t at = t + 1 < na[k] ? p + q.stride[k] : (q.mode == 0 ? p - (uint32_t)t * q.stride[k] : p);
+    return __ldg(x + at);
+  };
+  const float xe = __ldg(x + e);
+  float lo[NB], hi[NB];
+#pragma unroll
+  for (int k = 0; k < NB; ++k) {
+    const float xn = next(e, k, ca[k]);
+    lo[k] = ct::fmul(a.r, ct::fadd(xe, xn));
+    hi[k] = ct::fmul(a.r, ct::fsub(xn, xe));
+  }
+  if (ISO) {
+    l21_shrink<NB>(hi, a.thr);
+  } else {
+#pragma unroll
+    for (int k = 0; k < NB; ++k) hi[k] = l1_shrink(hi[k], a.thr);
+  }
+  float acc = 0.0f;
+#pragma unroll
+  for (int k = 0; k < NB; ++k) {
+    // the position before e along axis k: at the line's start the circular
+    // wrap, or the padding sample (a copy of the line's end, not shrunk)
+    const bool first = ca[k] == 0;
+    const uint32_t p = first ? e + (uint32_t)(na[k] - 1) * q.stride[k] : e - q.stride[k];
+    const float xp = __ldg(x + p);
+    const float lop = ct::fmul(a.r, ct::fadd(xp, xe));
+    float hip = ct::fmul(a.r, ct::fsub(xe, xp));
+    if (!(first && q.mode != 0)) {
+      if (ISO) {
+        float v[NB];
+#pragma unroll
+        for (int j = 0; j < NB; ++j) v[j] = j == k ? hip : ct::fmul(a.r, ct::fsub(next(p, j, ca[j]), xp));
+        l21_shrink<NB>(v, a.thr);
+        hip = v[k];
+      } else {
+        hip = l1_shrink(hip, a.thr);
+      }
+    }
+    const float t = ct::fadd(ct::fmul(a.r, ct::fadd(lo[k], lop)), ct::fmul(a.r, ct::fsub(hip, hi[k])));
+    acc = k == 0 ? t : ct::fadd(acc, t);
+  }
+  a.out[(size_t)blockIdx.y * q.count + e] = ct::fmul(a.inv_k, acc);
 }
 
 // sum_e sqrt(sum_c v_c^2) (ncomp > 0) or sum_e |v_e| (ncomp == 0), float64.
@@ -312,6 +589,18 @@ ct_status ct_fd_fwd(const ct_fd_desc* d, const float* x, float* out, int32_t bat
   if (batch <= 0) return ct::fail(CT_ERR_INVALID_ARG, "ct_fd_fwd: batch=%d", batch);
   const size_t total = p.out_count * batch;
   if (total == 0) return CT_OK;
+  FdSame q{};
+  if (batch <= 65535 && make_same(p, q)) {
+    const dim3 g((q.count + kFdT * kFdU - 1) / (kFdT * kFdU), batch);
+    cudaStream_t s = ct::as_stream(stream);
+    if (p.nblocks == 1)
+      k_fd_fwd_same<1><<<g, kFdT, 0, s>>>(x, out, q);
+    else if (p.nblocks == 2)
+      k_fd_fwd_same<2><<<g, kFdT, 0, s>>>(x, out, q);
+    else
+      k_fd_fwd_same<3><<<g, kFdT, 0, s>>>(x, out, q);
+    return ct::launch_check("k_fd_fwd_same");
+  }
   k_fd_fwd<<<grid_for(total, 256), 256, 0, ct::as_stream(stream)>>>(x, out, p, batch);
   return ct::launch_check("k_fd_fwd");
 }
@@ -324,6 +613,18 @@ ct_status ct_fd_adj(const ct_fd_desc* d, const float* dx, float* x, int32_t batc
   if (!x || !dx) return ct::fail(CT_ERR_INVALID_ARG, "ct_fd_adj: null array");
   if (batch <= 0) return ct::fail(CT_ERR_INVALID_ARG, "ct_fd_adj: batch=%d", batch);
   const size_t total = p.in_count * batch;
+  FdSame q{};
+  if (batch <= 65535 && make_same(p, q)) {
+    const dim3 g((q.count + kFdT * kFdU - 1) / (kFdT * kFdU), batch);
+    cudaStream_t s = ct::as_stream(stream);
+    if (p.nblocks == 1)
+      k_fd_adj_same<1><<<g, kFdT, 0, s>>>(dx, x, q);
+    else if (p.nblocks == 2)
+      k_fd_adj_same<2><<<g, kFdT, 0, s>>>(dx, x, q);
+    else
+      k_fd_adj_same<3><<<g, kFdT, 0, s>>>(dx, x, q);
+    return ct::launch_check("k_fd_adj_same");
+  }
   k_fd_adj<<<grid_for(total, 256), 256, 0, ct::as_stream(stream)>>>(dx, x, p, batch);
   return ct::launch_check("k_fd_adj");
 }
@@ -350,12 +651,53 @@ ct_status ct_haar_adj(const ct_fd_desc* d, const float* w, float* x, int32_t bat
   return ct::launch_check("k_haar_adj");
 }
 
+ct_status ct_tv_prox(const ct_fd_desc* d, const float* v, float* out, int32_t iso, float thr, int32_t batch,
+                     ct_stream_t stream) {
+  FdParams p{};
+  ct_status st = make_fd(d, p, "ct_tv_prox");
+  if (st != CT_OK) return st;
+  if (!v || !out) return ct::fail(CT_ERR_INVALID_ARG, "ct_tv_prox: null array");
+  if (batch <= 0) return ct::fail(CT_ERR_INVALID_ARG, "ct_tv_prox: batch=%d", batch);
+  if (!p.circular && (p.append != 0 || p.prepend >= 0))
+    return ct::fail(CT_ERR_INVALID_ARG, "ct_tv_prox: the differences are circular or have append = 0");
+  TvArgs a{};
+  if (batch > 65535 || !make_same(p, a.q))
+    return ct::fail(CT_ERR_UNSUPPORTED, "ct_tv_prox: batch above 65535 or an array of 2^31 elements or more");
+  a.x = v;
+  a.out = out;
+  a.r = (float)(1.0 / sqrt(2.0));
+  a.thr = thr;
+  a.inv_k = (float)(1.0 / (2.0 * p.nblocks));
+  const dim3 g((a.q.count + 255) / 256, batch);
+  cudaStream_t s = ct::as_stream(stream);
+  switch (2 * p.nblocks + (iso ? 1 : 0)) {
+    case 2: k_tv_prox<1, false><<<g, 256, 0, s>>>(a); break;
+    case 3: k_tv_prox<1, true><<<g, 256, 0, s>>>(a); break;
+    case 4: k_tv_prox<2, false><<<g, 256, 0, s>>>(a); break;
+    case 5: k_tv_prox<2, true><<<g, 256, 0, s>>>(a); break;
+    case 6: k_tv_prox<3, false><<<g, 256, 0, s>>>(a); break;
+    default: k_tv_prox<3, true><<<g, 256, 0, s>>>(a); break;
+  }
+  return ct::launch_check("k_tv_prox");
+}
+
 ct_status ct_l21_prox(const float* v, float* out, int32_t ncomp, int64_t n, float lam,
                       ct_stream_t stream) {
   if (!v || !out) return ct::fail(CT_ERR_INVALID_ARG, "ct_l21_prox: null array");
   if (ncomp < 1 || n < 0)
     return ct::fail(CT_ERR_INVALID_ARG, "ct_l21_prox: ncomp=%d n=%lld", ncomp, (long long)n);
   if (n == 0) return CT_OK;
+  const size_t blocks = ((size_t)n + 256 * kPxU - 1) / (256 * kPxU);
+  if (ncomp <= 3 && blocks < (1ull << 31)) {
+    cudaStream_t s = ct::as_stream(stream);
+    if (ncomp == 1)
+      k_l21_prox_few<1><<<(unsigned)blocks, 256, 0, s>>>(v, out, (size_t)n, lam);
+    else if (ncomp == 2)
+      k_l21_prox_few<2><<<(unsigned)blocks, 256, 0, s>>>(v, out, (size_t)n, lam);
+    else
+      k_l21_prox_few<3><<<(unsigned)blocks, 256, 0, s>>>(v, out, (size_t)n, lam);
+    return ct::launch_check("k_l21_prox_few");
+  }
   k_l21_prox<<<grid_for((size_t)n, 256), 256, 0, ct::as_stream(stream)>>>(v, out, ncomp,
                                                                            (size_t)n, lam);
   return ct::launch_check("k_l21_prox");

@@ -199,6 +199,12 @@ def _haar_desc(shape, axes):
     return _fd_desc(tuple(shape), tuple(axes), None, None, True)
 
 
+def _tv_desc(shape, axes, circular: bool):
+    from .linop import _fd_desc
+
+    return _fd_desc(tuple(shape), tuple(axes), None, None if circular else 0, circular)
+
+
 def _haar_fwd(x: torch.Tensor, axes) -> torch.Tensor:
     """Single-level shift-invariant Haar transform (HaarTransform,
     _tvnorm.py:458-538) by ct_haar_fwd: per axis a lowpass (x + x shifted by
@@ -280,6 +286,15 @@ class TVNorm(Functional):
         # evaluated in float32 as jax evaluates it
         f = np.float32
         thr = float(f(f(np.sqrt(f(2.0))) * f(K)) * f(lam))
+        # one pass for the two TV norms; a base norm of another kind (or an
+        # array of 2^31 elements or more) takes the composed path, which gives the same bits
+        iso = type(self.norm) is L21Norm and self.norm.l2_axis == 0
+        if (iso or type(self.norm) is L1Norm) and v.numel() < 2**31:
+            d = _tv_desc(v.shape, axes, self.circular)
+            out = torch.empty_like(v)
+            _lib.call("ct_tv_prox", ctypes.addressof(d), v.data_ptr(), out.data_ptr(), int(iso), thr, 1,
+                      _device.stream())
+            return out
         if self.circular:
             w = _haar_fwd(v, axes)
             hi = w[:, 1].contiguous()
