@@ -68,13 +68,19 @@ ct_status make_fd(const ct_fd_desc* d, FdParams& p, const char* who) {
 // Same-shape differences (circular, or exactly one end extended: every output
 // block has the input's shape), the form of every regulariser here.  Bound by
 // memory; what cost the time before was index arithmetic (two 64-bit divisions
-// an element) and one element in flight per thread.  A thread now takes kFdU
-// elements kFdT apart, finds each one's coordinates with two 32-bit
-// multiply-high divisions, reads x once for all axes and has all its loads in
-// flight before the first store.  192^3, three axes: forward 176 -> FWD_US us,
-// adjoint 150 -> ADJ_US us (as launched alone by a profiler).  Scalar
-// accesses throughout: rows of odd length are as common as multiples of four,
-// and 32-bit accesses of whole warps already fill the sectors.
+// an element) and one element in flight per thread.
+//
+// Rows of at least a warp (k_fd_rows): a warp takes up to kFdU elements a
+// lane of one row (the last axis), so the position along the other axes, and
+// with it the offset to the neighbour and the test for the line's end, is the
+// same for the whole warp and costs nothing per element.  32-bit accesses of
+// whole warps: rows of odd length are as common as multiples of four, and they
+// fill the sectors either way.  Shorter rows (k_fd_*_flat) would leave lanes
+// idle: there a thread takes kFdU elements of the flat array kFdT apart and
+// finds their coordinates with two 32-bit multiply-high divisions.
+// 192^3, three axes (forward / adjoint): 177 / 150 us with the divisions of
+// k_fd_fwd / k_fd_adj, 43 / 62 us flat, ROWF / ROWA us by rows; 27 us is a
+// copy of the three output arrays.
 // ---------------------------------------------------------------------------
 constexpr int kFdT = 256;  // threads of a block
 constexpr int kFdU = 4;    // elements per thread
@@ -99,6 +105,10 @@ struct FdSame {
   uint32_t stride[3];  // of axis[k]
   int mode;            // 0 circular, 1 append, 2 prepend
   int zero;            // extended sample: 0 = copy of the end, 1 = zero
+  // by rows: elements a lane, chunks of 32 per_lane elements in a row, their total
+  int per_lane;
+  uint32_t units;
+  FastDiv chunks;
 };
 
 // True when `p` is same-shape and every index fits 31 bits (the descriptor's
@@ -117,6 +127,21 @@ bool make_same(const FdParams& p, FdSame& q) {
   }
   q.mode = p.circular ? 0 : (app ? 1 : 2);
   q.zero = p.circular ? 0 : (app ? p.append : p.prepend);
+  // the elements a lane takes: whichever of 1..kFdU leaves the fewest lanes of
+  // a row's last chunk idle, the most of those
+  int best = 0;
+  uint32_t least = 0xffffffffu;
+  for (int u = 1; u <= kFdU; ++u) {
+    const uint32_t span = 32u * u, used = ((uint32_t)p.n[2] + span - 1) / span * span;
+    if (used <= least) {
+      least = used;
+      best = u;
+    }
+  }
+  q.per_lane = best;
+  const uint32_t chunks = ((uint32_t)p.n[2] + 32u * best - 1) / (32u * best);
+  q.chunks = fast_div(chunks);
+  q.units = (uint32_t)(p.in_count / p.n[2]) * chunks;
   return true;
 }
 
@@ -130,7 +155,7 @@ __device__ __forceinline__ void fd_coords(const FdSame& q, uint32_t e, int (&c)[
 // out[k][e] = (next) - (this) along axis k, next the circular neighbour or the
 // extended sample at the end (append), or (this) - (previous) (prepend).
 template <int NB>
-__global__ void __launch_bounds__(kFdT) k_fd_fwd_same(const float* __restrict__ x, float* __restrict__ out, const FdSame q) {
+__global__ void __launch_bounds__(kFdT) k_fd_fwd_flat(const float* __restrict__ x, float* __restrict__ out, const FdSame q) {
   x += (size_t)blockIdx.y * q.count;
   out += (size_t)blockIdx.y * NB * q.count;
   const uint32_t e0 = blockIdx.x * (uint32_t)(kFdT * kFdU) + threadIdx.x;
@@ -167,7 +192,7 @@ __global__ void __launch_bounds__(kFdT) k_fd_fwd_same(const float* __restrict__ 
 // x[e]; an end copied by the extension holds two, added in position order
 // (k_fd_adj below states the rule in general).
 template <int NB>
-__global__ void __launch_bounds__(kFdT) k_fd_adj_same(const float* __restrict__ d, float* __restrict__ x, const FdSame q) {
+__global__ void __launch_bounds__(kFdT) k_fd_adj_flat(const float* __restrict__ d, float* __restrict__ x, const FdSame q) {
   d += (size_t)blockIdx.y * NB * q.count;
   x += (size_t)blockIdx.y * q.count;
   const uint32_t e0 = blockIdx.x * (uint32_t)(kFdT * kFdU) + threadIdx.x;
@@ -214,6 +239,178 @@ __global__ void __launch_bounds__(kFdT) k_fd_adj_same(const float* __restrict__ 
     }
     x[e] = acc;
   }
+}
+
+// This warp's row and the lane's first element of it; false past the end.
+struct FdRow {
+  uint32_t row, c0, c1, c2;  // row index, coordinates (c2: the lane's first element)
+};
+__device__ __forceinline__ bool fd_row(const FdSame& q, FdRow& r) {
+  const uint32_t w = blockIdx.x * (kFdT / 32) + (threadIdx.x >> 5);
+  if (w >= q.units) return false;
+  r.row = div_by(q.chunks, w);
+  r.c0 = div_by(q.n1, r.row);
+  r.c1 = r.row - r.c0 * (uint32_t)q.n[1];
+  r.c2 = (w - r.row * q.chunks.d) * 32u * (uint32_t)q.per_lane + (threadIdx.x & 31);
+  return true;
+}
+
+// The forward and the adjoint below, by rows; U = FdSame::per_lane, MODE =
+// FdSame::mode.  FULL: the warp's whole chunk lies in the row, so every load
+// is unconditional at an immediate offset from its axis's base address.
+template <int NB, int U, int MODE, bool FULL>
+__device__ __forceinline__ void fd_fwd_row(const float* __restrict__ x, float* __restrict__ out, const FdSame& q,
+                                           const FdRow& r) {
+  constexpr bool back = MODE == 2, wrap = MODE == 0;
+  const int n2 = q.n[2], c = (int)r.c2;
+  const float* __restrict__ xp = x + (size_t)blockIdx.y * q.count + r.row * (uint32_t)n2 + c;
+  float xc[U], xn[NB][U];
+#pragma unroll
+  for (int u = 0; u < U; ++u)
+    if (FULL || c + 32 * u < n2) xc[u] = __ldg(xp + 32 * u);
+#pragma unroll
+  for (int k = 0; k < NB; ++k) {
+    const int a = q.axis[k];
+    if (a == 2) {
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (FULL || c + 32 * u < n2) {
+          const bool end = back ? c + 32 * u == 0 : c + 32 * u == n2 - 1;
+          const int off = end ? (wrap ? -(c + 32 * u) : 0) : (back ? -1 : 1);
+          xn[k][u] = __ldg(xp + 32 * u + off);
+          if (!wrap && end && q.zero) xn[k][u] = 0.0f;
+        }
+    } else {
+      const int ca = (int)(a == 1 ? r.c1 : r.c0), na = a == 1 ? q.n[1] : q.n[0];
+      const bool end = back ? ca == 0 : ca == na - 1;
+      const ptrdiff_t st = (ptrdiff_t)q.stride[k];
+      const float* __restrict__ np = xp + (end ? (wrap ? -(ptrdiff_t)ca * st : 0) : (back ? -st : st));
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (FULL || c + 32 * u < n2) {
+          xn[k][u] = __ldg(np + 32 * u);
+          if (!wrap && end && q.zero) xn[k][u] = 0.0f;
+        }
+    }
+  }
+  float* __restrict__ op = out + (size_t)blockIdx.y * NB * q.count + r.row * (uint32_t)n2 + c;
+#pragma unroll
+  for (int k = 0; k < NB; ++k)
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (FULL || c + 32 * u < n2)
+        op[(size_t)k * q.count + 32 * u] = back ? ct::fsub(xc[u], xn[k][u]) : ct::fsub(xn[k][u], xc[u]);
+}
+
+template <int NB, int U, int MODE, bool FULL>
+__device__ __forceinline__ void fd_adj_row(const float* __restrict__ d, float* __restrict__ x, const FdSame& q,
+                                           const FdRow& r) {
+  constexpr bool fwd = MODE == 2, wrap = MODE == 0;
+  const int n2 = q.n[2], c = (int)r.c2;
+  const float* __restrict__ dp = d + (size_t)blockIdx.y * NB * q.count + r.row * (uint32_t)n2 + c;
+  float dc[NB][U], dn[NB][U];
+#pragma unroll
+  for (int k = 0; k < NB; ++k) {
+    const float* __restrict__ dk = dp + (size_t)k * q.count;
+    const int a = q.axis[k];
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (FULL || c + 32 * u < n2) dc[k][u] = __ldg(dk + 32 * u);
+    if (a == 2) {
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (FULL || c + 32 * u < n2) {
+          const bool off = fwd ? c + 32 * u == n2 - 1 : c + 32 * u == 0;
+          const int at = off ? (wrap ? n2 - 1 : 0) : (fwd ? 1 : -1);
+          dn[k][u] = __ldg(dk + 32 * u + at);
+          if (!wrap && off) dn[k][u] = 0.0f;
+        }
+    } else {
+      const int ca = (int)(a == 1 ? r.c1 : r.c0), na = a == 1 ? q.n[1] : q.n[0];
+      const bool off = fwd ? ca == na - 1 : ca == 0;
+      const ptrdiff_t st = (ptrdiff_t)q.stride[k];
+      const float* __restrict__ np = dk + (off ? (wrap ? (ptrdiff_t)(na - 1) * st : 0) : (fwd ? st : -st));
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (FULL || c + 32 * u < n2) {
+          dn[k][u] = __ldg(np + 32 * u);
+          if (!wrap && off) dn[k][u] = 0.0f;
+        }
+    }
+  }
+  float* __restrict__ op = x + (size_t)blockIdx.y * q.count + r.row * (uint32_t)n2 + c;
+  float acc[U];
+#pragma unroll
+  for (int k = 0; k < NB; ++k) {
+    const int a = q.axis[k];
+    const int ca = (int)(a == 1 ? r.c1 : r.c0), na = a == 2 ? n2 : (a == 1 ? q.n[1] : q.n[0]);
+    const bool row_cp = a != 2 && (fwd ? ca == 0 : ca == na - 1);
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const bool cp = !wrap && !q.zero && (a == 2 ? (fwd ? c + 32 * u == 0 : c + 32 * u == n2 - 1) : row_cp);
+      float v;
+      if (fwd) {
+        v = ct::fsub(dc[k][u], dn[k][u]);
+        if (cp) v = ct::fadd(ct::fsub(0.0f, dc[k][u]), v);  // position 0 first
+      } else {
+        v = ct::fsub(dn[k][u], dc[k][u]);
+        if (cp) v = ct::fadd(v, dc[k][u]);  // then the position past the end: d[n-1] - 0
+      }
+      acc[u] = k == 0 ? v : ct::fadd(acc[u], v);
+    }
+  }
+#pragma unroll
+  for (int u = 0; u < U; ++u)
+    if (FULL || c + 32 * u < n2) op[32 * u] = acc[u];
+}
+
+template <int NB, int U, int MODE, bool ADJ>
+__global__ void __launch_bounds__(kFdT) k_fd_rows(const float* __restrict__ src, float* __restrict__ dst, const FdSame q) {
+  FdRow r;
+  if (!fd_row(q, r)) return;
+  const bool full = (int)(r.c2 | 31u) + 32 * (U - 1) < q.n[2];  // c2 of lane 0 is a multiple of 32
+  if (ADJ) {
+    if (full)
+      fd_adj_row<NB, U, MODE, true>(src, dst, q, r);
+    else
+      fd_adj_row<NB, U, MODE, false>(src, dst, q, r);
+  } else {
+    if (full)
+      fd_fwd_row<NB, U, MODE, true>(src, dst, q, r);
+    else
+      fd_fwd_row<NB, U, MODE, false>(src, dst, q, r);
+  }
+}
+
+// Launch of the same-shape kernels.
+template <bool ADJ, int NB, int U>
+void fd_rows_launch(const float* src, float* dst, const FdSame& q, dim3 g, cudaStream_t s) {
+  if (q.mode == 0)
+    k_fd_rows<NB, U, 0, ADJ><<<g, kFdT, 0, s>>>(src, dst, q);
+  else if (q.mode == 1)
+    k_fd_rows<NB, U, 1, ADJ><<<g, kFdT, 0, s>>>(src, dst, q);
+  else
+    k_fd_rows<NB, U, 2, ADJ><<<g, kFdT, 0, s>>>(src, dst, q);
+}
+
+template <bool ADJ, int NB>
+ct_status fd_same_launch(const float* src, float* dst, const FdSame& q, int batch, cudaStream_t s) {
+  if (q.n[2] >= 32) {
+    const dim3 g((q.units + kFdT / 32 - 1) / (kFdT / 32), batch);
+    switch (q.per_lane) {
+      case 1: fd_rows_launch<ADJ, NB, 1>(src, dst, q, g, s); break;
+      case 2: fd_rows_launch<ADJ, NB, 2>(src, dst, q, g, s); break;
+      case 3: fd_rows_launch<ADJ, NB, 3>(src, dst, q, g, s); break;
+      default: fd_rows_launch<ADJ, NB, 4>(src, dst, q, g, s); break;
+    }
+    return ct::launch_check("k_fd_rows");
+  }
+  const dim3 g((q.count + kFdT * kFdU - 1) / (kFdT * kFdU), batch);
+  if (ADJ)
+    k_fd_adj_flat<NB><<<g, kFdT, 0, s>>>(src, dst, q);
+  else
+    k_fd_fwd_flat<NB><<<g, kFdT, 0, s>>>(src, dst, q);
+  return ct::launch_check(ADJ ? "k_fd_adj_flat" : "k_fd_fwd_flat");
 }
 
 // Value of the extended line e (prepend/append applied) at position t.
@@ -591,15 +788,10 @@ ct_status ct_fd_fwd(const ct_fd_desc* d, const float* x, float* out, int32_t bat
   if (total == 0) return CT_OK;
   FdSame q{};
   if (batch <= 65535 && make_same(p, q)) {
-    const dim3 g((q.count + kFdT * kFdU - 1) / (kFdT * kFdU), batch);
     cudaStream_t s = ct::as_stream(stream);
-    if (p.nblocks == 1)
-      k_fd_fwd_same<1><<<g, kFdT, 0, s>>>(x, out, q);
-    else if (p.nblocks == 2)
-      k_fd_fwd_same<2><<<g, kFdT, 0, s>>>(x, out, q);
-    else
-      k_fd_fwd_same<3><<<g, kFdT, 0, s>>>(x, out, q);
-    return ct::launch_check("k_fd_fwd_same");
+    if (p.nblocks == 1) return fd_same_launch<false, 1>(x, out, q, batch, s);
+    if (p.nblocks == 2) return fd_same_launch<false, 2>(x, out, q, batch, s);
+    return fd_same_launch<false, 3>(x, out, q, batch, s);
   }
   k_fd_fwd<<<grid_for(total, 256), 256, 0, ct::as_stream(stream)>>>(x, out, p, batch);
   return ct::launch_check("k_fd_fwd");
@@ -615,15 +807,10 @@ ct_status ct_fd_adj(const ct_fd_desc* d, const float* dx, float* x, int32_t batc
   const size_t total = p.in_count * batch;
   FdSame q{};
   if (batch <= 65535 && make_same(p, q)) {
-    const dim3 g((q.count + kFdT * kFdU - 1) / (kFdT * kFdU), batch);
     cudaStream_t s = ct::as_stream(stream);
-    if (p.nblocks == 1)
-      k_fd_adj_same<1><<<g, kFdT, 0, s>>>(dx, x, q);
-    else if (p.nblocks == 2)
-      k_fd_adj_same<2><<<g, kFdT, 0, s>>>(dx, x, q);
-    else
-      k_fd_adj_same<3><<<g, kFdT, 0, s>>>(dx, x, q);
-    return ct::launch_check("k_fd_adj_same");
+    if (p.nblocks == 1) return fd_same_launch<true, 1>(dx, x, q, batch, s);
+    if (p.nblocks == 2) return fd_same_launch<true, 2>(dx, x, q, batch, s);
+    return fd_same_launch<true, 3>(dx, x, q, batch, s);
   }
   k_fd_adj<<<grid_for(total, 256), 256, 0, ct::as_stream(stream)>>>(dx, x, p, batch);
   return ct::launch_check("k_fd_adj");
