@@ -12,19 +12,31 @@ from . import _lib
 _reduce_ws: dict[tuple[int, int], torch.Tensor] = {}
 
 
+# torch.device objects by index, made once a CUDA device has been seen (a
+# device that is there stays there; asking again costs more than a small
+# projection's launches)
+_devices: dict[int, torch.device] = {}
+
+
 def require_cuda() -> torch.device:
     """Return the current CUDA device; raise if there is none (no CPU path)."""
-    if not torch.cuda.is_available():
-        raise RuntimeError(
-            "scico_gb300 runs its operators on a CUDA device only and found none; "
-            "there is no CPU fallback"
-        )
-    return torch.device("cuda", torch.cuda.current_device())
+    if not _devices:
+        if not torch.cuda.is_available():
+            raise RuntimeError(
+                "scico_gb300 runs its operators on a CUDA device only and found none; "
+                "there is no CPU fallback"
+            )
+        torch.cuda.current_device()  # initialises CUDA
+    index = torch._C._cuda_getDevice()
+    dev = _devices.get(index)
+    if dev is None:
+        dev = _devices[index] = torch.device("cuda", index)
+    return dev
 
 
 def stream() -> int:
     """Handle of the current torch CUDA stream (passed to the C ABI)."""
-    return torch.cuda.current_stream().cuda_stream
+    return torch._C._cuda_getCurrentRawStream(require_cuda().index)
 
 
 def to_device(x, shape=None, name: str = "array") -> torch.Tensor:

@@ -79,7 +79,7 @@ ct_status make_fd(const ct_fd_desc* d, FdParams& p, const char* who) {
 // idle: there a thread takes kFdU elements of the flat array kFdT apart and
 // finds their coordinates with two 32-bit multiply-high divisions.
 // 192^3, three axes (forward / adjoint): 177 / 150 us with the divisions of
-// k_fd_fwd / k_fd_adj, 43 / 62 us flat, ROWF / ROWA us by rows; 27 us is a
+// k_fd_fwd / k_fd_adj, 43 / 62 us flat, 19 / 29 us by rows; 26 us is a
 // copy of the three output arrays.
 // ---------------------------------------------------------------------------
 constexpr int kFdT = 256;  // threads of a block
@@ -599,7 +599,7 @@ __device__ __forceinline__ void l21_shrink(float (&v)[NC], float lam) {
 
 // The prox of up to three components (every image gradient): the components
 // are read once and kept in registers, kPxU vectors in flight per thread.
-// 3 x 192^3: 43 -> PROX_US us.
+// 3 x 192^3: 43 -> 27.7 us, the time of a copy.
 constexpr int kPxU = 4;
 template <int NC>
 __global__ void __launch_bounds__(256) k_l21_prox_few(const float* __restrict__ v, float* __restrict__ out, size_t n,
@@ -671,7 +671,7 @@ __global__ void k_l1_prox(const float* __restrict__ v, float* __restrict__ out, 
 // ct_l1_prox and ct_haar_adj round, in their order: same bits.  Bound by the
 // divisions and roots (L2,1) or by launch latency at small sizes; the composed
 // path took eight launches and passed over 2 naxes arrays: 512^2, L2,1, edge
-// padding 280 -> TVP_US us, 1024^2 TVP1_US us.
+// padding 40 us of kernels (and 280 us of launches around them) -> 5 us.
 // ---------------------------------------------------------------------------
 struct TvArgs {
   const float* x;

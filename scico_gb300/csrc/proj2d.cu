@@ -58,6 +58,7 @@ constexpr int kAdjThreads = 256;  // adjoint CTA: 64 x 64 pixels = kAdjThreads x
 constexpr int kAVC = 32;        // views staged per adjoint run
 constexpr int kAdjTargetCtas = 1216;  // 152 SMs x 8: view splits until the CTAs balance over the SMs
 constexpr int kAdjMinViewsPerSplit = 16;
+constexpr size_t kMaxSmem = 200 * 1024;  // dynamic shared memory of a projector CTA
 constexpr uint32_t kMaxPolls = 1u << 24;
 // Poll limit of the forward's strip-copy wait, read when a call launches
 // (ct_set_wait_poll_limit); a solver graph keeps the value it was captured
@@ -837,8 +838,8 @@ ct_status proj2d_check(const ct_geom2d* g, const char* who) {
   if (!(g->max_width > 0.0f) || g->max_width > 16.0f)
     return fail(CT_ERR_UNSUPPORTED, "%s: max projected pixel width %g outside (0, 16]", who,
                 (double)g->max_width);
-  const Proj2dPlan p = proj2d_plan(g, 1);
-  if (p.fwd_smem > 200 * 1024 || p.adj_smem > 200 * 1024)
+  const Proj2dPlan p = proj2d_plan_sched(g, 1, Sched2d{});  // the spans do not depend on the schedule
+  if (p.fwd_smem > kMaxSmem || p.adj_smem > kMaxSmem)
     return fail(CT_ERR_UNSUPPORTED, "%s: tile spans of %d / %d bins too large", who, p.L, p.W);
   return CT_OK;
 }
@@ -938,20 +939,25 @@ Proj2dPlan proj2d_plan(const ct_geom2d* g, int batch) {
   return proj2d_plan_sched(g, batch, sched_lookup(g, batch, v) ? v.s : Sched2d{});
 }
 
+// The kernels' dynamic shared memory limit, raised once per device to the most
+// that proj2d_check lets through (asking at every call cost three driver calls).
 ct_status proj2d_prepare(const Proj2dPlan& p) {
+  (void)p;
   if (!errflag_ptr()) return fail(CT_ERR_CUDA, "proj2d: error-word address unavailable");
-  ct_status st = cuda_check(cudaFuncSetAttribute(k_proj2d_fwd_strips<kLSDefault>,
-                                                 cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                 (int)p.fwd_smem),
-                            "fwd smem attribute");
+  static std::atomic<uint64_t> done{0};
+  int dev = 0;
+  ct_status st = cuda_check(cudaGetDevice(&dev), "current device");
   if (st != CT_OK) return st;
-  st = cuda_check(cudaFuncSetAttribute(k_proj2d_fwd_strips<0>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)p.fwd_smem),
-                  "fwd smem attribute");
-  if (st != CT_OK) return st;
-  return cuda_check(cudaFuncSetAttribute(k_proj2d_adj, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)p.adj_smem),
-                    "adj smem attribute");
+  const uint64_t bit = dev < 64 ? 1ull << dev : 0;
+  if (done.load(std::memory_order_acquire) & bit) return CT_OK;
+  auto raise = [](auto* kernel, const char* what) {
+    return cuda_check(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem), what);
+  };
+  if ((st = raise(k_proj2d_fwd_strips<kLSDefault>, "fwd smem attribute")) != CT_OK) return st;
+  if ((st = raise(k_proj2d_fwd_strips<0>, "fwd smem attribute")) != CT_OK) return st;
+  if ((st = raise(k_proj2d_adj, "adj smem attribute")) != CT_OK) return st;
+  done.fetch_or(bit, std::memory_order_release);
+  return CT_OK;
 }
 
 ct_status proj2d_fwd_launch(const ct_geom2d* g, const Proj2dPlan& p, const float* img, float* sino,

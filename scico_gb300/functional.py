@@ -18,6 +18,7 @@ proxes run in the ctgpu kernels.
 from __future__ import annotations
 
 import ctypes
+import math
 from typing import Tuple, Union
 
 import numpy as np
@@ -110,6 +111,10 @@ class SeparableFunctional(Functional):
 def _l2_layout(x: torch.Tensor, l2_axis) -> Tuple[torch.Tensor, int, int, tuple]:
     """Move the l2 axes to the front; return (contiguous (ncomp, n) view, ncomp, n, perm)."""
     nd = x.ndim
+    if type(l2_axis) is int and l2_axis == 0 and nd >= 1:  # the stacked differences: already in place
+        ncomp = x.shape[0]
+        n = math.prod(x.shape[1:])
+        return x.contiguous().reshape(ncomp, n), ncomp, n, tuple(range(nd))
     if l2_axis is None:
         ax = tuple(range(nd))
     elif isinstance(l2_axis, (int, np.integer)):
@@ -192,6 +197,9 @@ class L1Norm(Functional):
 # ---------------------------------------------------------------------------
 # TV norms (scico/functional/_tvnorm.py)
 # ---------------------------------------------------------------------------
+
+_SQRT2 = np.sqrt(np.float32(2.0))
+
 
 def _haar_desc(shape, axes):
     from .linop import _fd_desc
@@ -284,8 +292,7 @@ class TVNorm(Functional):
         K = 2 * len(axes)
         # the base norm's prox parameter snp.sqrt(2) * K * lam (_tvnorm.py:203),
         # evaluated in float32 as jax evaluates it
-        f = np.float32
-        thr = float(f(f(np.sqrt(f(2.0))) * f(K)) * f(lam))
+        thr = float(_SQRT2 * np.float32(K) * np.float32(lam))
         # one pass for the two TV norms; a base norm of another kind (or an
         # array of 2^31 elements or more) takes the composed path, which gives the same bits
         iso = type(self.norm) is L21Norm and self.norm.l2_axis == 0

@@ -16,6 +16,7 @@ Every operator evaluation runs in the ctgpu kernels through the C ABI.
 
 from __future__ import annotations
 
+import functools
 import math
 import warnings
 from typing import Callable, Optional, Sequence, Tuple, Union
@@ -28,9 +29,15 @@ from . import _device, _lib
 Shape = Tuple[int, ...]
 
 
+_NP_OF_TORCH: dict = {}
+
+
 def _np_dtype(dt) -> np.dtype:
     if isinstance(dt, torch.dtype):
-        return np.dtype(str(dt).replace("torch.", ""))
+        got = _NP_OF_TORCH.get(dt)
+        if got is None:
+            got = _NP_OF_TORCH[dt] = np.dtype(str(dt).replace("torch.", ""))
+        return got
     return np.dtype(dt)
 
 
@@ -196,7 +203,7 @@ class LinearOperator:
 def _size(shape) -> int:
     if len(shape) and isinstance(shape[0], tuple):
         return sum(_size(s) for s in shape)
-    return int(np.prod(shape)) if len(shape) else 1
+    return math.prod(int(n) for n in shape)
 
 
 def _add(a, b):
@@ -424,6 +431,7 @@ class XRayTransform2D(LinearOperator):
             )
         self._views_dev = None
         self._geom = None
+        self._ws_bytes: dict = {}
 
         super().__init__(
             input_shape=self.input_shape,
@@ -446,12 +454,19 @@ class XRayTransform2D(LinearOperator):
         return self._geom
 
     def workspace_bytes(self, batch: int = 1) -> Tuple[int, int]:
-        fwd = _lib.c_size_t(0)
-        adj = _lib.c_size_t(0)
-        g = self.geometry()
-        _lib.call("ct_proj2d_workspace", _lib.ctypes.addressof(g), batch,
-                  _lib.ctypes.addressof(fwd), _lib.ctypes.addressof(adj))
-        return int(fwd.value), int(adj.value)
+        """Scratch bytes of :meth:`project` and :meth:`back_project`: a function
+        of the geometry, the batch and the device alone (it covers every schedule
+        that :meth:`autotune` may record), so asked once."""
+        key = (batch, _device.require_cuda().index)
+        got = self._ws_bytes.get(key)
+        if got is None:
+            fwd = _lib.c_size_t(0)
+            adj = _lib.c_size_t(0)
+            g = self.geometry()
+            _lib.call("ct_proj2d_workspace", _lib.ctypes.addressof(g), batch,
+                      _lib.ctypes.addressof(fwd), _lib.ctypes.addressof(adj))
+            got = self._ws_bytes[key] = (int(fwd.value), int(adj.value))
+        return got
 
     def autotune(self, batch: int = 1, reps: int = 10) -> dict:
         """Measure the projector's launch schedules for this geometry and
@@ -595,6 +610,7 @@ class XRayTransform3D(LinearOperator):
         self._row_offset = int(row_offset.value)
         self._dev_tables = None
         self._geom = None
+        self._ws_bytes: dict = {}
         super().__init__(
             input_shape=self.input_shape,
             input_dtype=np.float32,
@@ -623,12 +639,19 @@ class XRayTransform3D(LinearOperator):
         return self._geom
 
     def workspace_bytes(self, batch: int = 1) -> Tuple[int, int]:
-        fwd = _lib.c_size_t(0)
-        adj = _lib.c_size_t(0)
-        g = self.geometry()
-        _lib.call("ct_proj3d_workspace", _lib.ctypes.addressof(g), batch,
-                  _lib.ctypes.addressof(fwd), _lib.ctypes.addressof(adj))
-        return int(fwd.value), int(adj.value)
+        """Scratch bytes of :meth:`project` and :meth:`back_project`: a function
+        of the geometry, the batch and the device alone (it covers every schedule
+        that :meth:`autotune` may record), so asked once."""
+        key = (batch, _device.require_cuda().index)
+        got = self._ws_bytes.get(key)
+        if got is None:
+            fwd = _lib.c_size_t(0)
+            adj = _lib.c_size_t(0)
+            g = self.geometry()
+            _lib.call("ct_proj3d_workspace", _lib.ctypes.addressof(g), batch,
+                      _lib.ctypes.addressof(fwd), _lib.ctypes.addressof(adj))
+            got = self._ws_bytes[key] = (int(fwd.value), int(adj.value))
+        return got
 
     def autotune(self, reps: int = 5) -> dict:
         """Measure the 3D projector's launch schedules for this geometry
@@ -774,10 +797,11 @@ class FiniteDifference(LinearOperator):
         super().__init__(input_shape=input_shape, output_shape=out_shape, input_dtype=input_dtype,
                          output_dtype=input_dtype, eval_fn=self._fwd, adj_fn=self._adjoint)
         self.block_shapes = shapes
+        self._out_count = sum(_size(sh) for sh in shapes)
 
     def _fwd(self, x):
         t, batch, has_batch = _batch_of(x, self.input_shape, "x")
-        flat = _device.empty((batch, sum(_size(s) for s in self.block_shapes)))
+        flat = _device.empty((batch, self._out_count))
         _lib.call("ct_fd_fwd", _lib.ctypes.addressof(self._desc), t.data_ptr(), flat.data_ptr(), batch,
                   _device.stream())
         if self.collapsed:
@@ -856,7 +880,9 @@ class SingleAxisFiniteDifference(LinearOperator):
         return out
 
 
+@functools.lru_cache(maxsize=256)
 def _fd_desc(input_shape, axes, prepend, append, circular) -> _lib.FdDesc:
+    """ct_fd_desc of a difference operator (read by the library, never written)."""
     if len(input_shape) > 3:
         raise ValueError("finite differences are implemented for up to 3 axes")
     d = _lib.FdDesc()
