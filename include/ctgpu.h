@@ -128,6 +128,17 @@ ct_status ct_proj2d_adj(const ct_geom2d* g, const float* sino, float* img,
                         ct_stream_t stream);
 
 /*
+ * img[b] = (mask * scale) * A^T sino[b]: the last step of XRayTransform2D.fbp
+ * (_xray2d.py:190-197) with its detector mask, rows x cols bytes, non-zero
+ * where the pixel is kept; float32(mask ? scale : 0) times the adjoint's float32
+ * result.  Workspace as ct_proj2d_adj.
+ */
+ct_status ct_proj2d_adj_masked(const ct_geom2d* g, const float* sino,
+                               const uint8_t* mask, float scale, float* img,
+                               int32_t batch, void* workspace,
+                               size_t workspace_bytes, ct_stream_t stream);
+
+/*
  * Device-side checks.  The projector kernels never trap: a check that fails
  * on the device sets a bit of a per-device error word and skips the work it
  * guards (bit 0: a forward tile's bins exceed the plan; bit 1: a forward

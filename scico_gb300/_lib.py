@@ -193,6 +193,7 @@ _SIGNATURES = {
     "ct_proj2d_fwd": (ctypes.c_int, [P, P, P, c_int32, P, c_size_t, P]),
     "ct_proj2d_fwd_noalloc": (ctypes.c_int, [P, P, P, c_int32, P]),
     "ct_proj2d_adj": (ctypes.c_int, [P, P, P, c_int32, P, c_size_t, P]),
+    "ct_proj2d_adj_masked": (ctypes.c_int, [P, P, P, c_float, P, c_int32, P, c_size_t, P]),
     "ct_proj2d_check": (ctypes.c_int, [P]),
     "ct_proj2d_errflag": (ctypes.c_int, []),
     "ct_proj3d_errflag": (ctypes.c_int, []),

@@ -745,13 +745,27 @@ __global__ void __launch_bounds__(kAdjThreads) k_proj2d_adj(const AdjArgs a) {
   }
 }
 
-// out[e] = sum_s part[s*stride + e] in split order.
-__global__ void k_sum_splits(const float* __restrict__ part, float* __restrict__ out, size_t n,
-                             int nsplit, size_t stride) {
+// out[e] = sum_s part[s*stride + e] in split order; with a mask (of n_img
+// pixels, one per image of the batch), times `scale` where it is set and 0
+// where it is not (out may be part when there is one split).  Latency-bound:
+// kSumU splits are loaded before they are added.
+constexpr int kSumU = 8;
+template <bool MASK>
+__global__ void __launch_bounds__(256) k_sum_splits(const float* part, float* out, size_t n, int nsplit, size_t stride,
+                                                    const uint8_t* __restrict__ mask, size_t n_img, float scale) {
   for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < n;
        e += (size_t)gridDim.x * blockDim.x) {
     float s = 0.0f;
-    for (int k = 0; k < nsplit; ++k) s += part[(size_t)k * stride + e];
+    for (int k = 0; k < nsplit; k += kSumU) {
+      float v[kSumU];
+#pragma unroll
+      for (int u = 0; u < kSumU; ++u)
+        if (k + u < nsplit) v[u] = part[(size_t)(k + u) * stride + e];
+#pragma unroll
+      for (int u = 0; u < kSumU; ++u)
+        if (k + u < nsplit) s += v[u];
+    }
+    if (MASK) s = ct::fmul(mask[n_img == n ? e : e % n_img] ? scale : 0.0f, s);
     out[e] = s;
   }
 }
@@ -930,7 +944,7 @@ uint32_t proj2d_wait_polls() { return g_wait_polls.load(std::memory_order_relaxe
 
 ct_status proj2d_sum_splits(const float* part, float* out, size_t n, int nsplit, cudaStream_t s) {
   const int blocks = (int)std::min<size_t>((n + 255) / 256, 4096);
-  k_sum_splits<<<blocks, 256, 0, s>>>(part, out, n, nsplit, n);
+  k_sum_splits<false><<<blocks, 256, 0, s>>>(part, out, n, nsplit, n, nullptr, n, 1.0f);
   return launch_check("k_sum_splits");
 }
 
@@ -1047,28 +1061,41 @@ ct_status ct_proj2d_fwd(const ct_geom2d* g, const float* img, float* sino, int32
                                ct::as_stream(stream), nullptr);
 }
 
-ct_status ct_proj2d_adj(const ct_geom2d* g, const float* sino, float* img, int32_t batch,
-                        void* workspace, size_t workspace_bytes, ct_stream_t stream) {
-  ct_status st = ct::proj2d_check(g, "ct_proj2d_adj");
+static ct_status adj_call(const char* who, const ct_geom2d* g, const float* sino, float* img, int32_t batch,
+                          void* workspace, size_t workspace_bytes, const uint8_t* mask, float scale,
+                          ct_stream_t stream) {
+  ct_status st = ct::proj2d_check(g, who);
   if (st != CT_OK) return st;
-  if (!img || !sino) return ct::fail(CT_ERR_INVALID_ARG, "ct_proj2d_adj: null array");
-  if (batch <= 0) return ct::fail(CT_ERR_INVALID_ARG, "ct_proj2d_adj: batch=%d", batch);
+  if (!img || !sino) return ct::fail(CT_ERR_INVALID_ARG, "%s: null array", who);
+  if (batch <= 0) return ct::fail(CT_ERR_INVALID_ARG, "%s: batch=%d", who, batch);
   const ct::Proj2dPlan p = ct::proj2d_plan(g, batch);
   cudaStream_t s = ct::as_stream(stream);
   if (p.nsplit > 1) {
     if (!workspace || workspace_bytes < p.adj_bytes || !ct::aligned(workspace, 256))
-      return ct::fail(CT_ERR_WORKSPACE, "ct_proj2d_adj: need %zu bytes (256-B aligned), got %zu",
-                      p.adj_bytes, workspace_bytes);
+      return ct::fail(CT_ERR_WORKSPACE, "%s: need %zu bytes (256-B aligned), got %zu", who, p.adj_bytes,
+                      workspace_bytes);
   }
   st = ct::proj2d_prepare(p);
   if (st != CT_OK) return st;
   float* part = static_cast<float*>(workspace);
   st = ct::proj2d_adj_launch(g, p, sino, img, part, batch, s, nullptr);
-  if (st != CT_OK || p.nsplit == 1) return st;
-  const size_t n = (size_t)batch * g->rows * g->cols;
+  if (st != CT_OK || (p.nsplit == 1 && !mask)) return st;
+  const size_t n_img = (size_t)g->rows * g->cols, n = (size_t)batch * n_img;
+  if (!mask) return ct::proj2d_sum_splits(part, img, n, p.nsplit, s);
   const int blocks = (int)std::min<size_t>((n + 255) / 256, 4096);
-  k_sum_splits<<<blocks, 256, 0, s>>>(part, img, n, p.nsplit, n);
+  k_sum_splits<true><<<blocks, 256, 0, s>>>(p.nsplit == 1 ? img : part, img, n, p.nsplit, n, mask, n_img, scale);
   return ct::launch_check("k_sum_splits");
+}
+
+ct_status ct_proj2d_adj(const ct_geom2d* g, const float* sino, float* img, int32_t batch,
+                        void* workspace, size_t workspace_bytes, ct_stream_t stream) {
+  return adj_call("ct_proj2d_adj", g, sino, img, batch, workspace, workspace_bytes, nullptr, 1.0f, stream);
+}
+
+ct_status ct_proj2d_adj_masked(const ct_geom2d* g, const float* sino, const uint8_t* mask, float scale, float* img,
+                               int32_t batch, void* workspace, size_t workspace_bytes, ct_stream_t stream) {
+  if (!mask) return ct::fail(CT_ERR_INVALID_ARG, "ct_proj2d_adj_masked: null mask");
+  return adj_call("ct_proj2d_adj_masked", g, sino, img, batch, workspace, workspace_bytes, mask, scale, stream);
 }
 
 }  // extern "C"
@@ -1157,9 +1184,7 @@ ct_status ct_proj2d_autotune(const ct_geom2d* g, int32_t batch, float* img, floa
         [&] {
           ct_status r = ct::proj2d_adj_launch(g, p, sino, img, ws, batch, s, nullptr);
           if (r != CT_OK || p.nsplit == 1) return r;
-          const int blocks = (int)std::min<size_t>((n + 255) / 256, 4096);
-          k_sum_splits<<<blocks, 256, 0, s>>>(ws, img, n, p.nsplit, n);
-          return ct::launch_check("k_sum_splits");
+          return ct::proj2d_sum_splits(ws, img, n, p.nsplit, s);
         },
         reps, s, us);
     if (st != CT_OK) return st;

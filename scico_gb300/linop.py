@@ -549,7 +549,17 @@ class XRayTransform2D(LinearOperator):
             ones = _device.to_device(torch.ones(self.output_shape))
             self.fbp_mask = self.back_project(ones) >= nv * (1.0 - 1e-5)
         scale = float(np.pi * self.dx[0] * self.dx[1] / nv)
-        return scale * self.fbp_mask.to(torch.float32) * self.back_project(hy)
+        mask = self.fbp_mask
+        if not (isinstance(mask, torch.Tensor) and mask.dtype == torch.bool and mask.device == t.device
+                and tuple(mask.shape) == self.input_shape and mask.is_contiguous()):  # one set by the caller
+            return scale * mask.to(torch.float32) * self.back_project(hy)
+        g = self.geometry()
+        out = _device.empty(((batch,) if has_batch else ()) + self.input_shape)
+        _, adj_bytes = self.workspace_bytes(batch)
+        ws = _device.workspace(adj_bytes)
+        _lib.call("ct_proj2d_adj_masked", _lib.ctypes.addressof(g), hy.data_ptr(), mask.data_ptr(), scale,
+                  out.data_ptr(), batch, ws.data_ptr(), ws.numel(), _device.stream())
+        return out
 
 
 class XRayTransform3D(LinearOperator):
