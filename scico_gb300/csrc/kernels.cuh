@@ -59,8 +59,12 @@ struct Proj3dPlan {
   // AXIS0 forward: slices padded to the CTA's 64, tiles, tile groups, views per CTA
   int Spad = 0, tiles_k = 0, n_tiles = 0, G = 1, vpc = 16;
   size_t fwd_smem = 0;
+  // GENERAL forward: windows of a view (bound), segments of the planes, views per launch
+  int nwin = 0, nseg = 1, gen_views = 1;
+  size_t gen_plan = 0, gen_turn = 0;  // bytes of the views' plans and of the turned volume
   // adjoint view splits (both kinds)
   int nsplit = 1, per_split = 0;
+  size_t adj_least = 0, adj_tune = 0;  // GENERAL: scratch below which an adjoint / its tuning is refused
   size_t fwd_bytes = 0, adj_bytes = 0;
   // the same for the largest tile-group / split counts a schedule may use
   // (workspaces sized with these stay valid after ct_proj3d_autotune)
@@ -79,7 +83,8 @@ Proj3dPlan proj3d_plan(const ct_geom3d* g, int batch);  // recorded schedule, el
 Proj3dPlan proj3d_plan_sched(const ct_geom3d* g, Sched3d s);
 // One-time per-process function attributes; must run before any stream capture.
 ct_status proj3d_prepare(const ct_geom3d* g, const Proj3dPlan& p);
-// proj = A vol for one volume; `ws` holds p.fwd_bytes.  `skip` as for 2D.
+// proj = A vol for one volume; `ws` holds p.fwd_bytes (GENERAL: or is null, the
+// slower kernel).  `skip` as for 2D.
 ct_status proj3d_fwd_launch(const ct_geom3d* g, const Proj3dPlan& p, const float* vol, float* proj,
                             void* ws, cudaStream_t s, const double* skip);
 // A^T proj for one projection set.  With p.nsplit == 1 the result goes to

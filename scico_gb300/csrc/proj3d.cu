@@ -29,12 +29,7 @@
 //               accumulators per thread; the view's detector rows of the
 //               CTA's slices are staged as (y[c], y[c+1]) pairs, read with
 //               one 8-byte shared load per slice.
-//  * GENERAL -- any matrices.  The adjoint is voxel-driven (four gathers per
-//    view, as the reference's _back_project_single).  The forward is
-//    detector-driven: each detector pixel marches along the axis on which
-//    the ray direction is largest and, in each plane, visits the voxels whose
-//    footprint can cover it (an exact membership test on the rounded ul
-//    decides), so each output has a single owner and no atomics are needed.
+//  * GENERAL -- any matrices: proj3d_gen.cuh.
 #include <algorithm>
 #include <cmath>
 #include <map>
@@ -57,7 +52,6 @@ constexpr int kFwdViewsPerCta = 16;
 constexpr int kFwdViewsPerWarp = kFwdViewsPerCta / 8;
 constexpr int kAdjRows = 16;  // AXIS0 adjoint tile: 16 (axis 1) x 32 (axis 2) pixels
 constexpr int kAdjTargetCtas = 304;
-constexpr int kGenViewChunk = 64;
 
 static_assert(kTileJ * kTileK == kOrd, "order table covers one tile");
 
@@ -103,6 +97,14 @@ __device__ __forceinline__ void cp_async4(uint32_t dst, const float* src, bool v
 __device__ __forceinline__ void cp_async_wait_all() {
   asm volatile("cp.async.wait_all;" ::: "memory");
 }
+
+}  // namespace
+}  // namespace ct
+
+#include "proj3d_gen.cuh"
+
+namespace ct {
+namespace {
 
 // ---------------------------------------------------------------------------
 // AXIS0 forward
@@ -512,59 +514,10 @@ __global__ void __launch_bounds__(256, 2) k_p3_ax0_adj(const Ax0AdjArgs a) {
 }
 
 // ---------------------------------------------------------------------------
-// GENERAL adjoint: one voxel per thread, views in order, four gathers each
-// (_back_project_single, :192-204).
-// ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) k_p3_gen_adj(const float* __restrict__ proj,
-                                                    float* __restrict__ out,
-                                                    const float* __restrict__ views, int n0,
-                                                    int n1, int n2, int V, int R, int C,
-                                                    int per_split, size_t split_stride,
-                                                    const double* skip) {
-  if (skip && *skip != 0.0) return;
-  __shared__ float sm[kGenViewChunk * 8];
-  const size_t n = (size_t)n0 * n1 * n2;
-  const size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int split = blockIdx.y;
-  const int vs = split * per_split, ve = min(V, vs + per_split);
-  int i0 = 0, i1 = 0, i2 = 0;
-  if (e < n) {
-    i2 = (int)(e % n2);
-    const size_t r = e / n2;
-    i1 = (int)(r % n1);
-    i0 = (int)(r / n1);
-  }
-  const float x0 = (float)i0 + 0.5f, x1 = (float)i1 + 0.5f, x2 = (float)i2 + 0.5f;
-  float acc = 0.f;
-  for (int vc = vs; vc < ve; vc += kGenViewChunk) {
-    const int nvc = min(kGenViewChunk, ve - vc);
-    __syncthreads();
-    for (int q = threadIdx.x; q < nvc * 8; q += blockDim.x)
-      sm[q] = views[(size_t)(vc + q / 8) * kVT + (q & 7)];
-    __syncthreads();
-    if (e >= n) continue;
-    for (int vi = 0; vi < nvc; ++vi) {
-      const float* m = sm + vi * 8;
-      int u0, u1;
-      float t0, t1;
-      edge3(px3(m[0], m[1], m[2], m[3], x0, x1, x2), u0, t0);
-      edge3(px3(m[4], m[5], m[6], m[7], x0, x1, x2), u1, t1);
-      const float s0 = fsub(0.5f, t0), s1 = fsub(0.5f, t1);
-      const bool r0 = u0 >= 0 && u0 < R, r1 = u0 + 1 >= 0 && u0 + 1 < R;
-      const bool c0 = u1 >= 0 && u1 < C, c1 = u1 + 1 >= 0 && u1 + 1 < C;
-      const float* y = proj + (size_t)(vc + vi) * R * C;
-      if (r0 && c0) acc = fmaf(__ldg(y + (size_t)u0 * C + u1), fmul(fmul(t0, t1), 4.0f), acc);
-      if (r1 && c0) acc = fmaf(__ldg(y + (size_t)(u0 + 1) * C + u1), fmul(fmul(s0, t1), 4.0f), acc);
-      if (r0 && c1) acc = fmaf(__ldg(y + (size_t)u0 * C + u1 + 1), fmul(fmul(t0, s1), 4.0f), acc);
-      if (r1 && c1)
-        acc = fmaf(__ldg(y + (size_t)(u0 + 1) * C + u1 + 1), fmul(fmul(s0, s1), 4.0f), acc);
-    }
-  }
-  if (e < n) out[(size_t)split * split_stride + e] = acc;
-}
-
-// ---------------------------------------------------------------------------
-// GENERAL forward: one detector pixel per thread.
+// GENERAL forward, the march: one detector pixel per thread.  Taps are found
+// plane by plane along the ray's dominant axis; an exact test on the rounded ul
+// decides membership, so each output has one owner.  plan: only the views that
+// the window kernels (proj3d_gen.cuh) leave out; null = every view.
 // ---------------------------------------------------------------------------
 // x range [lo, hi] of voxel centres along one axis allowed by the detector
 // window [wlo, whi] on one detector axis, given Px = beta + mq * x.
@@ -580,16 +533,15 @@ __device__ __forceinline__ void narrow(float beta, float mq, float wlo, float wh
   }
 }
 
-__global__ void __launch_bounds__(256) k_p3_gen_fwd(const float* __restrict__ vol,
-                                                    float* __restrict__ proj,
-                                                    const float* __restrict__ views, int n0,
-                                                    int n1, int n2, int V, int R, int C,
-                                                    const double* skip) {
+__global__ void __launch_bounds__(256) k_p3_gen_march(const float* __restrict__ vol,
+                                                      float* __restrict__ proj,
+                                                      const float* __restrict__ views, int n0,
+                                                      int n1, int n2, int R, int C,
+                                                      const GenView* __restrict__ plan,
+                                                      const double* skip) {
   if (skip && *skip != 0.0) return;
   const int v = blockIdx.y;
-  const int pix = blockIdx.x * blockDim.x + threadIdx.x;
-  if (pix >= R * C) return;
-  const int r = pix / C, c = pix - (pix / C) * C;
+  if (plan && plan[v].ok) return;
   const float* m = views + (size_t)v * kVT;
   float mm[8];
 #pragma unroll
@@ -608,55 +560,58 @@ __global__ void __launch_bounds__(256) k_p3_gen_fwd(const float* __restrict__ vo
               mq0 = pick(mm[0], mm[1], mm[2], 2);
   const float ma1 = pick(mm[4], mm[5], mm[6], 0), mp1 = pick(mm[4], mm[5], mm[6], 1),
               mq1 = pick(mm[4], mm[5], mm[6], 2);
-  // taps reaching (r, c) come from voxels with floor(left) in {r-1, r} x
-  // {c-1, c}: Px in [r-0.75, r+1.25) x [c-0.75, c+1.25); widened by a margin
-  // far above the rounding of the range arithmetic (the exact test decides)
-  const float mg = 0.05f;
-  const float w0lo = (float)r - 0.75f - mg, w0hi = (float)r + 1.25f + mg;
-  const float w1lo = (float)c - 0.75f - mg, w1hi = (float)c + 1.25f + mg;
-  // |x_p - centre_p| <= e_p from the 2x2 system of the (p, q) plane
-  const float det = mp0 * mq1 - mq0 * mp1;
-  const float h0 = 0.5f * (w0hi - w0lo), h1 = 0.5f * (w1hi - w1lo);
-  const float ep = (fabsf(mq1) * h0 + fabsf(mq0) * h1) / fabsf(det);
   // voxel strides of the marching, p and q axes
-  const size_t sa = (size_t)pick((float)((size_t)n1 * n2), (float)n2, 1.0f, 0);
+  const size_t sa = ax == 0 ? (size_t)n1 * n2 : (ax == 1 ? (size_t)n2 : 1);
   const size_t sp = ax == 0 ? (size_t)n2 : (size_t)n1 * n2;
   const size_t sq = ax == 2 ? (size_t)n2 : 1;
-  float acc = 0.f;
-  for (int ia = 0; ia < na; ++ia) {
-    const float xa = (float)ia + 0.5f;
-    const float al0 = ma0 * xa + mm[3], al1 = ma1 * xa + mm[7];
-    const float cr0 = 0.5f * (w0lo + w0hi) - al0, cr1 = 0.5f * (w1lo + w1hi) - al1;
-    const float cp = (mq1 * cr0 - mq0 * cr1) / det;
-    const float plo = fmaxf(0.5f, cp - ep - mg), phi = fminf((float)np - 0.5f, cp + ep + mg);
-    if (!(plo <= phi)) continue;
-    const int ip0 = max(0, (int)ceilf(plo - 0.5f)), ip1 = min(np - 1, (int)floorf(phi - 0.5f));
-    for (int ip = ip0; ip <= ip1; ++ip) {
-      const float xp = (float)ip + 0.5f;
-      float qlo = 0.5f, qhi = (float)nq - 0.5f;
-      narrow(al0 + mp0 * xp, mq0, w0lo, w0hi, qlo, qhi);
-      narrow(al1 + mp1 * xp, mq1, w1lo, w1hi, qlo, qhi);
-      if (!(qlo <= qhi)) continue;
-      const int iq0 = max(0, (int)ceilf(qlo - 0.5f - mg)), iq1 = min(nq - 1, (int)floorf(qhi - 0.5f + mg));
-      for (int iq = iq0; iq <= iq1; ++iq) {
-        const int i0 = ax == 0 ? ia : ip;
-        const int i1 = ax == 0 ? ip : (ax == 1 ? ia : iq);
-        const int i2 = ax == 2 ? ia : iq;
-        const float x0 = (float)i0 + 0.5f, x1 = (float)i1 + 0.5f, x2 = (float)i2 + 0.5f;
-        int u0, u1;
-        float t0, t1;
-        edge3(px3(mm[0], mm[1], mm[2], mm[3], x0, x1, x2), u0, t0);
-        edge3(px3(mm[4], mm[5], mm[6], mm[7], x0, x1, x2), u1, t1);
-        const int d0 = r - u0, d1 = c - u1;
-        if ((unsigned)d0 > 1u || (unsigned)d1 > 1u) continue;
-        const float f0 = d0 ? fsub(0.5f, t0) : t0;
-        const float f1 = d1 ? fsub(0.5f, t1) : t1;
-        const float w = fmul(fmul(f0, f1), 4.0f);
-        acc = fmaf(w, __ldg(vol + ia * sa + ip * sp + iq * sq), acc);
+  for (int pix = blockIdx.x * blockDim.x + threadIdx.x; pix < R * C; pix += gridDim.x * blockDim.x) {
+    const int r = pix / C, c = pix - (pix / C) * C;
+    // taps reaching (r, c) come from voxels with floor(left) in {r-1, r} x
+    // {c-1, c}: Px in [r-0.75, r+1.25) x [c-0.75, c+1.25); widened by a margin
+    // far above the rounding of the range arithmetic (the exact test decides)
+    const float mg = 0.05f;
+    const float w0lo = (float)r - 0.75f - mg, w0hi = (float)r + 1.25f + mg;
+    const float w1lo = (float)c - 0.75f - mg, w1hi = (float)c + 1.25f + mg;
+    // |x_p - centre_p| <= e_p from the 2x2 system of the (p, q) plane
+    const float det = mp0 * mq1 - mq0 * mp1;
+    const float h0 = 0.5f * (w0hi - w0lo), h1 = 0.5f * (w1hi - w1lo);
+    const float ep = (fabsf(mq1) * h0 + fabsf(mq0) * h1) / fabsf(det);
+    float acc = 0.f;
+    for (int ia = 0; ia < na; ++ia) {
+      const float xa = (float)ia + 0.5f;
+      const float al0 = ma0 * xa + mm[3], al1 = ma1 * xa + mm[7];
+      const float cr0 = 0.5f * (w0lo + w0hi) - al0, cr1 = 0.5f * (w1lo + w1hi) - al1;
+      const float cp = (mq1 * cr0 - mq0 * cr1) / det;
+      const float plo = fmaxf(0.5f, cp - ep - mg), phi = fminf((float)np - 0.5f, cp + ep + mg);
+      if (!(plo <= phi)) continue;
+      const int ip0 = max(0, (int)ceilf(plo - 0.5f)), ip1 = min(np - 1, (int)floorf(phi - 0.5f));
+      for (int ip = ip0; ip <= ip1; ++ip) {
+        const float xp = (float)ip + 0.5f;
+        float qlo = 0.5f, qhi = (float)nq - 0.5f;
+        narrow(al0 + mp0 * xp, mq0, w0lo, w0hi, qlo, qhi);
+        narrow(al1 + mp1 * xp, mq1, w1lo, w1hi, qlo, qhi);
+        if (!(qlo <= qhi)) continue;
+        const int iq0 = max(0, (int)ceilf(qlo - 0.5f - mg)), iq1 = min(nq - 1, (int)floorf(qhi - 0.5f + mg));
+        for (int iq = iq0; iq <= iq1; ++iq) {
+          const int i0 = ax == 0 ? ia : ip;
+          const int i1 = ax == 0 ? ip : (ax == 1 ? ia : iq);
+          const int i2 = ax == 2 ? ia : iq;
+          const float x0 = (float)i0 + 0.5f, x1 = (float)i1 + 0.5f, x2 = (float)i2 + 0.5f;
+          int u0, u1;
+          float t0, t1;
+          edge3(px3(mm[0], mm[1], mm[2], mm[3], x0, x1, x2), u0, t0);
+          edge3(px3(mm[4], mm[5], mm[6], mm[7], x0, x1, x2), u1, t1);
+          const int d0 = r - u0, d1 = c - u1;
+          if ((unsigned)d0 > 1u || (unsigned)d1 > 1u) continue;
+          const float f0 = d0 ? fsub(0.5f, t0) : t0;
+          const float f1 = d1 ? fsub(0.5f, t1) : t1;
+          const float w = fmul(fmul(f0, f1), 4.0f);
+          acc = fmaf(w, __ldg(vol + ia * sa + ip * sp + iq * sq), acc);
+        }
       }
     }
+    proj[((size_t)v * R + r) * C + c] = acc;
   }
-  proj[((size_t)v * R + r) * C + c] = acc;
 }
 
 __global__ void k_p3_sum_splits(const float* __restrict__ part, float* __restrict__ out, size_t n,
@@ -697,6 +652,7 @@ ct_status proj3d_check(const ct_geom3d* g, const char* who) {
 // adjoint view splits.
 constexpr int kMaxGroups = 8;
 constexpr int kMaxSplits3d = 4;
+constexpr size_t kGenScratch = 96u << 20;  // bytes of GENERAL forward tiles per launch
 
 // The AXIS0 span bounds need max |M[1][1]| and |M[1][2]|; ct_proj3d_views
 // guarantees both <= 1, so the bounds are fixed.
@@ -734,10 +690,44 @@ Proj3dPlan proj3d_plan_sched(const ct_geom3d* g, Sched3d sc) {
     if (ctas < kAdjTargetCtas) ns = (int)((kAdjTargetCtas + ctas - 1) / ctas);
     ns_max = std::max(1, V / 16);
   } else {
-    const double n = (double)S * NJ * NK;
-    const long ctas = (long)((n + 255) / 256);
-    if (ctas < 4L * sms) ns = (int)((4L * sms + ctas - 1) / ctas);
+    // adjoint: the view splits (up to 16, each costs a pass over its partial
+    // volume) with the fewest rounds of the SMs' three CTAs per view
+    const long ctas = (long)((S + kBrick - 1) / kBrick) * ((NJ + kBrick - 1) / kBrick) * ((NK + kBrick - 1) / kBrick);
+    double least = 1e300;
+    for (int k = 1; k <= 16; ++k) {
+      const double cost = std::ceil((double)ctas * k / (3.0 * sms)) / k * (1.0 + 0.02 * (k - 1));
+      if (cost < 0.98 * least) {
+        least = cost;
+        ns = k;
+      }
+    }
     ns_max = std::max(1, V / 8);
+    // the scratch that a call has always needed (a voxel per thread, four CTAs
+    // of 256 an SM); one with no more runs the splits that fit (ct_proj3d_adj)
+    const long old_ctas = (long)(((double)S * NJ * NK + 255) / 256);
+    const int old_ns = std::min(old_ctas < 4L * sms ? (int)((4L * sms + old_ctas - 1) / old_ctas) : 1, ns_max);
+    const int old_per = (V + old_ns - 1) / old_ns, old_split = (V + old_per - 1) / old_per;
+    const int tune = std::max(old_ns, std::min(kMaxSplits3d, ns_max));
+    p.adj_tune = tune > 1 ? round_up(sizeof(float) * (size_t)tune * S * NJ * NK, 256) : 0;
+    p.adj_least = old_split > 1 ? round_up(sizeof(float) * (size_t)old_split * S * NJ * NK, 256) : 0;
+    // forward: windows of a view (bound over the marching axes), plane segments
+    // until two warps a slot are there, views per launch until the tiles of a
+    // launch pass kGenScratch (they are read back from L2)
+    const int n3[3] = {S, NJ, NK};
+    long nwin = 0;
+    for (int ax = 0; ax < 3; ++ax) {
+      const long na = n3[ax], np = n3[ax == 0 ? 1 : 0], nq = n3[ax == 2 ? 1 : 2];
+      nwin = std::max(nwin, ((np + na) / kWin + 2) * ((nq + na) / kWin + 2));
+    }
+    p.nwin = (int)std::min<long>(nwin, 1 << 20);
+    const long warps = std::max(1L, p.nwin / 4L * V), target = 40L * sms;
+    p.nseg = (int)std::min<long>(std::max(1L, (target + warps - 1) / warps),
+                                 std::max(1, std::min(S, std::min(NJ, NK)) / 8));
+    const size_t per_view = sizeof(float) * (size_t)p.nseg * p.nwin * kTilePix;
+    p.gen_views = (int)std::max<size_t>(1, std::min<size_t>(std::min(V, 65535), kGenScratch / per_view));
+    p.gen_plan = round_up(sizeof(GenView) * (size_t)V, 256);
+    p.gen_turn = round_up(sizeof(float) * (size_t)S * NJ * NK, 256);
+    p.fwd_bytes = p.fwd_ws_bytes = p.gen_plan + p.gen_turn + round_up((size_t)p.gen_views * per_view, 256);
   }
   ns = std::min(ns, ns_max);
   const int ns_ws = std::max(ns, std::min(kMaxSplits3d, ns_max));
@@ -746,7 +736,7 @@ Proj3dPlan proj3d_plan_sched(const ct_geom3d* g, Sched3d sc) {
   p.nsplit = (V + p.per_split - 1) / p.per_split;
   p.adj_bytes = p.nsplit > 1 ? round_up(sizeof(float) * (size_t)p.nsplit * S * NJ * NK, 256) : 0;
   p.adj_ws_bytes = ns_ws > 1 ? round_up(sizeof(float) * (size_t)ns_ws * S * NJ * NK, 256) : 0;
-  p.adj_ws_bytes = std::max(p.adj_ws_bytes, p.adj_bytes);
+  p.adj_ws_bytes = std::max(p.adj_ws_bytes, std::max(p.adj_bytes, std::max(p.adj_least, p.adj_tune)));
   return p;
 }
 
@@ -787,7 +777,10 @@ ct_status need_ws(const char* who, size_t need, void* ws, size_t bytes) {
 
 ct_status proj3d_prepare(const ct_geom3d* g, const Proj3dPlan& p) {
   if (!errflag3_ptr()) return fail(CT_ERR_CUDA, "proj3d: error-word address unavailable");
-  if (g->kind != CT_PROJ3D_AXIS0) return CT_OK;
+  if (g->kind != CT_PROJ3D_AXIS0)
+    return cuda_check(cudaFuncSetAttribute(k_p3_gen_windows, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                           (int)(sizeof(float4) * kGenWarps * kSlots)),
+                      "k_p3_gen_windows smem attribute");
   return cuda_check(cudaFuncSetAttribute(k_p3_ax0_fwd, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)p.fwd_smem),
                     "k_p3_ax0_fwd smem attribute");
@@ -824,9 +817,44 @@ ct_status proj3d_fwd_launch(const ct_geom3d* g, const Proj3dPlan& p, const float
                                              g->row_offset, skip);
     return launch_check("k_p3_ax0_rows");
   }
-  dim3 grid((R * C + 255) / 256, V);
-  k_p3_gen_fwd<<<grid, 256, 0, s>>>(vol, proj, g->views, S, NJ, NK, V, R, C, skip);
-  return launch_check("k_p3_gen_fwd");
+  GenView* plan = static_cast<GenView*>(ws);
+  if (ws) {
+    GenFwdArgs a;
+    float* turned = reinterpret_cast<float*>(static_cast<char*>(ws) + p.gen_plan);
+    a.vol = vol;
+    a.vol_t = turned;
+    a.plan = plan;
+    a.part = reinterpret_cast<float*>(static_cast<char*>(ws) + p.gen_plan + p.gen_turn);
+    a.proj = proj;
+    a.n0 = S;
+    a.n1 = NJ;
+    a.n2 = NK;
+    a.R = R;
+    a.C = C;
+    a.nwin = p.nwin;
+    a.nseg = p.nseg;
+    a.skip = skip;
+    const unsigned turn_blocks = (unsigned)((S * (long)NJ + 31) / 32) * (unsigned)((NK + 31) / 32);
+    k_p3_gen_setup<<<(V + 7) / 8 + turn_blocks, 256, 0, s>>>(g->views, plan, vol, turned, S, NJ, NK, V, p.nwin, skip);
+    ct_status st = launch_check("k_p3_gen_setup");
+    if (st != CT_OK) return st;
+    for (a.v0 = 0; a.v0 < V; a.v0 += p.gen_views) {
+      const int nv = std::min(p.gen_views, V - a.v0);
+      const dim3 gw((unsigned)(((long)p.nwin * p.nseg + kGenWarps - 1) / kGenWarps), nv);
+      k_p3_gen_windows<<<gw, kGenWarps * 32, sizeof(float4) * kGenWarps * kSlots, s>>>(a);
+      st = launch_check("k_p3_gen_windows");
+      if (st != CT_OK) return st;
+      const dim3 gg((unsigned)((C + 31) / 32) * (unsigned)((R + kGatherWarps - 1) / kGatherWarps), nv);
+      k_p3_gen_gather<<<gg, kGatherWarps * 32, 0, s>>>(a);
+      st = launch_check("k_p3_gen_gather");
+      if (st != CT_OK) return st;
+    }
+  }
+  // with windows, few blocks a view: most find it taken
+  const int full = (int)(((long)R * C + 255) / 256);
+  dim3 grid(ws ? std::min(full, std::max(16, 16 * sm_count() / V)) : full, V);
+  k_p3_gen_march<<<grid, 256, 0, s>>>(vol, proj, g->views, S, NJ, NK, R, C, plan, skip);
+  return launch_check("k_p3_gen_march");
 }
 
 ct_status proj3d_adj_launch(const ct_geom3d* g, const Proj3dPlan& p, const float* proj, float* out,
@@ -855,7 +883,7 @@ ct_status proj3d_adj_launch(const ct_geom3d* g, const Proj3dPlan& p, const float
     k_p3_ax0_adj<<<grid, 256, 0, s>>>(a);
     return launch_check("k_p3_ax0_adj");
   }
-  dim3 grid((unsigned)((vol_n + 255) / 256), p.nsplit);
+  const dim3 grid((unsigned)((NK + kBrick - 1) / kBrick) * ((NJ + kBrick - 1) / kBrick) * ((S + kBrick - 1) / kBrick), p.nsplit);
   k_p3_gen_adj<<<grid, 256, 0, s>>>(proj, dst, g->views, S, NJ, NK, V, R, C, p.per_split, vol_n,
                                     skip);
   return launch_check("k_p3_gen_adj");
@@ -957,7 +985,10 @@ ct_status ct_proj3d_fwd(const ct_geom3d* g, const float* vol, float* proj, int32
   if (!vol || !proj) return fail(CT_ERR_INVALID_ARG, "ct_proj3d_fwd: null array");
   if (batch <= 0) return fail(CT_ERR_INVALID_ARG, "ct_proj3d_fwd: batch=%d", batch);
   const Proj3dPlan p = proj3d_plan(g, batch);
-  st = need_ws("ct_proj3d_fwd", p.fwd_bytes, workspace, workspace_bytes);
+  if (g->kind == CT_PROJ3D_AXIS0)
+    st = need_ws("ct_proj3d_fwd", p.fwd_bytes, workspace, workspace_bytes);
+  else if (workspace_bytes < p.fwd_bytes || !aligned(workspace, 256))
+    workspace = nullptr;  // GENERAL runs without scratch, slower
   if (st != CT_OK) return st;
   st = proj3d_prepare(g, p);
   if (st != CT_OK) return st;
@@ -978,9 +1009,17 @@ ct_status ct_proj3d_adj(const ct_geom3d* g, const float* proj, float* vol, int32
   if (st != CT_OK) return st;
   if (!vol || !proj) return fail(CT_ERR_INVALID_ARG, "ct_proj3d_adj: null array");
   if (batch <= 0) return fail(CT_ERR_INVALID_ARG, "ct_proj3d_adj: batch=%d", batch);
-  const Proj3dPlan p = proj3d_plan(g, batch);
-  st = need_ws("ct_proj3d_adj", p.adj_bytes, workspace, workspace_bytes);
+  Proj3dPlan p = proj3d_plan(g, batch);
+  st = need_ws("ct_proj3d_adj", g->kind == CT_PROJ3D_AXIS0 ? p.adj_bytes : p.adj_least, workspace, workspace_bytes);
   if (st != CT_OK) return st;
+  if (g->kind != CT_PROJ3D_AXIS0 && (!workspace || workspace_bytes < p.adj_bytes || !aligned(workspace, 256))) {
+    // as many splits as the scratch given holds
+    const size_t one = sizeof(float) * (size_t)g->shape[0] * g->shape[1] * g->shape[2];
+    const bool use = workspace && aligned(workspace, 256);
+    const int ns = std::max(1, (int)std::min<size_t>(p.nsplit, use ? workspace_bytes / one : 1));
+    p.per_split = (g->n_views + ns - 1) / ns;
+    p.nsplit = (g->n_views + p.per_split - 1) / p.per_split;
+  }
   st = proj3d_prepare(g, p);
   if (st != CT_OK) return st;
   cudaStream_t s = as_stream(stream);
@@ -1015,7 +1054,8 @@ ct_status ct_proj3d_autotune(const ct_geom3d* g, float* vol, float* proj, void* 
   if (st != CT_OK) return st;
   if (cap != cudaStreamCaptureStatusNone) return fail(CT_ERR_INVALID_ARG, "%s: cannot measure inside a stream capture", who);
   const Proj3dPlan p0 = proj3d_plan_sched(g, Sched3d{});
-  const size_t need = std::max(p0.fwd_ws_bytes, p0.adj_ws_bytes);
+  // GENERAL tunes the adjoint alone
+  const size_t need = g->kind == CT_PROJ3D_AXIS0 ? std::max(p0.fwd_ws_bytes, p0.adj_ws_bytes) : p0.adj_tune;
   st = need_ws(who, need, workspace, workspace_bytes);
   if (st != CT_OK) return st;
   st = proj3d_prepare(g, p0);
