@@ -64,7 +64,8 @@ struct Proj3dPlan {
   size_t gen_plan = 0, gen_turn = 0;  // bytes of the views' plans and of the turned volume
   // adjoint view splits (both kinds)
   int nsplit = 1, per_split = 0;
-  size_t adj_least = 0, adj_tune = 0;  // GENERAL: scratch below which an adjoint / its tuning is refused
+  int adj_sl = 4;        // AXIS0 adjoint: slices a lane
+  size_t adj_least = 0, adj_tune = 0;  // scratch below which an adjoint / its tuning is refused
   size_t fwd_bytes = 0, adj_bytes = 0;
   // the same for the largest tile-group / split counts a schedule may use
   // (workspaces sized with these stay valid after ct_proj3d_autotune)

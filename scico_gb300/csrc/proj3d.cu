@@ -25,10 +25,9 @@
 //               slice of a [group][view][col][slice] accumulator in global
 //               memory (old values loaded three bins ahead), which
 //               k_p3_ax0_rows transposes into the sinogram.
-//      adjoint  k_p3_ax0_adj: lanes = pixels along axis 2, 32 slices of
-//               accumulators per thread; the view's detector rows of the
-//               CTA's slices are staged as (y[c], y[c+1]) pairs, read with
-//               one 8-byte shared load per slice.
+//      adjoint  k_p3_ax0_adj: lanes = slices (up to four each), a warp owns
+//               4x4 pixels; the view's detector columns are staged as
+//               [column][slice] and kept in registers from pixel to pixel.
 //  * GENERAL -- any matrices: proj3d_gen.cuh.
 #include <algorithm>
 #include <cmath>
@@ -50,8 +49,6 @@ constexpr int kSvStride = 66;   // shared [pixel][slice] row stride (floats, eve
 constexpr int kWalkGroup = 8;   // walk entries whose loads are issued together
 constexpr int kFwdViewsPerCta = 16;
 constexpr int kFwdViewsPerWarp = kFwdViewsPerCta / 8;
-constexpr int kAdjRows = 16;  // AXIS0 adjoint tile: 16 (axis 1) x 32 (axis 2) pixels
-constexpr int kAdjTargetCtas = 304;
 
 static_assert(kTileJ * kTileK == kOrd, "order table covers one tile");
 
@@ -92,6 +89,10 @@ __device__ __forceinline__ void cp_async4(uint32_t dst, const float* src, bool v
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src),
                "r"(valid ? 4 : 0)
                : "memory");
+}
+
+__device__ __forceinline__ void cp_async4_all(uint32_t dst, const float* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
 }
 
 __device__ __forceinline__ void cp_async_wait_all() {
@@ -377,139 +378,261 @@ __global__ void k_p3_ax0_rows(const float* __restrict__ acc, float* __restrict__
 }
 
 // ---------------------------------------------------------------------------
-// AXIS0 adjoint
+// AXIS0 adjoint.  A CTA owns 16 x 16 pixels and 32 SL slices, a warp 4 x 4 of
+// the pixels with SL slices a lane: 16 SL accumulators in registers.  The
+// views' detector windows are staged as [column][slice] (rows of 32 SL + 4
+// floats: the transposing copies of 8 columns x 4 slices a warp hit 32 banks,
+// a warp reads a row in 16-byte pieces without conflicts), kAdjViews views per
+// barrier, the next ones copied meanwhile.  A pixel takes the rows of its two
+// columns for all its slices.  Even rows live in one set of registers and odd
+// rows in another, each reloaded only when a pixel needs another row, and the
+// 4 x 4 pixels are visited back and forth along the axis whose step on the
+// detector is the smaller: about half of the pixels load one row, some 2 bytes
+// of shared reads per interaction instead of the 8 of one (y[c], y[c+1]) pair
+// each, which bound the version before (lane = pixel, 32 slices of
+// accumulators).  Weights and row offsets come from a table that a warp makes
+// for its pixels, half a warp per view.  256^3 x 360 views: 2258 -> 1544 us (two view
+// splits), of issue slots (19 a pixel and view) and shared reads alike.
 // ---------------------------------------------------------------------------
+constexpr int kAdjTile = 16;   // tile edge (pixels)
+constexpr int kAdjCols = 40;   // staged columns: 15 (|m11| + |m12|) + 6 for |m| <= 1, whole copies of 8
+constexpr int kAdjViews = 4;   // views per barrier
+constexpr int kAdjWarps = 16;
+constexpr int kAdjChunk3 = 512;  // views whose windows are laid out at once
+
 struct Ax0AdjArgs {
   const float* proj;  // (V, R, C)
   float* out;         // (S, NJ, NK), or split partials
   const float* views;
   int S, NJ, NK, V, R, C, row_offset;
+  int tiles_k, nsg;   // tiles along axis 2, slice groups
   int per_split;
   size_t split_stride;
   int* errflag;
   const double* skip;
 };
 
-// staged detector columns per slice row of the 16 x 32 adjoint tile:
-// 15|m11| + 31|m12| + 5 <= 51 for |m11|, |m12| <= 1
-constexpr int kAW = (kAdjRows - 1) + 31 + 6;
-constexpr int kAdjStage = (32 * kAW + 255) / 256;  // staging slots per thread
-
-__device__ __forceinline__ float2 ld_shared_f2(uint32_t addr) {
-  float2 v;
-  asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(addr));
-  return v;
+__host__ __device__ constexpr int adj_row(int SL) { return 32 * SL + 4; }  // floats of a staged column
+constexpr size_t adj3_smem(int SL) {
+  return sizeof(float) * 2 * kAdjViews * kAdjCols * adj_row(SL) +
+         (sizeof(float2) + sizeof(unsigned)) * kAdjWarps * kAdjViews * 16 + (sizeof(float4) + sizeof(int)) * kAdjChunk3;
 }
 
-// Window [lo, lo + nb) of detector columns that the 16x32 tile at (j0, k0)
-// reads in one view (corner bound as tile_bins, two extra columns above).
+// Window [lo, lo + nb) of detector columns that the tile at (j0, k0) reads in
+// one view: every operation of the rounded Px is monotone in each pixel index,
+// so the extremes are at corners (one column spare below, two above).
 __device__ __forceinline__ void adj_window(float m11, float m12, float m13, int j0, int k0,
                                            int& lo, int& nb) {
-  const float ja = (float)j0 + 0.5f, jb = (float)(j0 + kAdjRows - 1) + 0.5f;
-  const float ka = (float)k0 + 0.5f, kb = (float)(k0 + 31) + 0.5f;
+  const float ja = (float)j0 + 0.5f, jb = (float)(j0 + kAdjTile - 1) + 0.5f;
+  const float ka = (float)k0 + 0.5f, kb = (float)(k0 + kAdjTile - 1) + 0.5f;
   const float a0 = fmul(m11, ja), a1 = fmul(m11, jb), b0 = fmul(m12, ka), b1 = fmul(m12, kb);
   lo = (int)floorf(fadd(fminf(a0, a1) + fminf(b0, b1), m13) - 0.25f) - 1;
   nb = (int)floorf(fadd(fmaxf(a0, a1) + fmaxf(b0, b1), m13) - 0.25f) + 3 - lo;
 }
 
-__global__ void __launch_bounds__(256, 2) k_p3_ax0_adj(const Ax0AdjArgs a) {
-  if (a.skip && *a.skip != 0.0) return;
-  // [2][32][kAW] pairs (y[c], y[c+1]) of the slice rows, double-buffered
-  __shared__ __align__(16) float2 sy[2 * 32 * kAW];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int k0 = blockIdx.x * 32, j0 = blockIdx.y * kAdjRows;
-  const int nsg = (a.S + 31) / 32;
-  const int sg = blockIdx.z % nsg, split = blockIdx.z / nsg;
-  const int i0 = sg * 32;
-  const int k = k0 + lane;
-  const int jj[2] = {j0 + warp, j0 + warp + 8};
-  const int vs = split * a.per_split, ve = min(a.V, vs + a.per_split);
-  const uint32_t sbase = (uint32_t)__cvta_generic_to_shared(sy);
-
-  // issue the copies of view v's window into buffer `buf`
-  auto stage = [&](int v, int buf, int lo, int nb) {
-    const float* src = a.proj + (size_t)v * a.R * a.C;
+// SL floats a lane of a staged column.
+template <int SL>
+struct AdjVec {
+  float p[SL];
+  // the row at `at`, when it is not the one held
+  __device__ __forceinline__ void reload(uint32_t at, uint32_t held) {
+    if constexpr (SL == 4)
+      asm volatile("{\n.reg .pred p;\nsetp.ne.u32 p, %4, %5;\n@p ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];\n}"
+                   : "+f"(p[0]), "+f"(p[1]), "+f"(p[2]), "+f"(p[3])
+                   : "r"(at), "r"(held));
+    else if constexpr (SL == 2)
+      asm volatile("{\n.reg .pred p;\nsetp.ne.u32 p, %2, %3;\n@p ld.shared.v2.f32 {%0, %1}, [%2];\n}"
+                   : "+f"(p[0]), "+f"(p[1])
+                   : "r"(at), "r"(held));
+    else
+      asm volatile("{\n.reg .pred p;\nsetp.ne.u32 p, %1, %2;\n@p ld.shared.f32 %0, [%1];\n}"
+                   : "+f"(p[0])
+                   : "r"(at), "r"(held));
+  }
+  __device__ __forceinline__ void fma(float w, const AdjVec& y) {
 #pragma unroll
-    for (int it = 0; it < kAdjStage; ++it) {
-      const int e = tid + 256 * it;
-      if (e < 32 * kAW) {
-        const int s = e / kAW, bl = e - s * kAW;
-        const int r = i0 + s + a.row_offset, c = lo + bl;
-        const bool row_ok = bl < nb && i0 + s < a.S && r >= 0 && r < a.R;
-        const float* row = src + (size_t)(row_ok ? r : 0) * a.C;
-        const bool ok0 = row_ok && c >= 0 && c < a.C;
-        const bool ok1 = row_ok && c + 1 >= 0 && c + 1 < a.C;
-        const uint32_t d = sbase + (uint32_t)(buf * 32 * kAW + e) * 8u;
-        cp_async4(d, ok0 ? row + c : a.proj, ok0);
-        cp_async4(d + 4, ok1 ? row + c + 1 : a.proj, ok1);
+    for (int i = 0; i < SL; ++i) p[i] = fmaf(w, y.p[i], p[i]);
+  }
+  __device__ __forceinline__ void zero() {
+#pragma unroll
+    for (int i = 0; i < SL; ++i) p[i] = 0.0f;
+  }
+  __device__ __forceinline__ void store(float* o) const {
+#pragma unroll
+    for (int i = 0; i < SL; ++i) o[i] = p[i];
+  }
+};
+
+// Position t of a visit of the 4 x 4 pixels: back and forth along axis 2
+// (COL = false) or axis 1; returns 4 (axis-1 offset) + (axis-2 offset).
+template <bool COL>
+__host__ __device__ constexpr int visit(int t) {
+  const int o = t >> 2, i = (o & 1) ? 3 - (t & 3) : (t & 3);
+  return COL ? 4 * i + o : 4 * o + i;
+}
+
+template <int SL, bool COL>
+__device__ __forceinline__ void adj_view(const float2* wt, const uint2* ot, uint32_t base, AdjVec<SL> (&acc)[16]) {
+  AdjVec<SL> ye, yo;
+  ye.zero();
+  yo.zero();
+  uint32_t he = 0xffffffffu, ho = 0xffffffffu;
+#pragma unroll
+  for (int t = 0; t < 16; t += 2) {
+    const uint2 o = ot[t / 2];  // two pixels: offset of the even row, of the odd row (16 bits each)
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const float2 w = wt[t + h];  // their weights
+      const uint32_t oh = h ? o.y : o.x;
+      const uint32_t ae = base + (oh & 0xffffu), ao = base + (oh >> 16);
+      ye.reload(ae, he);
+      yo.reload(ao, ho);
+      he = ae;
+      ho = ao;
+      AdjVec<SL>& a = acc[visit<COL>(t + h)];
+      a.fma(w.x, ye);
+      a.fma(w.y, yo);
+    }
+  }
+}
+
+// grid = (tiles, slice groups x splits), block = 512.
+template <int SL>
+__global__ void __launch_bounds__(kAdjWarps * 32, 1) k_p3_ax0_adj(const Ax0AdjArgs a) {
+  if (a.skip && *a.skip != 0.0) return;
+  extern __shared__ __align__(16) float smem[];
+  constexpr int kRow = adj_row(SL), kBuf = kAdjViews * kAdjCols * kRow;
+  float2* wtab = reinterpret_cast<float2*>(smem + 2 * kBuf);  // [warp][view][16] weight of the even row, of the odd row
+  unsigned* otab = reinterpret_cast<unsigned*>(wtab + kAdjWarps * kAdjViews * 16);  // [warp][view][16] byte offsets
+  float4* vtab = reinterpret_cast<float4*>(otab + kAdjWarps * kAdjViews * 16);  // M[1][1..3], first column
+  int* ntab = reinterpret_cast<int*>(vtab + kAdjChunk3);                // columns
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int j0 = (blockIdx.x / a.tiles_k) * kAdjTile, k0 = (blockIdx.x % a.tiles_k) * kAdjTile;
+  const int sg = blockIdx.y % a.nsg, split = blockIdx.y / a.nsg;
+  const int i0 = sg * 32 * SL;
+  const int vs = split * a.per_split, ve = min(a.V, vs + a.per_split);
+  const uint32_t sbase = (uint32_t)__cvta_generic_to_shared(smem);
+
+  // staging: lane = 8 columns x 4 slices; a warp takes the slice quads
+  // warp, warp + 16, ..
+  const int c8 = lane & 7, s4 = lane >> 3;
+  constexpr int kQuads = (8 * SL + kAdjWarps - 1) / kAdjWarps;
+  const bool has = 8 * SL >= kAdjWarps || 4 * warp < 32 * SL;
+  bool rows_ok = true;
+  bool row_ok[kQuads];
+  const float* row[kQuads];
+#pragma unroll
+  for (int q = 0; q < kQuads; ++q) {
+    const int s = 4 * (warp + kAdjWarps * q) + s4, r = i0 + s + a.row_offset;
+    row_ok[q] = has && i0 + s < a.S && r >= 0 && r < a.R;
+    rows_ok = rows_ok && row_ok[q];
+    row[q] = a.proj + (size_t)(row_ok[q] ? r : 0) * a.C + c8;
+  }
+  rows_ok = __all_sync(0xffffffffu, rows_ok);
+  const uint32_t dst0 = sbase + 4u * (uint32_t)(c8 * kRow + 4 * warp + s4);
+  auto stage = [&](int v, int slot, int lo, int nb) {
+    const uint32_t d = dst0 + 4u * (uint32_t)(slot * kAdjCols * kRow);
+    const ptrdiff_t off = (ptrdiff_t)v * a.R * a.C + lo;
+    if (rows_ok && lo >= 0 && lo + 8 * ((nb + 7) / 8) <= a.C) {  // warp-uniform: every copy reads
+#pragma unroll
+      for (int q = 0; q < kQuads; ++q) {
+        const float* src = row[q] + off;
+#pragma unroll
+        for (int g = 0; g < kAdjCols / 8; ++g)
+          if (8 * g < nb) cp_async4_all(d + 4u * (uint32_t)(8 * g * kRow + 4 * kAdjWarps * q), src + 8 * g);
+      }
+    } else if (has) {
+#pragma unroll
+      for (int q = 0; q < kQuads; ++q) {
+#pragma unroll
+        for (int g = 0; g < kAdjCols / 8; ++g)
+          if (8 * g < nb) {
+            const bool ok = row_ok[q] && (unsigned)(lo + 8 * g + c8) < (unsigned)a.C;
+            cp_async4(d + 4u * (uint32_t)(8 * g * kRow + 4 * kAdjWarps * q), ok ? row[q] + off + 8 * g : a.proj, ok);
+          }
       }
     }
   };
 
-  float acc[2][32];
+  AdjVec<SL> acc[16];
 #pragma unroll
-  for (int q = 0; q < 2; ++q)
-#pragma unroll
-    for (int s = 0; s < 32; ++s) acc[q][s] = 0.f;
+  for (int p = 0; p < 16; ++p) acc[p].zero();
+  const int jw = j0 + 4 * (warp >> 2), kw = k0 + 4 * (warp & 3);
+  float2* wt = wtab + warp * kAdjViews * 16;
+  unsigned* ot = otab + warp * kAdjViews * 16;
 
-  int lo = 0, nb = 0;
-  if (vs < ve) {
-    const float* m = a.views + (size_t)vs * kVT;
-    adj_window(m[5], m[6], m[7], j0, k0, lo, nb);
-    stage(vs, 0, lo, min(nb, kAW));
-    cp_async_wait_all();
-  }
-  __syncthreads();
-  for (int v = vs; v < ve; ++v) {
-    const int buf = (v - vs) & 1;
-    const float* m = a.views + (size_t)v * kVT;
-    const float m11 = m[5], m12 = m[6], m13 = m[7];
-    if (nb > kAW && tid == 0) atomicOr(a.errflag, 2);  // cannot happen for |m| <= 1
-    const int nbc = min(nb, kAW);
-    // next view's copies run while this view is computed
-    int lo_n = 0, nb_n = 0;
-    if (v + 1 < ve) {
-      const float* mn = a.views + (size_t)(v + 1) * kVT;
-      adj_window(mn[5], mn[6], mn[7], j0, k0, lo_n, nb_n);
-      stage(v + 1, buf ^ 1, lo_n, min(nb_n, kAW));
+  for (int vc = vs; vc < ve; vc += kAdjChunk3) {
+    const int nc = min(kAdjChunk3, ve - vc);
+    for (int u = tid; u < nc; u += kAdjWarps * 32) {
+      const float* m = a.views + (size_t)(vc + u) * kVT;
+      int lo, nb;
+      adj_window(m[5], m[6], m[7], j0, k0, lo, nb);
+      if (nb > kAdjCols) atomicOr(a.errflag, 2);  // cannot happen for |m| <= 1
+      vtab[u] = make_float4(m[5], m[6], m[7], __int_as_float(lo));
+      ntab[u] = min(nb, kAdjCols);
     }
-    const uint32_t vbase = sbase + (uint32_t)(buf * 32 * kAW) * 8u;
+    __syncthreads();
+    auto stage_batch = [&](int c, int buf) {
 #pragma unroll
-    for (int q = 0; q < 2; ++q) {
-      const float x1 = (float)jj[q] + 0.5f, x2 = (float)k + 0.5f;
-      const float px = fadd(fadd(fmul(m11, x1), fmul(m12, x2)), m13);
-      int ul;
-      float t1;
-      edge3(px, ul, t1);
-      float w0 = (ul >= 0 && ul < a.C) ? fmul(2.0f, t1) : 0.0f;
-      float w1 = (ul + 1 >= 0 && ul + 1 < a.C) ? fmul(2.0f, fsub(0.5f, t1)) : 0.0f;
-      int rel = ul - lo;
-      if (rel < 0 || rel >= nbc - 1) {  // outside the staged window (cannot happen)
-        rel = 0;
-        w0 = 0.f;
-        w1 = 0.f;
-      }
-      const uint32_t addr = vbase + (uint32_t)rel * 8u;
-#pragma unroll
-      for (int s = 0; s < 32; ++s) {
-        const float2 y = ld_shared_f2(addr + (uint32_t)(s * kAW * 8));
-        acc[q][s] = fmaf(w0, y.x, acc[q][s]);
-        acc[q][s] = fmaf(w1, y.y, acc[q][s]);
-      }
-    }
+      for (int u = 0; u < kAdjViews; ++u)
+        if (c + u < nc) stage(vc + c + u, buf * kAdjViews + u, __float_as_int(vtab[c + u].w), ntab[c + u]);
+    };
+    stage_batch(0, 0);
     cp_async_wait_all();
     __syncthreads();
-    lo = lo_n;
-    nb = nb_n;
-  }
-  float* out = a.out + (size_t)split * a.split_stride;
+    int buf = 0;
+    for (int c = 0; c < nc; c += kAdjViews, buf ^= 1) {
+      if (c + kAdjViews < nc) stage_batch(c + kAdjViews, buf ^ 1);
+      const int nv = min(kAdjViews, nc - c);
+      // weights and rows of the warp's pixels in visiting order, two views at
+      // a time (half a warp each)
 #pragma unroll
-  for (int q = 0; q < 2; ++q) {
-    if (jj[q] >= a.NJ || k >= a.NK) continue;
-#pragma unroll
-    for (int s = 0; s < 32; ++s) {
-      if (i0 + s < a.S) out[((size_t)(i0 + s) * a.NJ + jj[q]) * a.NK + k] = acc[q][s];
+      for (int u = 0; u < kAdjViews; u += 2) {
+        const int vu = u + (lane >> 4), t = lane & 15;
+        if (vu < nv) {
+          const float4 m = vtab[c + vu];
+          const int p = fabsf(m.y) > fabsf(m.x) ? visit<true>(t) : visit<false>(t);
+          const float x1 = (float)(jw + (p >> 2)) + 0.5f, x2 = (float)(kw + (p & 3)) + 0.5f;
+          const float px = fadd(fadd(fmul(m.x, x1), fmul(m.y, x2)), m.z);
+          int ul;
+          float t1;
+          edge3(px, ul, t1);
+          // columns off the detector are staged as zeros; inside the window
+          // by the corner bound
+          const int rel = min(max(ul - __float_as_int(m.w), 0), ntab[c + vu] - 2), odd = rel & 1;
+          const float w0 = fmul(2.0f, t1), w1 = fmul(2.0f, fsub(0.5f, t1));
+          wt[16 * vu + t] = make_float2(odd ? w1 : w0, odd ? w0 : w1);
+          ot[16 * vu + t] = (unsigned)((rel + odd) * kRow * 4) | (unsigned)((rel + 1 - odd) * kRow * 4) << 16;
+        }
+      }
+      __syncwarp();
+      const uint32_t vb = sbase + 4u * (uint32_t)(buf * kBuf) + 4u * SL * (uint32_t)lane;
+#pragma unroll 1
+      for (int u = 0; u < nv; ++u) {
+        const float4 m = vtab[c + u];
+        const uint32_t base = vb + 4u * (uint32_t)(u * kAdjCols * kRow);
+        if (fabsf(m.y) > fabsf(m.x))
+          adj_view<SL, true>(wt + 16 * u, reinterpret_cast<const uint2*>(ot + 16 * u), base, acc);
+        else
+          adj_view<SL, false>(wt + 16 * u, reinterpret_cast<const uint2*>(ot + 16 * u), base, acc);
+      }
+      cp_async_wait_all();
+      __syncthreads();
     }
+  }
+  // the accumulators through shared memory, [pixel][slice], so that the rows
+  // along axis 2 are written whole
+#pragma unroll
+  for (int p = 0; p < 16; ++p) {
+    const int pix = (4 * (warp >> 2) + (p >> 2)) * kAdjTile + 4 * (warp & 3) + (p & 3);
+    acc[p].store(smem + pix * kRow + SL * lane);
+  }
+  __syncthreads();
+  float* out = a.out + (size_t)split * a.split_stride;
+  for (int e = tid; e < 32 * SL * kAdjTile * kAdjTile; e += kAdjWarps * 32) {
+    const int k = e & 15, j = (e >> 4) & 15, s = e >> 8;
+    if (i0 + s < a.S && j0 + j < a.NJ && k0 + k < a.NK)
+      out[((size_t)(i0 + s) * a.NJ + j0 + j) * a.NK + k0 + k] = smem[(j * kAdjTile + k) * kRow + s];
   }
 }
 
@@ -662,6 +785,15 @@ Proj3dPlan proj3d_plan_sched(const ct_geom3d* g, Sched3d sc) {
   const int C = g->det_shape[1];
   const int sms = std::max(1, sm_count());
   int ns = 1, ns_max = 1;
+  // adjoint scratch below which a call (old_ns splits) and its tuning (the
+  // splits that it tries) have always been refused
+  auto least_scratch = [&](int old_ns, int tried) {
+    const size_t one = sizeof(float) * (size_t)S * NJ * NK;
+    const int eff = sc.ns > 0 ? std::min(sc.ns, ns_max) : old_ns;
+    const int per = (V + eff - 1) / eff, split = (V + per - 1) / per, tune = std::max(old_ns, tried);
+    p.adj_least = split > 1 ? round_up((size_t)split * one, 256) : 0;
+    p.adj_tune = tune > 1 ? round_up((size_t)tune * one, 256) : 0;
+  };
   if (g->kind == CT_PROJ3D_AXIS0) {
     p.Spad = (S + kFwdSlices - 1) / kFwdSlices * kFwdSlices;
     p.tiles_k = (NK + kTileK - 1) / kTileK;
@@ -686,9 +818,32 @@ Proj3dPlan proj3d_plan_sched(const ct_geom3d* g, Sched3d sc) {
     p.fwd_smem = sizeof(float) * (size_t)kOrd * kSvStride + sizeof(float2) * 8 * kOrd;
     p.fwd_bytes = round_up(sizeof(float) * (size_t)p.G * V * C * p.Spad, 256);
     p.fwd_ws_bytes = round_up(sizeof(float) * (size_t)g_max * V * C * p.Spad, 256);
-    const long ctas = (long)((NK + 31) / 32) * ((NJ + kAdjRows - 1) / kAdjRows) * (p.Spad / 32);
-    if (ctas < kAdjTargetCtas) ns = (int)((kAdjTargetCtas + ctas - 1) / ctas);
+    // adjoint: slices a lane (SL) and view splits by the time of the busiest SM,
+    // in units of a CTA's view: 1 at SL = 4, 0.62 and 0.42 at 2 and 1 (the
+    // per-pixel work is shared by fewer slices); a split costs a pass over
+    // its partial volume
+    const long tiles = (long)((NK + kAdjTile - 1) / kAdjTile) * ((NJ + kAdjTile - 1) / kAdjTile);
+    auto cost = [&](int sl, int k) {
+      const long ctas = tiles * ((S + 32 * sl - 1) / (32 * sl));
+      return std::ceil((double)ctas * k / sms) * (sl == 4 ? 1.0 : (sl == 2 ? 0.62 : 0.42)) / k * (k > 1 ? 1.0 + 4.0 * (k + 0.5) / V : 1.0);
+    };
+    auto lanes = [&](int k) { return cost(4, k) <= std::min(cost(2, k), cost(1, k)) ? 4 : (cost(2, k) <= cost(1, k) ? 2 : 1); };
+    const int most = std::max(1, V / (2 * kAdjViews));
+    double least = 1e300;
+    for (int k = 1; k <= std::min(16, most); ++k) {
+      const double c = cost(lanes(k), k);
+      if (c < 0.98 * least) {
+        least = c;
+        ns = k;
+      }
+    }
+    p.adj_sl = lanes(sc.ns > 0 ? std::min(sc.ns, most) : ns);
     ns_max = std::max(1, V / 16);
+    // the scratch that a call has always needed (32 x 16 pixel tiles of 32 slices)
+    const long old_ctas = (long)((NK + 31) / 32) * ((NJ + 15) / 16) * (p.Spad / 32);
+    const int old_ns = std::min(old_ctas < 304 ? (int)((304 + old_ctas - 1) / old_ctas) : 1, ns_max);
+    least_scratch(old_ns, std::min(kMaxSplits3d, ns_max));
+    ns_max = most;
   } else {
     // adjoint: the view splits (up to 16, each costs a pass over its partial
     // volume) with the fewest rounds of the SMs' three CTAs per view
@@ -706,10 +861,7 @@ Proj3dPlan proj3d_plan_sched(const ct_geom3d* g, Sched3d sc) {
     // of 256 an SM); one with no more runs the splits that fit (ct_proj3d_adj)
     const long old_ctas = (long)(((double)S * NJ * NK + 255) / 256);
     const int old_ns = std::min(old_ctas < 4L * sms ? (int)((4L * sms + old_ctas - 1) / old_ctas) : 1, ns_max);
-    const int old_per = (V + old_ns - 1) / old_ns, old_split = (V + old_per - 1) / old_per;
-    const int tune = std::max(old_ns, std::min(kMaxSplits3d, ns_max));
-    p.adj_tune = tune > 1 ? round_up(sizeof(float) * (size_t)tune * S * NJ * NK, 256) : 0;
-    p.adj_least = old_split > 1 ? round_up(sizeof(float) * (size_t)old_split * S * NJ * NK, 256) : 0;
+    least_scratch(old_ns, std::min(kMaxSplits3d, ns_max));
     // forward: windows of a view (bound over the marching axes), plane segments
     // until two warps a slot are there, views per launch until the tiles of a
     // launch pass kGenScratch (they are read back from L2)
@@ -781,9 +933,14 @@ ct_status proj3d_prepare(const ct_geom3d* g, const Proj3dPlan& p) {
     return cuda_check(cudaFuncSetAttribute(k_p3_gen_windows, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                            (int)(sizeof(float4) * kGenWarps * kSlots)),
                       "k_p3_gen_windows smem attribute");
-  return cuda_check(cudaFuncSetAttribute(k_p3_ax0_fwd, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)p.fwd_smem),
-                    "k_p3_ax0_fwd smem attribute");
+  auto raise = [](auto* kernel, size_t bytes, const char* what) {
+    return cuda_check(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes), what);
+  };
+  ct_status st = raise(k_p3_ax0_adj<4>, adj3_smem(4), "k_p3_ax0_adj smem attribute");
+  if (st == CT_OK) st = raise(k_p3_ax0_adj<2>, adj3_smem(2), "k_p3_ax0_adj smem attribute");
+  if (st == CT_OK) st = raise(k_p3_ax0_adj<1>, adj3_smem(1), "k_p3_ax0_adj smem attribute");
+  if (st == CT_OK) st = raise(k_p3_ax0_fwd, p.fwd_smem, "k_p3_ax0_fwd smem attribute");
+  return st;
 }
 
 ct_status proj3d_fwd_launch(const ct_geom3d* g, const Proj3dPlan& p, const float* vol, float* proj,
@@ -875,12 +1032,19 @@ ct_status proj3d_adj_launch(const ct_geom3d* g, const Proj3dPlan& p, const float
     a.R = R;
     a.C = C;
     a.row_offset = g->row_offset;
+    a.tiles_k = (NK + kAdjTile - 1) / kAdjTile;
+    a.nsg = (S + 32 * p.adj_sl - 1) / (32 * p.adj_sl);
     a.per_split = p.per_split;
     a.split_stride = vol_n;
     a.errflag = errflag3_ptr();
     a.skip = skip;
-    dim3 grid((NK + 31) / 32, (NJ + kAdjRows - 1) / kAdjRows, ((S + 31) / 32) * p.nsplit);
-    k_p3_ax0_adj<<<grid, 256, 0, s>>>(a);
+    const dim3 grid((unsigned)a.tiles_k * ((NJ + kAdjTile - 1) / kAdjTile), a.nsg * p.nsplit);
+    if (p.adj_sl == 4)
+      k_p3_ax0_adj<4><<<grid, kAdjWarps * 32, adj3_smem(4), s>>>(a);
+    else if (p.adj_sl == 2)
+      k_p3_ax0_adj<2><<<grid, kAdjWarps * 32, adj3_smem(2), s>>>(a);
+    else
+      k_p3_ax0_adj<1><<<grid, kAdjWarps * 32, adj3_smem(1), s>>>(a);
     return launch_check("k_p3_ax0_adj");
   }
   const dim3 grid((unsigned)((NK + kBrick - 1) / kBrick) * ((NJ + kBrick - 1) / kBrick) * ((S + kBrick - 1) / kBrick), p.nsplit);
@@ -1010,9 +1174,9 @@ ct_status ct_proj3d_adj(const ct_geom3d* g, const float* proj, float* vol, int32
   if (!vol || !proj) return fail(CT_ERR_INVALID_ARG, "ct_proj3d_adj: null array");
   if (batch <= 0) return fail(CT_ERR_INVALID_ARG, "ct_proj3d_adj: batch=%d", batch);
   Proj3dPlan p = proj3d_plan(g, batch);
-  st = need_ws("ct_proj3d_adj", g->kind == CT_PROJ3D_AXIS0 ? p.adj_bytes : p.adj_least, workspace, workspace_bytes);
+  st = need_ws("ct_proj3d_adj", p.adj_least, workspace, workspace_bytes);
   if (st != CT_OK) return st;
-  if (g->kind != CT_PROJ3D_AXIS0 && (!workspace || workspace_bytes < p.adj_bytes || !aligned(workspace, 256))) {
+  if (p.nsplit > 1 && (!workspace || workspace_bytes < p.adj_bytes || !aligned(workspace, 256))) {
     // as many splits as the scratch given holds
     const size_t one = sizeof(float) * (size_t)g->shape[0] * g->shape[1] * g->shape[2];
     const bool use = workspace && aligned(workspace, 256);
@@ -1055,7 +1219,7 @@ ct_status ct_proj3d_autotune(const ct_geom3d* g, float* vol, float* proj, void* 
   if (cap != cudaStreamCaptureStatusNone) return fail(CT_ERR_INVALID_ARG, "%s: cannot measure inside a stream capture", who);
   const Proj3dPlan p0 = proj3d_plan_sched(g, Sched3d{});
   // GENERAL tunes the adjoint alone
-  const size_t need = g->kind == CT_PROJ3D_AXIS0 ? std::max(p0.fwd_ws_bytes, p0.adj_ws_bytes) : p0.adj_tune;
+  const size_t need = g->kind == CT_PROJ3D_AXIS0 ? std::max(p0.fwd_ws_bytes, p0.adj_tune) : p0.adj_tune;
   st = need_ws(who, need, workspace, workspace_bytes);
   if (st != CT_OK) return st;
   st = proj3d_prepare(g, p0);
