@@ -56,9 +56,9 @@ ct_status proj2d_adj_launch(const ct_geom2d* g, const Proj2dPlan& p, const float
 
 // ---- 3D projector (proj3d.cu) ---------------------------------------------
 struct Proj3dPlan {
-  // AXIS0 forward: slices padded to the CTA's 64, tiles, tile groups, views per CTA
-  int Spad = 0, tiles_k = 0, n_tiles = 0, G = 1, vpc = 16;
-  size_t fwd_smem = 0;
+  // AXIS0 forward: slices padded to 64, tiles, tile groups, slices a lane
+  // and warps (views) a CTA
+  int Spad = 0, tiles_k = 0, n_tiles = 0, G = 1, fwd_sl = 4, fwd_nw = 16;
   // GENERAL forward: windows of a view (bound), segments of the planes, views per launch
   int nwin = 0, nseg = 1, gen_views = 1;
   size_t gen_plan = 0, gen_turn = 0;  // bytes of the views' plans and of the turned volume
@@ -67,6 +67,7 @@ struct Proj3dPlan {
   int adj_sl = 4;        // AXIS0 adjoint: slices a lane
   size_t adj_least = 0, adj_tune = 0;  // scratch below which an adjoint / its tuning is refused
   size_t fwd_bytes = 0, adj_bytes = 0;
+  size_t fwd_least = 0;  // AXIS0: forward scratch below which a call is refused
   // the same for the largest tile-group / split counts a schedule may use
   // (workspaces sized with these stay valid after ct_proj3d_autotune)
   size_t fwd_ws_bytes = 0, adj_ws_bytes = 0;

@@ -17,23 +17,26 @@
 //    i + row_offset with t0 = 0.5.  Then ul = 2*t1, ll = 2*(0.5-t1) (both
 //    exact) and the two other taps are zero, and the column weights of pixel
 //    (i1, i2) are the same for every slice.  The kernels compute each column
-//    weight once per view and tile and apply it to 32 slices at a time:
-//      forward  k_p3_ax0_fwd: lanes = slice pairs; a warp walks a 16x16 pixel
-//               tile (staged in shared memory, [pixel][slice]) in the per-view
-//               detector order of the order table, carrying the two open bins
-//               in registers; each completed bin is added into the warp's own
-//               slice of a [group][view][col][slice] accumulator in global
-//               memory (old values loaded three bins ahead), which
-//               k_p3_ax0_rows transposes into the sinogram.
+//    weight once per view and tile and apply it to up to 128 slices at a time:
+//      forward  k_p3_ax0_fwd: lanes = slices (up to four each); a warp walks a
+//               16x16 pixel tile (staged in shared memory, [pixel][slice]) in
+//               the per-view detector order of the order table, carrying the
+//               two open bins in registers; each completed bin is added into
+//               the warp's own slices of a [group][view][col][slice]
+//               accumulator in global memory (old values loaded three bins
+//               ahead), which k_p3_ax0_rows transposes into the sinogram.
 //      adjoint  k_p3_ax0_adj: lanes = slices (up to four each), a warp owns
 //               4x4 pixels; the view's detector columns are staged as
 //               [column][slice] and kept in registers from pixel to pixel.
 //  * GENERAL -- any matrices: proj3d_gen.cuh.
 #include <algorithm>
+#include <atomic>
 #include <cmath>
+#include <cstdlib>
 #include <map>
 #include <mutex>
 #include <tuple>
+#include <type_traits>
 #include <vector>
 
 #include "kernels.cuh"
@@ -44,11 +47,8 @@ namespace {
 constexpr int kVT = CT_VIEW3D_STRIDE;
 constexpr int kOrd = CT_PROJ3D_ORDER;
 constexpr int kTileJ = 16, kTileK = 16;  // AXIS0 forward pixel tile (axis 1 x axis 2)
-constexpr int kFwdSlices = 64;  // slices per forward CTA: two per lane
-constexpr int kSvStride = 66;   // shared [pixel][slice] row stride (floats, even: float2 reads)
-constexpr int kWalkGroup = 8;   // walk entries whose loads are issued together
-constexpr int kFwdViewsPerCta = 16;
-constexpr int kFwdViewsPerWarp = kFwdViewsPerCta / 8;
+constexpr int kFwdPad = 64;  // slices of the forward accumulator are padded to this
+constexpr int kWalkGroup = 4;   // walk entries tested together for a new bin
 
 static_assert(kTileJ * kTileK == kOrd, "order table covers one tile");
 
@@ -117,8 +117,6 @@ struct Ax0FwdArgs {
   const uint16_t* order;
   int S, NJ, NK, V, C, Spad;
   int tiles_k, n_tiles, G;
-  int vpc;   // views per CTA
-  int* errflag;
   const double* skip;  // device flag: return at once when non-zero (may be null)
 };
 
@@ -198,92 +196,215 @@ __device__ int zorder_select(int r, int nj, int nk) {
   return code;
 }
 
-__global__ void __launch_bounds__(256, 2) k_p3_ax0_fwd(const Ax0FwdArgs a) {
+// SL consecutive floats as one shared or global access.
+template <int SL>
+struct FwdVec {
+  float x[SL];
+  __device__ __forceinline__ void zero() {
+#pragma unroll
+    for (int i = 0; i < SL; ++i) x[i] = 0.0f;
+  }
+  // sums and differences by pairs (each half rounded as the scalar operation)
+  __device__ __forceinline__ FwdVec plus(const FwdVec& b) const {
+    FwdVec r;
+    if constexpr (SL > 1) {
+#pragma unroll
+      for (int i = 0; i < SL; i += 2) g_upk(g_add(g_pk(x[i], x[i + 1]), g_pk(b.x[i], b.x[i + 1])), r.x[i], r.x[i + 1]);
+    } else {
+      r.x[0] = x[0] + b.x[0];
+    }
+    return r;
+  }
+  __device__ __forceinline__ FwdVec minus(const FwdVec& b) const {
+    FwdVec r;
+    if constexpr (SL > 1) {
+#pragma unroll
+      for (int i = 0; i < SL; i += 2) g_upk(g_sub(g_pk(x[i], x[i + 1]), g_pk(b.x[i], b.x[i + 1])), r.x[i], r.x[i + 1]);
+    } else {
+      r.x[0] = x[0] - b.x[0];
+    }
+    return r;
+  }
+  // this += w x, sx += x
+  __device__ __forceinline__ void add(float w, const FwdVec& v, FwdVec& sx) {
+    if constexpr (SL > 1) {
+      const unsigned long long ww = g_pk(w, w);
+#pragma unroll
+      for (int i = 0; i < SL; i += 2) {
+        const unsigned long long xx = g_pk(v.x[i], v.x[i + 1]);
+        g_upk(g_fma(ww, xx, g_pk(x[i], x[i + 1])), x[i], x[i + 1]);
+        g_upk(g_add(g_pk(sx.x[i], sx.x[i + 1]), xx), sx.x[i], sx.x[i + 1]);
+      }
+    } else {
+      x[0] = fmaf(w, v.x[0], x[0]);
+      sx.x[0] += v.x[0];
+    }
+  }
+  static __device__ __forceinline__ FwdVec shared(uint32_t at) {
+    FwdVec v;
+    if constexpr (SL == 4)
+      asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x[0]), "=f"(v.x[1]), "=f"(v.x[2]), "=f"(v.x[3]) : "r"(at));
+    else if constexpr (SL == 2)
+      asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(v.x[0]), "=f"(v.x[1]) : "r"(at));
+    else
+      asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v.x[0]) : "r"(at));
+    return v;
+  }
+  static __device__ __forceinline__ FwdVec global(const float* p) {
+    FwdVec v;
+    if constexpr (SL == 4) {
+      const float4 f = __ldcg(reinterpret_cast<const float4*>(p));
+      v.x[0] = f.x;
+      v.x[1] = f.y;
+      v.x[2] = f.z;
+      v.x[3] = f.w;
+    } else if constexpr (SL == 2) {
+      const float2 f = __ldcg(reinterpret_cast<const float2*>(p));
+      v.x[0] = f.x;
+      v.x[1] = f.y;
+    } else {
+      v.x[0] = __ldcg(p);
+    }
+    return v;
+  }
+  __device__ __forceinline__ void store(float* p) const {
+    if constexpr (SL == 4)
+      __stcg(reinterpret_cast<float4*>(p), make_float4(x[0], x[1], x[2], x[3]));
+    else if constexpr (SL == 2)
+      __stcg(reinterpret_cast<float2*>(p), make_float2(x[0], x[1]));
+    else
+      __stcg(p, x[0]);
+  }
+};
+
+__host__ __device__ constexpr int fwd_row(int SL) { return 32 * SL + 4; }  // floats of a staged pixel
+constexpr size_t fwd3_smem(int SL, int NW) {
+  return sizeof(float) * kOrd * fwd_row(SL) + NW * (sizeof(float2) + sizeof(unsigned char)) * kOrd;
+}
+
+// AXIS0 forward: a CTA takes 32 SL slices, NW views (a warp each) and a run of
+// pixel tiles.  A tile is staged as [pixel][slice] (rows of 32 SL + 4 floats:
+// the transposing copies of 8 pixels x 4 slices a warp hit 32 banks, a warp
+// reads a pixel in 16-byte pieces without conflicts); a warp walks its 256
+// pixels in the view's detector order with the open bin and its successor in
+// registers, SL slices a lane: one shared read of x, one of the table entry
+// (weight, pixel offset) and two operations a slice per pixel.  Entries are
+// tested four at a time for a new bin, which about one in ten pixels opens.
+// Bound by shared reads (4 bytes an interaction) and issue slots.  SL and NW
+// are the plan's.  256^3 x 360 views with two slices a
+// lane, two views a warp and a test per entry 3853 us a call, this 1972 us.
+template <int SL, int NW>
+__global__ void __launch_bounds__(NW * 32, SL == 4 ? 1 : 2) k_p3_ax0_fwd(const Ax0FwdArgs a) {
   if (a.skip && *a.skip != 0.0) return;
   extern __shared__ __align__(16) float smem[];
-  float* sv = smem;                                           // [kOrd][kSvStride]
-  float2* tab = reinterpret_cast<float2*>(sv + kOrd * kSvStride);  // [8][kOrd]
-  __shared__ float vpar[kFwdViewsPerCta][4];
+  constexpr int kRow = fwd_row(SL);
+  float* sv = smem;                                               // [kOrd][kRow]
+  float2* tab = reinterpret_cast<float2*>(sv + kOrd * kRow);      // [NW][kOrd] weight, byte offset | new bin << 31
+  unsigned char* bins = reinterpret_cast<unsigned char*>(tab + NW * kOrd);  // [NW][kOrd] tile-relative bin
+  __shared__ int2 tlist[256];                                     // tile origins (j0, k0)
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int g = blockIdx.x, i0 = blockIdx.y * kFwdSlices, v0 = blockIdx.z * a.vpc;
-  const int nvh = min(a.vpc, a.V - v0);
+  const int g = blockIdx.x, i0 = blockIdx.y * 32 * SL, v = blockIdx.z * NW + warp;
+  const bool live = v < a.V;  // warp-uniform
   float2* tabw = tab + warp * kOrd;
+  unsigned char* binw = bins + warp * kOrd;
   const uint32_t sv_s = (uint32_t)__cvta_generic_to_shared(sv);
 
-  // zero this CTA's slices of the output accumulator; fetch the CTA's view
-  // parameters (M[1][1..3]) and each warp's walk orders (entry 32u + lane),
-  // which do not depend on the tile
-  for (int v = 0; v < nvh; ++v) {
-    float* o = a.acc_out + ((size_t)g * a.V + v0 + v) * a.C * a.Spad + i0;
-    for (int e = tid; e < a.C * kFwdSlices; e += 256)
-      o[(size_t)(e / kFwdSlices) * a.Spad + (e % kFwdSlices)] = 0.0f;
-  }
-  if (tid < 3 * nvh) vpar[tid / 3][tid % 3] = a.views[(size_t)(v0 + tid / 3) * kVT + 5 + tid % 3];
-  int ordr[kFwdViewsPerWarp][kOrd / 32];
+  // this warp's accumulator slices (column c at o + c Spad), zeroed; its view
+  // parameters and walk order (entry 32u + lane)
+  const bool mine = live && i0 + SL * lane < a.Spad;
+  float* o = a.acc_out + ((size_t)g * a.V + (live ? v : 0)) * a.C * a.Spad + i0 + SL * lane;
+  FwdVec<SL> zero;
+  zero.zero();
+  float m11 = 0.f, m12 = 0.f, m13 = 0.f;
+  unsigned ord[kOrd / 64];
+  if (live) {
+    if (mine)
+      for (int c = 0; c < a.C; ++c) zero.store(o + (size_t)c * a.Spad);
+    const float* m = a.views + (size_t)v * kVT;
+    m11 = m[5];
+    m12 = m[6];
+    m13 = m[7];
+    const uint16_t* q = a.order + (size_t)v * kOrd;
 #pragma unroll
-  for (int w = 0; w < kFwdViewsPerWarp; ++w) {
-    const int vi = warp + 8 * w;
-    const uint16_t* ord = a.order + (size_t)(v0 + min(vi, nvh - 1)) * kOrd;
-#pragma unroll
-    for (int u = 0; u < kOrd / 32; ++u) ordr[w][u] = __ldg(ord + 32 * u + lane);
+    for (int u = 0; u < kOrd / 64; ++u) ord[u] = __ldg(q + 64 * u + lane) | (unsigned)__ldg(q + 64 * u + 32 + lane) << 16;
   }
-  __syncthreads();
 
-  // this group's run of tiles in Z-order, ranks [g per, (g + 1) per): each
-  // thread looks up one rank, 256 tiles at a time
-  __shared__ int2 tlist[256];  // tile origins (j0, k0)
-  const int nrun = min((a.n_tiles + a.G - 1) / a.G, a.n_tiles - g * ((a.n_tiles + a.G - 1) / a.G));
+  const int per = (a.n_tiles + a.G - 1) / a.G, nrun = min(per, a.n_tiles - g * per);
+  const int c8 = lane & 7, s4 = lane >> 3;
   for (int q = 0; q < nrun; ++q) {
     if ((q & 255) == 0) {
-      if (q + tid < nrun) {
-        const int tiles_j = a.n_tiles / a.tiles_k, per = (a.n_tiles + a.G - 1) / a.G;
+      // this group's run of tiles in Z-order, ranks [g per, (g + 1) per)
+      for (int e = tid; e < 256 && q + e < nrun; e += NW * 32) {
+        const int tiles_j = a.n_tiles / a.tiles_k;
         int tj, tk;
-        zorder_decode(zorder_select(g * per + q + tid, tiles_j, a.tiles_k), bit_len(tiles_j),
-                      bit_len(a.tiles_k), tj, tk);
-        tlist[tid] = make_int2(tj * kTileJ, tk * kTileK);
+        zorder_decode(zorder_select(g * per + q + e, tiles_j, a.tiles_k), bit_len(tiles_j), bit_len(a.tiles_k), tj, tk);
+        tlist[e] = make_int2(tj * kTileJ, tk * kTileK);
       }
       __syncthreads();
     }
     const int2 t0 = tlist[q & 255];
     const int j0 = t0.x, k0 = t0.y;
-    // stage vol[i0+s][j0+j][k0+k] as sv[(j*16+k)*66 + s] with register-free
-    // 4-byte async copies, all in flight at once.  A warp copies two
-    // 16-float rows, slices s and s+1 of one j (lanes = k, then the second
-    // half-warp): shared banks 2k + s and 2k + s + 1 are all distinct
-#pragma unroll 8
-    for (int q = 0; q < kOrd * kFwdSlices / 256; ++q) {
-      const int row = 2 * (q * 8 + warp) + (lane >> 4);  // (s, j) = (row % 64, row / 64)
-      const int s = row % kFwdSlices, j = row / kFwdSlices, k = lane & 15;
-      const int gi = i0 + s, gj = j0 + j, gk = k0 + k;
-      const bool ok = gi < a.S && gj < a.NJ && gk < a.NK;
-      const float* src = ok ? a.vol + ((size_t)gi * a.NJ + gj) * a.NK + gk : a.vol;
-      cp_async4(sv_s + (uint32_t)((j * kTileK + k) * kSvStride + s) * 4u, src, ok);
-    }
-    cp_async_wait_all();
-    __syncthreads();
-
-#pragma unroll 1
-    for (int w = 0; w < kFwdViewsPerWarp; ++w) {
-      const int vi = warp + 8 * w;
-      if (vi >= nvh) break;
-      const int v = v0 + vi;
-      const float m11 = vpar[vi][0], m12 = vpar[vi][1], m13 = vpar[vi][2];
-      int lo, hi;
-      tile_bins(m11, m12, m13, j0, k0, lo, hi);
-      const int nb = hi - lo;
-      // table entries: (w0, bin << 16 | pixel*66).  The second tap's weight
-      // is 1 - w0 = 2*(0.5 - t1) exactly; taps on columns off the detector
-      // are accumulated and never written out, so no masks here
-      int po[kOrd / 32];  // this view's order entries (register select, no local memory)
+    // stage: a warp copies 8 pixels of a row x 4 slices per instruction, the
+    // slice quads warp, warp + NW, ..
+    const bool inside = j0 + kTileJ <= a.NJ && k0 + kTileK <= a.NK;
+    for (int sq = warp; sq < 8 * SL; sq += NW) {
+      const int s = 4 * sq + s4;
+      const float* src = a.vol + ((size_t)min(i0 + s, a.S - 1) * a.NJ + j0) * a.NK + k0 + c8;
+      uint32_t d = sv_s + 4u * (uint32_t)(c8 * kRow + s);
+      if (inside && i0 + 4 * sq + 4 <= a.S) {  // warp-uniform
 #pragma unroll
-      for (int u = 0; u < kOrd / 32; ++u) {
-        po[u] = ordr[0][u];
-#pragma unroll
-        for (int w2 = 1; w2 < kFwdViewsPerWarp; ++w2) po[u] = w == w2 ? ordr[w2][u] : po[u];
+        for (int j = 0; j < kTileJ; ++j) {
+          cp_async4_all(d, src);
+          cp_async4_all(d + 4u * 8 * kRow, src + 8);
+          src += a.NK;
+          d += 4u * kTileK * kRow;
+        }
+      } else {
+        for (int j = 0; j < kTileJ; ++j) {
+          const bool row = i0 + s < a.S && j0 + j < a.NJ;
+          const bool ok0 = row && k0 + c8 < a.NK, ok1 = row && k0 + c8 + 8 < a.NK;
+          cp_async4(d, ok0 ? src : a.vol, ok0);
+          cp_async4(d + 4u * 8 * kRow, ok1 ? src + 8 : a.vol, ok1);
+          src += a.NK;
+          d += 4u * kTileK * kRow;
+        }
       }
+    }
+    // the next tile's accumulator columns towards L2 (all the CTAs' accumulators
+    // are larger than it): 8 columns x 4 pieces of the slices an instruction
+    if (live && q + 1 < nrun && ((q + 1) & 255) != 0) {
+      const int2 t1 = tlist[(q + 1) & 255];
+      int lo, hi;
+      tile_bins(m11, m12, m13, t1.x, t1.y, lo, hi);
+      const float* ahead = o - SL * lane + 8 * SL * s4;
+      for (int c = lo + c8; c < hi; c += 8)
+        if (c >= 0 && c < a.C && i0 + 8 * SL * s4 < a.Spad)
+          asm volatile("prefetch.global.L2 [%0];" ::"l"(ahead + (ptrdiff_t)c * a.Spad));
+    }
+    // the view's table while the copies run.  The second tap's weight is
+    // 1 - w0 = 2 (0.5 - t1) exactly; taps on columns off the detector are
+    // accumulated and never written out, so no masks here
+    int lo = 0;
+    // the accumulator's values of the open bin's column and the next two
+    FwdVec<SL> r0 = zero, r1 = zero, r2 = zero;
+    auto old_at = [&](int c, const float* at, FwdVec<SL>& r) {
+      r = zero;
+      if (mine && (unsigned)c < (unsigned)a.C) r = FwdVec<SL>::global(at);
+    };
+    auto put = [&](int c, float* at, const FwdVec<SL>& r) {
+      if (mine && (unsigned)c < (unsigned)a.C) r.store(at);
+    };
+    if (live) {
+      int hi;
+      tile_bins(m11, m12, m13, j0, k0, lo, hi);
+      old_at(lo, o + (ptrdiff_t)lo * a.Spad, r0);
+      old_at(lo + 1, o + (ptrdiff_t)(lo + 1) * a.Spad, r1);
+      old_at(lo + 2, o + (ptrdiff_t)(lo + 2) * a.Spad, r2);
+      const int nb = hi - lo;
+      int last = 0;  // the bin of the entry before this round's first
 #pragma unroll
       for (int u = 0; u < kOrd / 32; ++u) {
-        const int p = po[u];
+        const int p = (int)((ord[u / 2] >> (16 * (u & 1))) & 0xffffu);
         const float x1 = (float)(j0 + p / kTileK) + 0.5f, x2 = (float)(k0 + p % kTileK) + 0.5f;
         // Px_1 with M[1][0] = 0: the x0 term is an exact zero
         const float px = fadd(fadd(fmul(m11, x1), fmul(m12, x2)), m13);
@@ -291,86 +412,111 @@ __global__ void __launch_bounds__(256, 2) k_p3_ax0_fwd(const Ax0FwdArgs a) {
         float t1;
         edge3(px, ul, t1);
         const int rel = min(max(ul - lo, 0), nb - 2);  // in range: extremes at corners
-        tabw[32 * u + lane] = make_float2(fmul(2.0f, t1), __int_as_float((rel << 16) | (p * kSvStride)));
+        const int before = __shfl_up_sync(0xffffffffu, rel, 1);
+        const bool opens = rel != (lane == 0 ? last : before);
+        last = __shfl_sync(0xffffffffu, rel, 31);
+        tabw[32 * u + lane] = make_float2(fmul(2.0f, t1), __int_as_float(p * kRow * 4 | (opens ? (int)0x80000000 : 0)));
+        binw[32 * u + lane] = (unsigned char)rel;
       }
-      __syncwarp();
-      // this warp's slices of the output accumulator: column c at o[c * Spad]
-      float2* o = reinterpret_cast<float2*>(a.acc_out + (((size_t)g * a.V + v) * a.C) * a.Spad + i0) + lane;
-      const size_t ostride = (size_t)a.Spad / 2;
-      auto old_at = [&](int c) {
-        return (c >= 0 && c < a.C) ? o[(size_t)c * ostride] : make_float2(0.f, 0.f);
+    }
+    cp_async_wait_all();
+    __syncthreads();
+
+    if (live) {
+      // Open bin c - lo: its total is cin + sum w0*x over its own pixels (av);
+      // the next bin receives sum (1-w0)*x = sx - av.
+      int c = lo;
+      float* at = o + (ptrdiff_t)lo * a.Spad;
+      FwdVec<SL> cin = zero, av = zero, sx = zero;
+      auto open_bin = [&](int nc) {
+        put(c, at, r0.plus(cin.plus(av)));
+        cin = sx.minus(av);
+        if (nc == c + 1) {
+          at += a.Spad;
+          r0 = r1;
+          r1 = r2;
+          old_at(c + 3, at + 2 * (ptrdiff_t)a.Spad, r2);
+        } else {  // a jump (rare: rounding at near-ties of the order)
+          put(c + 1, at + a.Spad, r1.plus(cin));
+          at = o + (ptrdiff_t)nc * a.Spad;
+          old_at(nc, at, r0);
+          old_at(nc + 1, at + a.Spad, r1);
+          old_at(nc + 2, at + 2 * (ptrdiff_t)a.Spad, r2);
+          cin = zero;
+        }
+        av = zero;
+        sx = zero;
+        c = nc;
       };
-      auto put = [&](int c, float2 val) {
-        if (c >= 0 && c < a.C) o[(size_t)c * ostride] = val;
-      };
-      // Open bin cb (tile-relative): its total is cin + sum w0*x over its
-      // own pixels (a); the next bin receives sum (1-w0)*x = s - a.  r0..r2
-      // hold the accumulator's values of bins cb..cb+2, loaded ahead.
-      int cb = 0;
-      float2 cin = make_float2(0.f, 0.f), av = cin, sx = cin;
-      float2 r0 = old_at(lo), r1 = old_at(lo + 1), r2 = old_at(lo + 2);
+      const uint32_t xb = sv_s + 4u * SL * (uint32_t)lane;
+#pragma unroll 2
       for (int e0 = 0; e0 < kOrd; e0 += kWalkGroup) {
-        float2 T[kWalkGroup], x[kWalkGroup];
-#pragma unroll
-        for (int u = 0; u < kWalkGroup; ++u) T[u] = tabw[e0 + u];
-#pragma unroll
-        for (int u = 0; u < kWalkGroup; ++u)
-          x[u] = *reinterpret_cast<const float2*>(sv + (__float_as_int(T[u].y) & 0xffff) + 2 * lane);
+        float2 T[kWalkGroup];
+        int any = 0;
 #pragma unroll
         for (int u = 0; u < kWalkGroup; ++u) {
-          const int rb = __float_as_int(T[u].y) >> 16;
-          if (__builtin_expect(rb != cb, 0)) {  // warp-uniform: every lane reads the same entry
-            put(lo + cb, make_float2(r0.x + (cin.x + av.x), r0.y + (cin.y + av.y)));
-            const float2 nxt = make_float2(sx.x - av.x, sx.y - av.y);
-            if (rb == cb + 1) {
-              r0 = r1;
-              r1 = r2;
-              r2 = old_at(lo + cb + 3);
-              cin = nxt;
-            } else {  // a jump (rare: rounding at near-ties of the order)
-              put(lo + cb + 1, make_float2(r1.x + nxt.x, r1.y + nxt.y));
-              r0 = old_at(lo + rb);
-              r1 = old_at(lo + rb + 1);
-              r2 = old_at(lo + rb + 2);
-              cin = make_float2(0.f, 0.f);
-            }
-            av = make_float2(0.f, 0.f);
-            sx = av;
-            cb = rb;
+          T[u] = tabw[e0 + u];
+          any |= __float_as_int(T[u].y);
+        }
+        FwdVec<SL> x[kWalkGroup];
+        if (any >= 0) {  // no new bin among them (warp-uniform)
+#pragma unroll
+          for (int u = 0; u < kWalkGroup; ++u) x[u] = FwdVec<SL>::shared(xb + (uint32_t)__float_as_int(T[u].y));
+#pragma unroll
+          for (int u = 0; u < kWalkGroup; ++u) av.add(T[u].x, x[u], sx);
+        } else {
+#pragma unroll
+          for (int u = 0; u < kWalkGroup; ++u)
+            x[u] = FwdVec<SL>::shared(xb + (uint32_t)(__float_as_int(T[u].y) & 0x7fffffff));
+#pragma unroll
+          for (int u = 0; u < kWalkGroup; ++u) {
+            if (__float_as_int(T[u].y) < 0) open_bin(lo + binw[e0 + u]);
+            av.add(T[u].x, x[u], sx);
           }
-          av.x = fmaf(T[u].x, x[u].x, av.x);
-          av.y = fmaf(T[u].x, x[u].y, av.y);
-          sx.x += x[u].x;
-          sx.y += x[u].y;
         }
       }
-      put(lo + cb, make_float2(r0.x + (cin.x + av.x), r0.y + (cin.y + av.y)));
-      put(lo + cb + 1, make_float2(r1.x + (sx.x - av.x), r1.y + (sx.y - av.y)));
-      __syncwarp();
+      put(c, at, r0.plus(cin.plus(av)));
+      put(c + 1, at + a.Spad, r1.plus(sx.minus(av)));
     }
     __syncthreads();
   }
 }
 
-// proj[v][r][c] = sum_g acc_out[g][v][c][r - row_offset] (0 where no slice
-// lands on row r).  32x32 (col, row) tiles through shared memory.
-__global__ void k_p3_ax0_rows(const float* __restrict__ acc, float* __restrict__ proj, int V,
+constexpr int kMaxGroups = 8;  // AXIS0 forward tile groups (the most a schedule uses)
+
+// proj[v][r][c] = sum_g acc_out[g][v][c][r - row_offset] in group order (0 where
+// no slice lands on row r).  32x32 (col, row) tiles through shared memory, the
+// groups' values of four columns all loaded before they are added.
+__global__ void __launch_bounds__(256) k_p3_ax0_rows(const float* __restrict__ acc, float* __restrict__ proj, int V,
                               int R, int C, int S, int Spad, int G, int row_offset,
                               const double* skip) {
   if (skip && *skip != 0.0) return;
   __shared__ float t[32][33];
   const int c0 = blockIdx.x * 32, r0 = blockIdx.y * 32, v = blockIdx.z;
   const int lx = threadIdx.x, ly = threadIdx.y;  // 32 x 8
-  for (int q = 0; q < 4; ++q) {
-    const int cl = ly + 8 * q, c = c0 + cl;
-    const int i = r0 + lx - row_offset;
-    float s = 0.f;
-    if (c < C && i >= 0 && i < S) {
-      for (int gg = 0; gg < G; ++gg) s += acc[(((size_t)gg * V + v) * C + c) * Spad + i];
-    }
-    t[cl][lx] = s;
+  const int i = r0 + lx - row_offset;
+  const bool slice = i >= 0 && i < S;
+  float s[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+  for (int gg = 0; gg < kMaxGroups; gg += 4) {
+    if (gg >= G) break;
+    float x[4][4];
+#pragma unroll
+    for (int h = 0; h < 4; ++h)
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const int c = c0 + ly + 8 * q;
+        x[h][q] = slice && c < C && gg + h < G ? __ldcs(acc + (((size_t)(gg + h) * V + v) * C + c) * Spad + i) : 0.f;
+      }
+#pragma unroll
+    for (int h = 0; h < 4; ++h)
+#pragma unroll
+      for (int q = 0; q < 4; ++q) s[q] += x[h][q];
   }
+#pragma unroll
+  for (int q = 0; q < 4; ++q) t[ly + 8 * q][lx] = s[q];
   __syncthreads();
+#pragma unroll
   for (int q = 0; q < 4; ++q) {
     const int rl = ly + 8 * q, r = r0 + rl, c = c0 + lx;
     if (r < R && c < C) proj[((size_t)v * R + r) * C + c] = t[lx][rl];
@@ -771,9 +917,7 @@ ct_status proj3d_check(const ct_geom3d* g, const char* who) {
   return CT_OK;
 }
 
-// Largest schedule values the tuner tries: AXIS0 forward tile groups and
-// adjoint view splits.
-constexpr int kMaxGroups = 8;
+// Most adjoint view splits the tuner tries.
 constexpr int kMaxSplits3d = 4;
 constexpr size_t kGenScratch = 96u << 20;  // bytes of GENERAL forward tiles per launch
 
@@ -795,29 +939,72 @@ Proj3dPlan proj3d_plan_sched(const ct_geom3d* g, Sched3d sc) {
     p.adj_tune = tune > 1 ? round_up((size_t)tune * one, 256) : 0;
   };
   if (g->kind == CT_PROJ3D_AXIS0) {
-    p.Spad = (S + kFwdSlices - 1) / kFwdSlices * kFwdSlices;
+    p.Spad = (S + kFwdPad - 1) / kFwdPad * kFwdPad;
     p.tiles_k = (NK + kTileK - 1) / kTileK;
     p.n_tiles = p.tiles_k * ((NJ + kTileJ - 1) / kTileJ);
-    const long base = (long)(p.Spad / kFwdSlices) * ((V + p.vpc - 1) / p.vpc);
     const int g_max = std::min(kMaxGroups, p.n_tiles);
-    if (sc.G > 0) {
-      p.G = std::min(sc.G, g_max);
-    } else {
-      // tile groups: fill the GPU (two CTAs per SM) with a small last wave
-      const long slots = 2L * sms;
+    // forward: slices a lane, warps a CTA and tile groups by the time of the
+    // busiest SM, in units of one view's walk of a tile with four slices a lane:
+    // 0.66 and 0.5 for two and one, a tile's copies, which nothing overlaps,
+    // about a quarter a slice of the lane, slower below 16 warps an SM (0.7 of
+    // the rate at 8, 1.15 at 32); fitted to 256^3 x 360, 128^3 x 180, 64^3 x 90
+    // and unequal sides
+    auto fwd_cost = [&](int sl, int nw, int G) {
+      const long ctas = (long)((S + 32 * sl - 1) / (32 * sl)) * ((V + nw - 1) / nw) * G;
+      const double rounds = std::ceil((double)ctas / sms);
+      const int fit = sl == 4 ? 1 : std::min((int)(220 * 1024 / fwd3_smem(sl, nw)), nw == 16 ? 2 : 20 / nw);
+      const double warps = nw * std::min((double)fit, rounds);
+      const double walk = sl == 4 ? 1.0 : (sl == 2 ? 0.66 : 0.5);
+      return rounds * ((p.n_tiles + G - 1) / G) * (nw * walk + 0.25 * sl) / std::min(1.15, std::pow(warps / 16.0, 0.55)) +
+             0.02 * (double)V * p.n_tiles * S / 128 / sms * G;  // the groups' sum
+    };
+    auto fwd_best = [&](int G, Proj3dPlan& q) {
+      double best = 1e300;
+      for (int sl = 4; sl >= 1; sl /= 2)
+        for (int nw = 16; nw >= 4; nw /= 2)
+          {
+            if (getenv("X_SL") && sl != atoi(getenv("X_SL"))) continue;
+            if (getenv("X_NW") && nw != atoi(getenv("X_NW"))) continue;
+            const double c = fwd_cost(sl, nw, G);
+            if (c < 0.98 * best) {
+              best = c;
+              q.fwd_sl = sl;
+              q.fwd_nw = nw;
+            }
+          }
+      return best;
+    };
+    p.G = std::min(std::max(sc.G, 1), g_max);
+    if (sc.G <= 0) {
+      double best = 1e300;
+      for (int G = 1; G <= g_max; ++G) {
+        const double c = fwd_best(G, p);
+        if (c < 0.98 * best) {
+          best = c;
+          p.G = G;
+        }
+      }
+    }
+    fwd_best(p.G, p);
+    // the groups that a call has always needed scratch for (64 slices and 16
+    // views a CTA, two CTAs an SM)
+    int old_G = std::min(std::max(sc.G, 1), g_max);
+    if (sc.G <= 0) {
+      const long base = (long)(p.Spad / 64) * ((V + 15) / 16), slots = 2L * sms;
       double best = -1.0;
       for (int G = 1; G <= g_max; ++G) {
         const double waves = (double)(base * G) / (double)slots;
         const double score = std::min(1.0, waves) * waves / std::ceil(waves);
         if (score > best + 1e-9) {
           best = score;
-          p.G = G;
+          old_G = G;
         }
       }
     }
-    p.fwd_smem = sizeof(float) * (size_t)kOrd * kSvStride + sizeof(float2) * 8 * kOrd;
-    p.fwd_bytes = round_up(sizeof(float) * (size_t)p.G * V * C * p.Spad, 256);
-    p.fwd_ws_bytes = round_up(sizeof(float) * (size_t)g_max * V * C * p.Spad, 256);
+    const size_t group = sizeof(float) * (size_t)V * C * p.Spad;
+    p.fwd_least = round_up(group * old_G, 256);
+    p.fwd_bytes = round_up(group * p.G, 256);
+    p.fwd_ws_bytes = round_up(group * g_max, 256);
     // adjoint: slices a lane (SL) and view splits by the time of the busiest SM,
     // in units of a CTA's view: 1 at SL = 4, 0.62 and 0.42 at 2 and 1 (the
     // per-pixel work is shared by fewer slices); a split costs a pass over
@@ -927,19 +1114,51 @@ ct_status need_ws(const char* who, size_t need, void* ws, size_t bytes) {
   return CT_OK;
 }
 
-ct_status proj3d_prepare(const ct_geom3d* g, const Proj3dPlan& p) {
-  if (!errflag3_ptr()) return fail(CT_ERR_CUDA, "proj3d: error-word address unavailable");
-  if (g->kind != CT_PROJ3D_AXIS0)
-    return cuda_check(cudaFuncSetAttribute(k_p3_gen_windows, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           (int)(sizeof(float4) * kGenWarps * kSlots)),
-                      "k_p3_gen_windows smem attribute");
-  auto raise = [](auto* kernel, size_t bytes, const char* what) {
-    return cuda_check(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes), what);
+// f(kernel, shared bytes, slices of a CTA) of the plan's AXIS0 forward.
+template <class F>
+void with_fwd(const Proj3dPlan& p, F&& f) {
+  auto by_warps = [&](auto sl) {
+    constexpr int SL = decltype(sl)::value;
+    if (p.fwd_nw == 16)
+      f(k_p3_ax0_fwd<SL, 16>, fwd3_smem(SL, 16), 32 * SL);
+    else if (p.fwd_nw == 8)
+      f(k_p3_ax0_fwd<SL, 8>, fwd3_smem(SL, 8), 32 * SL);
+    else
+      f(k_p3_ax0_fwd<SL, 4>, fwd3_smem(SL, 4), 32 * SL);
   };
-  ct_status st = raise(k_p3_ax0_adj<4>, adj3_smem(4), "k_p3_ax0_adj smem attribute");
-  if (st == CT_OK) st = raise(k_p3_ax0_adj<2>, adj3_smem(2), "k_p3_ax0_adj smem attribute");
-  if (st == CT_OK) st = raise(k_p3_ax0_adj<1>, adj3_smem(1), "k_p3_ax0_adj smem attribute");
-  if (st == CT_OK) st = raise(k_p3_ax0_fwd, p.fwd_smem, "k_p3_ax0_fwd smem attribute");
+  if (p.fwd_sl == 4)
+    by_warps(std::integral_constant<int, 4>());
+  else if (p.fwd_sl == 2)
+    by_warps(std::integral_constant<int, 2>());
+  else
+    by_warps(std::integral_constant<int, 1>());
+}
+
+// The kernels' dynamic shared memory limits, raised once per device (any plan
+// of a geometry may follow).
+ct_status proj3d_prepare(const ct_geom3d* g, const Proj3dPlan& p) {
+  (void)g;
+  (void)p;
+  if (!errflag3_ptr()) return fail(CT_ERR_CUDA, "proj3d: error-word address unavailable");
+  static std::atomic<uint64_t> done{0};
+  int dev = 0;
+  ct_status st = cuda_check(cudaGetDevice(&dev), "current device");
+  if (st != CT_OK) return st;
+  const uint64_t bit = dev < 64 ? 1ull << dev : 0;
+  if (done.load(std::memory_order_acquire) & bit) return CT_OK;
+  auto raise = [&](auto* kernel, size_t bytes, const char* what) {
+    if (st == CT_OK)
+      st = cuda_check(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes), what);
+  };
+  raise(k_p3_gen_windows, sizeof(float4) * kGenWarps * kSlots, "k_p3_gen_windows smem attribute");
+  raise(k_p3_ax0_adj<4>, adj3_smem(4), "k_p3_ax0_adj smem attribute");
+  raise(k_p3_ax0_adj<2>, adj3_smem(2), "k_p3_ax0_adj smem attribute");
+  raise(k_p3_ax0_adj<1>, adj3_smem(1), "k_p3_ax0_adj smem attribute");
+  Proj3dPlan each;
+  for (each.fwd_sl = 1; each.fwd_sl <= 4; each.fwd_sl *= 2)
+    for (each.fwd_nw = 4; each.fwd_nw <= 16; each.fwd_nw *= 2)
+      with_fwd(each, [&](auto* kernel, size_t bytes, int) { raise(kernel, bytes, "k_p3_ax0_fwd smem attribute"); });
+  if (st == CT_OK) done.fetch_or(bit, std::memory_order_release);
   return st;
 }
 
@@ -962,11 +1181,11 @@ ct_status proj3d_fwd_launch(const ct_geom3d* g, const Proj3dPlan& p, const float
     a.tiles_k = p.tiles_k;
     a.n_tiles = p.n_tiles;
     a.G = p.G;
-    a.vpc = p.vpc;
-    a.errflag = errflag3_ptr();
     a.skip = skip;
-    dim3 grid(p.G, p.Spad / kFwdSlices, (V + p.vpc - 1) / p.vpc);
-    k_p3_ax0_fwd<<<grid, 256, p.fwd_smem, s>>>(a);
+    with_fwd(p, [&](auto* kernel, size_t bytes, int slices) {
+      const dim3 grid(p.G, (S + slices - 1) / slices, (V + p.fwd_nw - 1) / p.fwd_nw);
+      kernel<<<grid, p.fwd_nw * 32, bytes, s>>>(a);
+    });
     ct_status st = launch_check("k_p3_ax0_fwd");
     if (st != CT_OK) return st;
     dim3 g2((C + 31) / 32, (R + 31) / 32, V);
@@ -1148,10 +1367,17 @@ ct_status ct_proj3d_fwd(const ct_geom3d* g, const float* vol, float* proj, int32
   if (st != CT_OK) return st;
   if (!vol || !proj) return fail(CT_ERR_INVALID_ARG, "ct_proj3d_fwd: null array");
   if (batch <= 0) return fail(CT_ERR_INVALID_ARG, "ct_proj3d_fwd: batch=%d", batch);
-  const Proj3dPlan p = proj3d_plan(g, batch);
-  if (g->kind == CT_PROJ3D_AXIS0)
-    st = need_ws("ct_proj3d_fwd", p.fwd_bytes, workspace, workspace_bytes);
-  else if (workspace_bytes < p.fwd_bytes || !aligned(workspace, 256))
+  Proj3dPlan p = proj3d_plan(g, batch);
+  if (g->kind == CT_PROJ3D_AXIS0) {
+    st = need_ws("ct_proj3d_fwd", p.fwd_least, workspace, workspace_bytes);
+    if (st == CT_OK && workspace_bytes < p.fwd_bytes) {  // the groups that fit
+      const size_t group = sizeof(float) * (size_t)g->n_views * g->det_shape[1] * p.Spad;
+      Sched3d fewer;
+      fewer.G = (int)std::max<size_t>(1, workspace_bytes / group);
+      fewer.ns = p.nsplit;
+      p = proj3d_plan_sched(g, fewer);
+    }
+  } else if (workspace_bytes < p.fwd_bytes || !aligned(workspace, 256))
     workspace = nullptr;  // GENERAL runs without scratch, slower
   if (st != CT_OK) return st;
   st = proj3d_prepare(g, p);
