@@ -11,10 +11,11 @@ struct Proj2dPlan {
   int tiles_i, n_chunks, n_strips, L, LS, cspan, vpc, fwd_groups;
   size_t fwd_bytes, fwd_smem;
   // adjoint: 16x64 tiles, view splits, staged window length
-  int adj_gx, adj_gy, nsplit, per_split, W;
+  int adj_gx, adj_gy, nsplit, per_split, W, adj_ni;  // adj_ni: images per CTA
   size_t adj_bytes;     // split partial images of this plan (0 when nsplit == 1)
   size_t adj_ws_bytes;  // the same for the largest split count a schedule may pick
   size_t adj_smem;
+  size_t adj_least;     // scratch below which an adjoint call is refused
 };
 
 // Launch schedule of the 2D projector: forward views per CTA and adjoint view

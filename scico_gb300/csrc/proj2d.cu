@@ -31,6 +31,7 @@
 // full-rate FP32 operations instead of conversion instructions.
 #include <algorithm>
 #include <atomic>
+#include <cmath>
 #include <cstring>
 #include <map>
 #include <tuple>
@@ -47,7 +48,8 @@ namespace {
 constexpr int kT = 32;          // forward tile edge: rows = lanes, columns = registers
 constexpr int kCW = 256;        // forward strip width (8 tiles)
 constexpr int kFW = 8;          // warps of a forward CTA (one tile each)
-constexpr int kFwdTargetCtas = 1824;
+constexpr int kSms = 152;
+constexpr int kFwdTargetCtas = 12 * kSms;
 constexpr int kLSDefault = 47;  // partial-row stride when projected pixels are at most one bin wide
 constexpr int kGL = 16;         // strips read per round by a forward gather warp
 constexpr int kAI = 64;         // adjoint tile rows
@@ -56,7 +58,7 @@ constexpr int kAPX = 4;         // columns per adjoint thread
 constexpr int kAR = 4;          // rows per adjoint thread
 constexpr int kAdjThreads = 256;  // adjoint CTA: 64 x 64 pixels = kAdjThreads x kAR x kAPX
 constexpr int kAVC = 32;        // views staged per adjoint run
-constexpr int kAdjTargetCtas = 1216;  // 152 SMs x 8: view splits until the CTAs balance over the SMs
+constexpr int kAdjTargetCtas = 8 * kSms;  // view splits at most until each SM has eight CTAs
 constexpr int kAdjMinViewsPerSplit = 16;
 constexpr size_t kMaxSmem = 200 * 1024;  // dynamic shared memory of a projector CTA
 constexpr uint32_t kMaxPolls = 1u << 24;
@@ -589,7 +591,7 @@ struct AdjArgs {
   const float* sino;
   float* out;
   const float* views;
-  int rows, cols, nv, det;
+  int rows, cols, nv, det, batch;
   int nsplit, per_split;
   size_t split_stride;
   int W;  // window length (bins) per staged view
@@ -597,15 +599,25 @@ struct AdjArgs {
   const double* skip;
 };
 
-// One view's contribution to this thread's pixels.  Fast path: the window
-// pair of key k lives at shared address off + 8 (kMagicBits + k) for the
-// float bits kMagicBits + k of kMagic + k.
+// One view's contribution to this thread's pixels of NI images.  Fast path: the
+// window pairs of key k (images side by side) live at shared address
+// off + 8 NI (kMagicBits + k) for the float bits kMagicBits + k of kMagic + k.
+// The Px, floor, distance and 1 - w steps of two pixels run as paired
+// instructions (bit-identical to the scalar form); the column products Pdx1 * j
+// are shared by the thread's rows and the weights by the images.
+template <int NI>
+__device__ __forceinline__ void ld_window(uint32_t at, float2 (&y)[NI]) {
+  if constexpr (NI == 1)
+    y[0] = ld_shared2(at);
+  else
+    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+                 : "=f"(y[0].x), "=f"(y[0].y), "=f"(y[1].x), "=f"(y[1].y)
+                 : "r"(at));
+}
 
-// adj_view_fast with the Px, floor, distance and 1 - w steps of two pixels
-// per paired instruction (bit-identical to the scalar form); the column
-// products Pdx1 * j are shared by the thread's rows.
+template <int NI>
 __device__ __forceinline__ void adj_view_fast2(const float4 pv, uint32_t off, const float (&fi)[kAR],
-                                               const float (&fj)[kAPX], float (&acc)[kAR][kAPX]) {
+                                               const float (&fj)[kAPX], float (&acc)[NI][kAR][kAPX]) {
   const unsigned long long M2 = pk2(kMagic, kMagic), M12 = pk2(kMagic - 1.0f, kMagic - 1.0f);
   const unsigned long long one2 = pk2(1.0f, 1.0f);
   float pj[kAPX];
@@ -626,19 +638,24 @@ __device__ __forceinline__ void adj_view_fast2(const float4 pv, uint32_t off, co
       const float w0 = __saturatef(ct::fmul(d0, pv.w)), w1 = __saturatef(ct::fmul(d1, pv.w));
       float o0, o1;
       upk2(fsub2(one2, pk2(w0, w1)), o0, o1);
-      const float2 y0 = ld_shared2(off + 8u * (uint32_t)__float_as_int(t0));
-      const float2 y1 = ld_shared2(off + 8u * (uint32_t)__float_as_int(t1));
-      acc[r][2 * h] = fmaf(y0.x, w0, acc[r][2 * h]);
-      acc[r][2 * h] = fmaf(y0.y, o0, acc[r][2 * h]);
-      acc[r][2 * h + 1] = fmaf(y1.x, w1, acc[r][2 * h + 1]);
-      acc[r][2 * h + 1] = fmaf(y1.y, o1, acc[r][2 * h + 1]);
+      float2 y0[NI], y1[NI];
+      ld_window<NI>(off + 8u * NI * (uint32_t)__float_as_int(t0), y0);
+      ld_window<NI>(off + 8u * NI * (uint32_t)__float_as_int(t1), y1);
+#pragma unroll
+      for (int n = 0; n < NI; ++n) {
+        acc[n][r][2 * h] = fmaf(y0[n].x, w0, acc[n][r][2 * h]);
+        acc[n][r][2 * h] = fmaf(y0[n].y, o0, acc[n][r][2 * h]);
+        acc[n][r][2 * h + 1] = fmaf(y1[n].x, w1, acc[n][r][2 * h + 1]);
+        acc[n][r][2 * h + 1] = fmaf(y1[n].y, o1, acc[n][r][2 * h + 1]);
+      }
     }
   }
 }
 
+template <int NI>
 __device__ __forceinline__ void adj_view_gen(const float4 pv, float width, int base, const float2* __restrict__ wy,
                                              const float (&fi)[kAR], const float (&fj)[kAPX],
-                                             float (&acc)[kAR][kAPX]) {
+                                             float (&acc)[NI][kAR][kAPX]) {
 #pragma unroll
   for (int r = 0; r < kAR; ++r) {
     const float R = ct::fadd(pv.x, ct::fmul(pv.y, fi[r]));
@@ -648,32 +665,39 @@ __device__ __forceinline__ void adj_view_gen(const float4 pv, float width, int b
       int key;
       float w;
       weight_floor(px, width, pv.w, base, key, w);
-      const float2 y = wy[key];
-      acc[r][q] = fmaf(y.x, w, acc[r][q]);
-      acc[r][q] = fmaf(y.y, ct::fsub(1.0f, w), acc[r][q]);
+      const float o = ct::fsub(1.0f, w);
+#pragma unroll
+      for (int n = 0; n < NI; ++n) {
+        const float2 y = wy[key * NI + n];
+        acc[n][r][q] = fmaf(y.x, w, acc[n][r][q]);
+        acc[n][r][q] = fmaf(y.y, o, acc[n][r][q]);
+      }
     }
   }
 }
 
-// grid = (ceil(cols/64), ceil(rows/64), batch*nsplit), block = 256: thread
-// (ty, tx) owns rows ty + 16 r (r < kAR) at columns tx + 16 q (q < kAPX) of
-// the 64 x 64 tile.
-__global__ void __launch_bounds__(kAdjThreads) k_proj2d_adj(const AdjArgs a) {
+// grid = (ceil(cols/64), ceil(rows/64), ceil(batch/NI)*nsplit), block = 256:
+// thread (ty, tx) owns rows ty + 16 r (r < kAR) at columns tx + 16 q (q < kAPX)
+// of the 64 x 64 tile, in NI images.  Images share the positions and weights
+// (some 7 of the 10.5 instructions a pixel and view): 16 x 256^2 x 180 views
+// 75 us with NI = 1, 57 us with 2 (103 us with 4: too few warps an SM).
+template <int NI>
+__device__ __forceinline__ void adj_tile(const AdjArgs& a) {
   ct::grid_dep_wait();  // before any global access (dependent launch)
   ct::grid_dep_trigger();
   if (a.skip && *a.skip != 0.0) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  float2* sy = reinterpret_cast<float2*>(smem_raw);          // [kAVC][W]
-  float4* sp = reinterpret_cast<float4*>(sy + kAVC * a.W);   // [kAVC] pxmin, pd0, pd1, 1/width
-  float* sw = reinterpret_cast<float*>(sp + kAVC);           // [kAVC] width
-  int* sb = reinterpret_cast<int*>(sw + kAVC);               // [kAVC] window base
-  int* sf = sb + kAVC;                                       // [kAVC] 1 = fast floor, -1 = skip
-  uint32_t* so = reinterpret_cast<uint32_t*>(sf + kAVC);     // [kAVC] fast-path address offset
+  float2* sy = reinterpret_cast<float2*>(smem_raw);             // [kAVC][W][NI]
+  float4* sp = reinterpret_cast<float4*>(sy + kAVC * a.W * NI);  // [kAVC] pxmin, pd0, pd1, 1/width
+  float* sw = reinterpret_cast<float*>(sp + kAVC);              // [kAVC] width
+  int* sb = reinterpret_cast<int*>(sw + kAVC);                  // [kAVC] window base
+  int* sf = sb + kAVC;                                          // [kAVC] 1 = fast floor, -1 = skip
+  uint32_t* so = reinterpret_cast<uint32_t*>(sf + kAVC);        // [kAVC] fast-path address offset
 
   constexpr int kWarps = kAdjThreads / 32;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int z = blockIdx.z;
-  const int b = z / a.nsplit, sidx = z - b * a.nsplit;
+  const int b = (z / a.nsplit) * NI, sidx = z % a.nsplit;
   const int vbeg = sidx * a.per_split, vend = min(a.nv, vbeg + a.per_split);
   const int i0 = blockIdx.y * kAI, j0 = blockIdx.x * kAJ;
   const int ty = tid >> 4, tx = tid & 15;
@@ -683,12 +707,15 @@ __global__ void __launch_bounds__(kAdjThreads) k_proj2d_adj(const AdjArgs a) {
   float fj[kAPX];
 #pragma unroll
   for (int q = 0; q < kAPX; ++q) fj[q] = (float)(j0 + tx + 16 * q);
-  float acc[kAR][kAPX];
+  float acc[NI][kAR][kAPX];
 #pragma unroll
-  for (int r = 0; r < kAR; ++r)
+  for (int n = 0; n < NI; ++n)
 #pragma unroll
-    for (int q = 0; q < kAPX; ++q) acc[r][q] = 0.0f;
-  const float* yb = a.sino + (size_t)b * a.nv * a.det;
+    for (int r = 0; r < kAR; ++r)
+#pragma unroll
+      for (int q = 0; q < kAPX; ++q) acc[n][r][q] = 0.0f;
+  const size_t sino_n = (size_t)a.nv * a.det;
+  const float* yb = a.sino + (size_t)b * sino_n;
 
   for (int a0 = vbeg; a0 < vend; a0 += kAVC) {
     const int n = min(kAVC, vend - a0);
@@ -708,42 +735,53 @@ __global__ void __launch_bounds__(kAdjThreads) k_proj2d_adj(const AdjArgs a) {
         f = -1;
       }
       sf[tid] = f;
-      so[tid] = ct::smem_u32(sy + tid * a.W) - 8u * (uint32_t)(kMagicBits + base);
+      so[tid] = ct::smem_u32(sy + tid * a.W * NI) - 8u * NI * (uint32_t)(kMagicBits + base);
     }
     __syncthreads();
     for (int v = warp; v < n; v += kWarps) {
       const float* yr = yb + (size_t)(a0 + v) * a.det;
       const int base = sb[v];
-      float2* wy = sy + v * a.W;
+      float2* wy = sy + v * a.W * NI;
       for (int k = lane; k < a.W; k += 32) {
         const int bin = base + k;
-        const float y0 = ((unsigned)bin < (unsigned)a.det) ? __ldg(yr + bin) : 0.0f;
-        const float y1 = ((unsigned)(bin + 1) < (unsigned)a.det) ? __ldg(yr + bin + 1) : 0.0f;
-        wy[k] = make_float2(y0, y1);
+        const bool in0 = (unsigned)bin < (unsigned)a.det, in1 = (unsigned)(bin + 1) < (unsigned)a.det;
+#pragma unroll
+        for (int m = 0; m < NI; ++m) {
+          const bool image = NI == 1 || b + m < a.batch;
+          const float* q = yr + m * sino_n + bin;
+          wy[k * NI + m] = make_float2(image && in0 ? __ldg(q) : 0.0f, image && in1 ? __ldg(q + 1) : 0.0f);
+        }
       }
     }
     __syncthreads();
     for (int v = 0; v < n; ++v) {
       const int f = sf[v];
       if (f == 1)
-        adj_view_fast2(sp[v], so[v], fi, fj, acc);
+        adj_view_fast2<NI>(sp[v], so[v], fi, fj, acc);
       else if (f == 0)
-        adj_view_gen(sp[v], sw[v], sb[v], sy + v * a.W, fi, fj, acc);
+        adj_view_gen<NI>(sp[v], sw[v], sb[v], sy + v * a.W * NI, fi, fj, acc);
     }
   }
+  auto store = [&](int m) {
 #pragma unroll
-  for (int r = 0; r < kAR; ++r) {
-    const int i = i0 + ty + (kAI / kAR) * r;
-    if (i < a.rows) {
-      float* o = a.out + (size_t)sidx * a.split_stride + (size_t)b * a.rows * a.cols + (size_t)i * a.cols;
+    for (int r = 0; r < kAR; ++r) {
+      const int i = i0 + ty + (kAI / kAR) * r;
+      if (i < a.rows) {
+        float* o = a.out + (size_t)sidx * a.split_stride + (size_t)(b + m) * a.rows * a.cols + (size_t)i * a.cols;
 #pragma unroll
-      for (int q = 0; q < kAPX; ++q) {
-        const int j = j0 + tx + 16 * q;
-        if (j < a.cols) o[j] = acc[r][q];
+        for (int q = 0; q < kAPX; ++q) {
+          const int j = j0 + tx + 16 * q;
+          if (j < a.cols) o[j] = acc[m][r][q];
+        }
       }
     }
-  }
+  };
+  store(0);
+  if (NI == 2 && b + 1 < a.batch) store(NI - 1);
 }
+
+__global__ void __launch_bounds__(kAdjThreads) k_proj2d_adj(const AdjArgs a) { adj_tile<1>(a); }
+__global__ void __launch_bounds__(kAdjThreads, 3) k_proj2d_adj_two(const AdjArgs a) { adj_tile<2>(a); }
 
 // out[e] = sum_s part[s*stride + e] in split order; with a mask (of n_img
 // pixels, one per image of the batch), times `scale` where it is set and 0
@@ -756,15 +794,15 @@ __global__ void __launch_bounds__(256) k_sum_splits(const float* part, float* ou
   for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < n;
        e += (size_t)gridDim.x * blockDim.x) {
     float s = 0.0f;
-    for (int k = 0; k < nsplit; k += kSumU) {
+    int k = 0;
+    for (; k + kSumU <= nsplit; k += kSumU) {
       float v[kSumU];
 #pragma unroll
-      for (int u = 0; u < kSumU; ++u)
-        if (k + u < nsplit) v[u] = part[(size_t)(k + u) * stride + e];
+      for (int u = 0; u < kSumU; ++u) v[u] = part[(size_t)(k + u) * stride + e];
 #pragma unroll
-      for (int u = 0; u < kSumU; ++u)
-        if (k + u < nsplit) s += v[u];
+      for (int u = 0; u < kSumU; ++u) s += v[u];
     }
+    for (; k < nsplit; ++k) s += part[(size_t)k * stride + e];
     if (MASK) s = ct::fmul(mask[n_img == n ? e : e % n_img] ? scale : 0.0f, s);
     out[e] = s;
   }
@@ -829,8 +867,8 @@ size_t fwd_smem_bytes(int LS, int L) {
   return 1008 + sizeof(float) * (fwd_region_floats(LS) + fwd_tbins_floats(L)) + sizeof(FwdViewSmem) + 16;
 }
 
-size_t adj_smem_bytes(int W) {
-  return sizeof(float2) * (size_t)kAVC * W + sizeof(float4) * kAVC + sizeof(float) * kAVC +
+size_t adj_smem_bytes(int W, int NI) {
+  return sizeof(float2) * (size_t)kAVC * W * NI + sizeof(float4) * kAVC + sizeof(float) * kAVC +
          3 * sizeof(int) * kAVC;
 }
 
@@ -883,13 +921,18 @@ Proj2dPlan proj2d_plan_sched(const ct_geom2d* g, int batch, Sched2d sc) {
   while ((p.LS & 31) != 15 && (p.LS & 31) != 17) ++p.LS;
   p.cspan = (int)floorf((float)(kCW - 1) * mw + 1.01f) + 3;
   const long work = (long)p.n_strips * g->n_views * batch;
-  p.vpc = sc.vpc > 0 ? std::min(sc.vpc, kMaxVpc)
-                     : (int)std::min<long>(kMaxVpc, std::max<long>(2, (work + kFwdTargetCtas - 1) / kFwdTargetCtas));
+  // Views per CTA: about kFwdTargetCtas CTAs, each with its staging to pay; a
+  // problem of at most eight rounds of single views instead takes one round of
+  // the SMs' three CTAs (200^2 x 500 views: 27.5 us at 2, 22.0 us at 8; 256^2 x
+  // 180: 14.9 us at 2, 13.9 us at 4; 384^2 x 270 stays: 37.0 us at 4, 39.5 us at 16).
+  const long round = 3L * kSms;
+  const long vpc = work <= 8 * round ? (work + round - 1) / round : (work + kFwdTargetCtas - 1) / kFwdTargetCtas;
+  p.vpc = sc.vpc > 0 ? std::min(sc.vpc, kMaxVpc) : (int)std::min<long>(kMaxVpc, std::max<long>(2, vpc));
   p.fwd_groups = (g->n_views + p.vpc - 1) / p.vpc;
   p.fwd_bytes = round_up((size_t)batch * p.n_strips * g->n_views * p.cspan * sizeof(float), 256);
   p.fwd_smem = fwd_smem_bytes(p.LS, p.L);
   p.W = (int)floorf((float)(std::max(kAI, kAJ) - 1) * mw + 1.01f) + 3;
-  p.adj_smem = adj_smem_bytes(p.W);
+  p.adj_smem = adj_smem_bytes(p.W, 1);
   p.adj_gx = (g->cols + kAJ - 1) / kAJ;
   p.adj_gy = (g->rows + kAI - 1) / kAI;
   const long ctas = (long)p.adj_gx * p.adj_gy * batch;
@@ -900,6 +943,40 @@ Proj2dPlan proj2d_plan_sched(const ct_geom2d* g, int batch, Sched2d sc) {
   } else {
     if (ctas < kAdjTargetCtas) ns = (int)((kAdjTargetCtas + ctas - 1) / ctas);
     ns = std::min(ns, std::max(1, g->n_views / kAdjMinViewsPerSplit));
+  }
+  // the scratch that a call has always needed
+  {
+    const int per = (g->n_views + ns - 1) / ns, split = (g->n_views + per - 1) / per;
+    p.adj_least = split > 1 ? round_up((size_t)split * batch * g->rows * g->cols * sizeof(float), 256) : 0;
+  }
+  // Images per CTA (NI) and, from 2 splits on, the count whose CTAs divide best
+  // over the SMs: rounds of the 4 CTAs (3 with two images) an SM holds, a partial
+  // round at less than its share of the rate, a single one with nothing to
+  // overlap, each CTA's staging, and each split's pass over its partial image.
+  // Fitted to: 256^2 x 180 views 12.6 us at 11 splits, 11.1 us at 9; 200^2 x 500
+  // 20.6 us at 30, 18.2 us at 19; 512^2 x 360 39.3 us at 19, 41.4 us at 9; 768^2 x
+  // 180 45.8 us at 9, 44.2 us at 8; two images a CTA against one: 16 x 256^2 x 180
+  // 57 against 75 us, 2 x 512^2 x 360 54 against 75 us, 4 x 300^2 x 200 28 against 35 us.
+  {
+    const int first = sc.ns > 0 ? ns : std::min(2, ns), most = sc.ns > 0 || ns == 1 ? ns : ns_max;
+    double least = 1e300;
+    for (int ni = 1; ni <= std::min(batch, 2); ++ni) {
+      if (adj_smem_bytes(p.W, ni) > 70 * 1024 && ni > 1) break;
+      const long units = (long)p.adj_gx * p.adj_gy * ((batch + ni - 1) / ni);
+      const int hold = ni == 1 ? 4 : 3;
+      for (int k = first; k <= most; ++k) {
+        const int per_sm = (int)((units * k + kSms - 1) / kSms), part = per_sm % hold;
+        const double rounds = per_sm - part + (part ? hold * std::pow((double)part / hold, 0.75) : 0.0);
+        const double views = (double)((g->n_views + k - 1) / k);
+        const double cost = rounds * (ni == 1 ? views + 2.0 : 1.5 * views + 10.0) * (per_sm <= hold ? 1.06 : 1.0) * (1.0 + 0.003 * k);
+        if (cost < least) {
+          least = cost;
+          ns = k;
+          p.adj_ni = ni;
+        }
+      }
+    }
+    p.adj_smem = adj_smem_bytes(p.W, p.adj_ni);
   }
   p.per_split = (g->n_views + ns - 1) / ns;
   p.nsplit = (g->n_views + p.per_split - 1) / p.per_split;
@@ -970,6 +1047,7 @@ ct_status proj2d_prepare(const Proj2dPlan& p) {
   if ((st = raise(k_proj2d_fwd_strips<kLSDefault>, "fwd smem attribute")) != CT_OK) return st;
   if ((st = raise(k_proj2d_fwd_strips<0>, "fwd smem attribute")) != CT_OK) return st;
   if ((st = raise(k_proj2d_adj, "adj smem attribute")) != CT_OK) return st;
+  if ((st = raise(k_proj2d_adj_two, "adj smem attribute")) != CT_OK) return st;
   done.fetch_or(bit, std::memory_order_release);
   return CT_OK;
 }
@@ -1018,6 +1096,7 @@ ct_status proj2d_adj_launch(const ct_geom2d* g, const Proj2dPlan& p, const float
   a.cols = g->cols;
   a.nv = g->n_views;
   a.det = g->det_count;
+  a.batch = batch;
   a.nsplit = p.nsplit;
   a.per_split = p.per_split;
   a.split_stride = p.nsplit > 1 ? (size_t)batch * g->rows * g->cols : 0;
@@ -1025,9 +1104,9 @@ ct_status proj2d_adj_launch(const ct_geom2d* g, const Proj2dPlan& p, const float
   a.errflag = errflag_ptr();
   a.skip = skip;
   if (!a.errflag) return fail(CT_ERR_CUDA, "proj2d: error-word address unavailable");
-  dim3 grid(p.adj_gx, p.adj_gy, batch * p.nsplit);
-  return cuda_check(launch_k(k_proj2d_adj, grid, dim3(kAdjThreads), p.adj_smem, s, dependent, a),
-                    "k_proj2d_adj");
+  dim3 grid(p.adj_gx, p.adj_gy, (batch + p.adj_ni - 1) / p.adj_ni * p.nsplit);
+  auto kernel = p.adj_ni == 2 ? k_proj2d_adj_two : k_proj2d_adj;
+  return cuda_check(launch_k(kernel, grid, dim3(kAdjThreads), p.adj_smem, s, dependent, a), "k_proj2d_adj");
 }
 
 }  // namespace ct
@@ -1068,12 +1147,17 @@ static ct_status adj_call(const char* who, const ct_geom2d* g, const float* sino
   if (st != CT_OK) return st;
   if (!img || !sino) return ct::fail(CT_ERR_INVALID_ARG, "%s: null array", who);
   if (batch <= 0) return ct::fail(CT_ERR_INVALID_ARG, "%s: batch=%d", who, batch);
-  const ct::Proj2dPlan p = ct::proj2d_plan(g, batch);
+  ct::Proj2dPlan p = ct::proj2d_plan(g, batch);
   cudaStream_t s = ct::as_stream(stream);
-  if (p.nsplit > 1) {
-    if (!workspace || workspace_bytes < p.adj_bytes || !ct::aligned(workspace, 256))
-      return ct::fail(CT_ERR_WORKSPACE, "%s: need %zu bytes (256-B aligned), got %zu", who, p.adj_bytes,
-                      workspace_bytes);
+  const bool usable = workspace && ct::aligned(workspace, 256);
+  if (p.adj_least > 0 && (!usable || workspace_bytes < p.adj_least))
+    return ct::fail(CT_ERR_WORKSPACE, "%s: need %zu bytes (256-B aligned), got %zu", who, p.adj_least,
+                    workspace_bytes);
+  if (p.nsplit > 1 && (!usable || workspace_bytes < p.adj_bytes)) {  // the splits that fit
+    ct::Sched2d fewer;
+    fewer.vpc = p.vpc;
+    fewer.ns = usable ? std::max(1, (int)(workspace_bytes / ((size_t)batch * g->rows * g->cols * sizeof(float)))) : 1;
+    p = ct::proj2d_plan_sched(g, batch, fewer);
   }
   st = ct::proj2d_prepare(p);
   if (st != CT_OK) return st;
