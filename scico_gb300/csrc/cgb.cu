@@ -46,50 +46,170 @@ __device__ __forceinline__ double* rec(double* scal, const Sys& s, int sy, int k
   return sys_scal(scal, s, sy) + C_HEAD + C_REC * k;
 }
 
-// Reduction of K (<= 4) sums over the blocks of one system (grid = (nb, nsys));
-// true in thread 0 of the system's last block.
+// Reduction of K (<= 4) sums over the blocks of one system (grid = (nb, nsys),
+// nb <= 64); true in thread 0 of the system's last block.  The block's first
+// warp finishes alone, both over the block's warps and, in the last block,
+// over the blocks' partials, in fixed shuffle trees: no thread adds a row of
+// float64 values one after the other and no second block-wide barrier stands
+// between the ticket and the result (as block_reduce has it for larger grids;
+// with that form the 16 images below take 2.88 instead of 2.82 ms).
+template <int K>
+__device__ __forceinline__ void warp_sums(double (&v)[K]) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+#pragma unroll
+    for (int k = 0; k < K; ++k) v[k] += __shfl_xor_sync(0xffffffffu, v[k], o);
+  }
+}
+
 template <int K>
 __device__ __forceinline__ bool sys_reduce(double (&v)[K], double* partials, unsigned int* tickets, const Sys& s,
                                            double (&out)[K]) {
-  return ct::grid_reduce_last<NT, K>(v, partials + (size_t)blockIdx.y * 4 * s.nb, tickets + blockIdx.y, out);
+  constexpr int NW = NT / 32;
+  __shared__ double red[K][NW];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  warp_sums<K>(v);
+  if (lane == 0) {
+#pragma unroll
+    for (int k = 0; k < K; ++k) red[k][warp] = v[k];
+  }
+  __syncthreads();
+  if (warp != 0) return false;
+  double* part = partials + (size_t)blockIdx.y * 4 * s.nb;
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    v[k] = red[k][lane & (NW - 1)];
+#pragma unroll
+    for (int o = NW / 2; o > 0; o >>= 1) v[k] += __shfl_xor_sync(0xffffffffu, v[k], o);
+  }
+  int last = 0;
+  if (lane == 0) {
+#pragma unroll
+    for (int k = 0; k < K; ++k) part[(size_t)K * blockIdx.x + k] = v[k];
+    __threadfence();
+    last = atomicAdd(tickets + blockIdx.y, 1u) == gridDim.x - 1;
+  }
+  if (!__shfl_sync(0xffffffffu, last, 0)) return false;
+  __threadfence();
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    double a = lane < s.nb ? __ldcg(part + (size_t)K * lane + k) : 0.0;
+    if (lane + 32 < s.nb) a += __ldcg(part + (size_t)K * (lane + 32) + k);
+    out[k] = a;
+  }
+  warp_sums<K>(out);
+  if (lane != 0) return false;
+  tickets[blockIdx.y] = 0u;
+  return true;
 }
 
-#define FOR_SYS(e, s)                                                     \
-  const int sy = blockIdx.y;                                              \
-  const size_t base = (size_t)sy * (s).n;                                 \
-  for (size_t e = base + (size_t)blockIdx.x * NT + threadIdx.x; e < base + (s).n; e += (size_t)(s).nb * NT)
+// The element passes below are read and write streams of a few vectors with one
+// or two float64 dots.  A thread takes kE = 8 elements at a time in accesses of
+// W (4: 128 bits, where the image size and every array allow it; else 1), all
+// loads of a group before its arithmetic, so that one memory latency covers a
+// whole image of 256^2 (32 blocks); dots go through ct::dot_group.
+// H^T H v is taken as the adjoint left it: the view splits are summed here, in
+// split order, instead of by a pass of their own.  16 images of 256^2, 6 steps,
+// forward and backward: 3.24 -> 2.82 ms with the projections, which did not
+// change (3.00 ms with each element's dot term converted to float64); one image
+// of 256^2 0.95 -> 0.68 ms, odd sizes (5 x 255^2, W = 1) 1.27 -> 1.04 ms.
+constexpr int kE = 8;
 
+struct Gram {        // H^T H v: `ns` partial images `stride` floats apart
+  const float* t;
+  int ns;
+  size_t stride;
+};
+
+template <int W>
+__device__ __forceinline__ void ld(const float* p, size_t e0, size_t step, size_t end, float (&v)[kE]) {
+#pragma unroll
+  for (int u = 0; u < kE / W; ++u) {
+    const size_t e = e0 + u * step;
+    if constexpr (W == 4) {
+      const float4 q = e < end ? *reinterpret_cast<const float4*>(p + e) : make_float4(0.f, 0.f, 0.f, 0.f);
+      v[4 * u] = q.x, v[4 * u + 1] = q.y, v[4 * u + 2] = q.z, v[4 * u + 3] = q.w;
+    } else {
+      v[u] = e < end ? p[e] : 0.0f;
+    }
+  }
+}
+
+template <int W>
+__device__ __forceinline__ void st(float* p, size_t e0, size_t step, size_t end, const float (&v)[kE]) {
+#pragma unroll
+  for (int u = 0; u < kE / W; ++u) {
+    const size_t e = e0 + u * step;
+    if (e < end) {
+      if constexpr (W == 4)
+        *reinterpret_cast<float4*>(p + e) = make_float4(v[4 * u], v[4 * u + 1], v[4 * u + 2], v[4 * u + 3]);
+      else
+        p[e] = v[u];
+    }
+  }
+}
+
+template <int W>
+__device__ __forceinline__ void ld(const Gram& g, size_t e0, size_t step, size_t end, float (&v)[kE]) {
+  ld<W>(g.t, e0, step, end, v);
+#pragma unroll 4
+  for (int k = 1; k < g.ns; ++k) {
+    float w[kE];
+    ld<W>(g.t + (size_t)k * g.stride, e0, step, end, w);
+#pragma unroll
+    for (int j = 0; j < kE; ++j) v[j] = ct::fadd(v[j], w[j]);
+  }
+}
+
+#define FOR_SYS(W, e, s)                                                                           \
+  const int sy = blockIdx.y;                                                                       \
+  const size_t end = (size_t)(sy + 1) * (s).n, step = (size_t)(s).nb * NT * (W);                   \
+  for (size_t e = (size_t)sy * (s).n + ((size_t)blockIdx.x * NT + threadIdx.x) * (W); e < end;     \
+       e += (kE / (W)) * step)
+#define EACH(j) _Pragma("unroll") for (int j = 0; j < kE; ++j)
+
+// x = x0 (or 0);  r_0 = p_0 = b - (gs t + lam x0) (or b);  num = <r_0, r_0>.
+template <int W>
 __global__ void __launch_bounds__(NT)
-    k_cgb_init(const float* __restrict__ b, const float* __restrict__ ax0, float* __restrict__ r0,
-               float* __restrict__ p0, Sys s, double* __restrict__ scal, double* __restrict__ partials,
-               unsigned int* __restrict__ tickets) {
+    k_cgb_init(const float* __restrict__ b, Gram t, const float* x0, float* x, float* __restrict__ r0,
+               float* __restrict__ p0, float gs, float lam, Sys s, double* __restrict__ scal,
+               double* __restrict__ partials, unsigned int* __restrict__ tickets) {
+  ct::grid_dep_wait();  // before any global access (dependent launch)
+  ct::grid_dep_trigger();
   double nn = 0.0;
-  FOR_SYS(e, s) {
-    const float r = ax0 ? ct::fsub(b[e], ax0[e]) : b[e];
-    r0[e] = r;
-    p0[e] = r;
-    nn += (double)r * (double)r;
+  FOR_SYS(W, e, s) {
+    float r[kE], xv[kE] = {};
+    ld<W>(b, e, step, end, r);
+    if (x0) {
+      float tv[kE];
+      ld<W>(t, e, step, end, tv);
+      ld<W>(x0, e, step, end, xv);
+      EACH(j) r[j] = ct::fsub(r[j], ct::fadd(ct::fmul(gs, tv[j]), ct::fmul(lam, xv[j])));
+    }
+    st<W>(x, e, step, end, xv);
+    st<W>(r0, e, step, end, r);
+    st<W>(p0, e, step, end, r);
+    nn += ct::dot_group(r, r);
   }
   double v[1] = {nn}, out[1];
   if (sys_reduce<1>(v, partials, tickets, s, out)) sys_scal(scal, s, sy)[C_NUM] = out[0];
 }
 
-// ax = gs t + lam x (t = H^T H x); ax may be t itself.
-__global__ void __launch_bounds__(NT)
-    k_cgb_axpy(const float* t, const float* __restrict__ x, float* ax, float gs, float lam, Sys s) {
-  FOR_SYS(e, s) ax[e] = ct::fadd(ct::fmul(gs, t[e]), ct::fmul(lam, x[e]));
-}
-
 // Ap = gs t + lam p (t = H^T H p), d = <p, Ap>, a = num / d.
+template <int W>
 __global__ void __launch_bounds__(NT)
-    k_cgb_ap(const float* __restrict__ t, const float* __restrict__ p, float* __restrict__ ap, float gs, float lam,
-             int k, Sys s, double* __restrict__ scal, double* __restrict__ partials, unsigned int* __restrict__ tickets) {
+    k_cgb_ap(Gram t, const float* __restrict__ p, float* __restrict__ ap, float gs, float lam, int k, Sys s,
+             double* __restrict__ scal, double* __restrict__ partials, unsigned int* __restrict__ tickets) {
+  ct::grid_dep_wait();  // before any global access (dependent launch)
+  ct::grid_dep_trigger();
   double d = 0.0;
-  FOR_SYS(e, s) {
-    const float pe = p[e];
-    const float a = ct::fadd(ct::fmul(gs, t[e]), ct::fmul(lam, pe));
-    ap[e] = a;
-    d += (double)pe * (double)a;
+  FOR_SYS(W, e, s) {
+    float a[kE], pv[kE];
+    ld<W>(p, e, step, end, pv);
+    ld<W>(t, e, step, end, a);
+    EACH(j) a[j] = ct::fadd(ct::fmul(gs, a[j]), ct::fmul(lam, pv[j]));
+    st<W>(ap, e, step, end, a);
+    d += ct::dot_group(pv, a);
   }
   double v[1] = {d}, out[1];
   if (sys_reduce<1>(v, partials, tickets, s, out)) {
@@ -102,17 +222,28 @@ __global__ void __launch_bounds__(NT)
 }
 
 // x += a p; r' = r - a Ap; num' = <r', r'>; b = num' / num.
+template <int W>
 __global__ void __launch_bounds__(NT)
     k_cgb_upd(float* __restrict__ x, const float* __restrict__ r, float* __restrict__ rn, const float* __restrict__ p,
               const float* __restrict__ ap, int k, Sys s, double* __restrict__ scal, double* __restrict__ partials,
               unsigned int* __restrict__ tickets) {
+  ct::grid_dep_wait();  // before any global access (dependent launch)
+  ct::grid_dep_trigger();
   const float a = (float)rec(scal, s, blockIdx.y, k)[R_A];
   double nn = 0.0;
-  FOR_SYS(e, s) {
-    x[e] = ct::fadd(x[e], ct::fmul(a, p[e]));
-    const float v = ct::fsub(r[e], ct::fmul(a, ap[e]));
-    rn[e] = v;
-    nn += (double)v * (double)v;
+  FOR_SYS(W, e, s) {
+    float xv[kE], rv[kE], pv[kE], av[kE];
+    ld<W>(x, e, step, end, xv);
+    ld<W>(p, e, step, end, pv);
+    ld<W>(r, e, step, end, rv);
+    ld<W>(ap, e, step, end, av);
+    EACH(j) {
+      xv[j] = ct::fadd(xv[j], ct::fmul(a, pv[j]));
+      rv[j] = ct::fsub(rv[j], ct::fmul(a, av[j]));
+    }
+    st<W>(x, e, step, end, xv);
+    st<W>(rn, e, step, end, rv);
+    nn += ct::dot_group(rv, rv);
   }
   double v[1] = {nn}, out[1];
   if (sys_reduce<1>(v, partials, tickets, s, out)) {
@@ -124,11 +255,20 @@ __global__ void __launch_bounds__(NT)
 }
 
 // p' = r' + b p.
+template <int W>
 __global__ void __launch_bounds__(NT)
     k_cgb_dir(const float* __restrict__ rn, const float* __restrict__ p, float* __restrict__ pn, int k, Sys s,
               double* __restrict__ scal) {
+  ct::grid_dep_wait();  // before any global access (dependent launch)
+  ct::grid_dep_trigger();
   const float bt = (float)rec(scal, s, blockIdx.y, k)[R_B];
-  FOR_SYS(e, s) pn[e] = ct::fadd(rn[e], ct::fmul(bt, p[e]));
+  FOR_SYS(W, e, s) {
+    float rv[kE], pv[kE];
+    ld<W>(rn, e, step, end, rv);
+    ld<W>(p, e, step, end, pv);
+    EACH(j) pv[j] = ct::fadd(rv[j], ct::fmul(bt, pv[j]));
+    st<W>(pn, e, step, end, pv);
+  }
 }
 
 // The backward's running scalars (numb, lamb) start at zero.
@@ -139,23 +279,30 @@ __global__ void k_cgb_reset(double* __restrict__ scal, Sys s) {
   }
 }
 
-// pb += gs t + lam Apb (the A Apb term of the previous backward step, when
-// t != null); then, for k >= 0: bb = <pb, p_k>, numb' = numb + bb / num_k,
-// nk = -bb num_{k+1} / num_k^2.
+// pb += gs t + lam Apb (the A Apb term of the previous backward step; pb = 0
+// and no such term in the first, t.t == null);  bb = <pb, p_k>,
+// numb' = numb + bb / num_k, nk = -bb num_{k+1} / num_k^2.
+template <int W>
 __global__ void __launch_bounds__(NT)
-    k_cgb_b1(float* __restrict__ pb, const float* __restrict__ t, const float* __restrict__ apb, float gs, float lam,
+    k_cgb_b1(float* __restrict__ pb, Gram t, const float* __restrict__ apb, float gs, float lam,
              const float* __restrict__ pk, int k, Sys s, double* __restrict__ scal, double* __restrict__ partials,
              unsigned int* __restrict__ tickets) {
+  ct::grid_dep_wait();  // before any global access (dependent launch)
+  ct::grid_dep_trigger();
   double bb = 0.0;
-  FOR_SYS(e, s) {
-    float v = pb[e];
-    if (t) {
-      v = ct::fadd(v, ct::fadd(ct::fmul(gs, t[e]), ct::fmul(lam, apb[e])));
-      pb[e] = v;
+  FOR_SYS(W, e, s) {
+    float v[kE] = {}, pv[kE];
+    ld<W>(pk, e, step, end, pv);
+    if (t.t) {
+      float tv[kE], gv[kE];
+      ld<W>(pb, e, step, end, v);
+      ld<W>(apb, e, step, end, gv);
+      ld<W>(t, e, step, end, tv);
+      EACH(j) v[j] = ct::fadd(v[j], ct::fadd(ct::fmul(gs, tv[j]), ct::fmul(lam, gv[j])));
     }
-    if (k >= 0) bb += (double)v * (double)pk[e];
+    st<W>(pb, e, step, end, v);
+    bb += ct::dot_group(v, pv);
   }
-  if (k < 0) return;  // uniform over the grid
   double v[1] = {bb}, out[1];
   if (sys_reduce<1>(v, partials, tickets, s, out)) {
     double* c = sys_scal(scal, s, sy);
@@ -165,19 +312,29 @@ __global__ void __launch_bounds__(NT)
   }
 }
 
-// rb += pb + 2 numb' r_{k+1};  ab = <xb, p_k> - <rb, Ap_k>;
-// numb = nk + ab / d_k;  db = -ab num_k / d_k^2.
+// rb += pb + 2 numb' r_{k+1} (rb = 0 before the first step);
+// ab = <xb, p_k> - <rb, Ap_k>;  numb = nk + ab / d_k;  db = -ab num_k / d_k^2.
+template <int W>
 __global__ void __launch_bounds__(NT)
-    k_cgb_b2(float* __restrict__ rb, const float* __restrict__ pb, const float* __restrict__ rn,
+    k_cgb_b2(float* __restrict__ rb, int first, const float* __restrict__ pb, const float* __restrict__ rn,
              const float* __restrict__ xb, const float* __restrict__ pk, const float* __restrict__ apk, int k, Sys s,
              double* __restrict__ scal, double* __restrict__ partials, unsigned int* __restrict__ tickets) {
+  ct::grid_dep_wait();  // before any global access (dependent launch)
+  ct::grid_dep_trigger();
   const float tn = (float)(2.0 * sys_scal(scal, s, blockIdx.y)[C_NUMB]);
   double s_xp = 0.0, s_ra = 0.0;
-  FOR_SYS(e, s) {
-    const float v = ct::fadd(ct::fadd(rb[e], pb[e]), ct::fmul(tn, rn[e]));
-    rb[e] = v;
-    s_xp += (double)xb[e] * (double)pk[e];
-    s_ra += (double)v * (double)apk[e];
+  FOR_SYS(W, e, s) {
+    float v[kE] = {}, w[kE], q[kE], xv[kE], pv[kE], av[kE];
+    if (!first) ld<W>(rb, e, step, end, v);
+    ld<W>(pb, e, step, end, w);
+    ld<W>(rn, e, step, end, q);
+    ld<W>(xb, e, step, end, xv);
+    ld<W>(pk, e, step, end, pv);
+    ld<W>(apk, e, step, end, av);
+    EACH(j) v[j] = ct::fadd(ct::fadd(v[j], w[j]), ct::fmul(tn, q[j]));
+    st<W>(rb, e, step, end, v);
+    s_xp += ct::dot_group(xv, pv);
+    s_ra += ct::dot_group(v, av);
   }
   double v[2] = {s_xp, s_ra}, out[2];
   if (sys_reduce<2>(v, partials, tickets, s, out)) {
@@ -190,42 +347,82 @@ __global__ void __launch_bounds__(NT)
 }
 
 // Apb = -a_k rb + db p_k;  pb = b_k pb + a_k xb + db Ap_k;  lamb += <Apb, p_k>.
+template <int W>
 __global__ void __launch_bounds__(NT)
     k_cgb_b3(const float* __restrict__ rb, const float* __restrict__ xb, float* __restrict__ pb,
              float* __restrict__ apb, const float* __restrict__ pk, const float* __restrict__ apk, int k, Sys s,
              double* __restrict__ scal, double* __restrict__ partials, unsigned int* __restrict__ tickets) {
+  ct::grid_dep_wait();  // before any global access (dependent launch)
+  ct::grid_dep_trigger();
   const double* r = rec(scal, s, blockIdx.y, k);
   const float a = (float)r[R_A], bt = (float)r[R_B], db = (float)sys_scal(scal, s, blockIdx.y)[C_DB];
   double lb = 0.0;
-  FOR_SYS(e, s) {
-    const float p = pk[e];
-    const float g = ct::fadd(ct::fmul(-a, rb[e]), ct::fmul(db, p));
-    apb[e] = g;
-    pb[e] = ct::fadd(ct::fadd(ct::fmul(bt, pb[e]), ct::fmul(a, xb[e])), ct::fmul(db, apk[e]));
-    lb += (double)g * (double)p;
+  FOR_SYS(W, e, s) {
+    float g[kE], xv[kE], bv[kE], pv[kE], av[kE];
+    ld<W>(rb, e, step, end, g);
+    ld<W>(pk, e, step, end, pv);
+    ld<W>(pb, e, step, end, bv);
+    ld<W>(xb, e, step, end, xv);
+    ld<W>(apk, e, step, end, av);
+    EACH(j) {
+      g[j] = ct::fadd(ct::fmul(-a, g[j]), ct::fmul(db, pv[j]));
+      bv[j] = ct::fadd(ct::fadd(ct::fmul(bt, bv[j]), ct::fmul(a, xv[j])), ct::fmul(db, av[j]));
+    }
+    st<W>(apb, e, step, end, g);
+    st<W>(pb, e, step, end, bv);
+    lb += ct::dot_group(g, pv);
   }
   double v[1] = {lb}, out[1];
   if (sys_reduce<1>(v, partials, tickets, s, out)) sys_scal(scal, s, sy)[C_LAMB] += out[0];
 }
 
-// gb = rb + pb + 2 numb r_0 (the adjoint of r_0, which is that of b).
+// gb = rb + (pb + gs t + lam Apb) + 2 numb r_0 (the adjoint of r_0, which is
+// that of b); rb = pb = 0 and no A Apb term where no step ran (t.t == null).
+template <int W>
 __global__ void __launch_bounds__(NT)
-    k_cgb_rb0(const float* __restrict__ rb, const float* __restrict__ pb, const float* __restrict__ r0,
-              float* __restrict__ gb, Sys s, double* __restrict__ scal) {
+    k_cgb_rb0(const float* __restrict__ rb, const float* __restrict__ pb, Gram t, const float* __restrict__ apb,
+              float gs, float lam, const float* __restrict__ r0, float* __restrict__ gb, Sys s,
+              double* __restrict__ scal) {
+  ct::grid_dep_wait();  // before any global access (dependent launch)
+  ct::grid_dep_trigger();
   const float tn = (float)(2.0 * sys_scal(scal, s, blockIdx.y)[C_NUMB]);
-  FOR_SYS(e, s) gb[e] = ct::fadd(ct::fadd(rb[e], pb[e]), ct::fmul(tn, r0[e]));
+  FOR_SYS(W, e, s) {
+    float v[kE] = {}, w[kE] = {}, q[kE];
+    ld<W>(r0, e, step, end, q);
+    if (t.t) {
+      float tv[kE], gv[kE];
+      ld<W>(rb, e, step, end, v);
+      ld<W>(pb, e, step, end, w);
+      ld<W>(apb, e, step, end, gv);
+      ld<W>(t, e, step, end, tv);
+      EACH(j) w[j] = ct::fadd(w[j], ct::fadd(ct::fmul(gs, tv[j]), ct::fmul(lam, gv[j])));
+    }
+    EACH(j) v[j] = ct::fadd(ct::fadd(v[j], w[j]), ct::fmul(tn, q[j]));
+    st<W>(gb, e, step, end, v);
+  }
 }
 
 // gx0 = xb - (gs t + lam gb) (t = H^T H gb, gx0 may be null);  lamb -= <gb, x0>.
+template <int W>
 __global__ void __launch_bounds__(NT)
-    k_cgb_x0(const float* __restrict__ xb, const float* __restrict__ t, const float* __restrict__ gb,
-             const float* __restrict__ x0, float* __restrict__ gx0, float gs, float lam, Sys s,
-             double* __restrict__ scal, double* __restrict__ partials, unsigned int* __restrict__ tickets) {
+    k_cgb_x0(const float* __restrict__ xb, Gram t, const float* __restrict__ gb, const float* __restrict__ x0,
+             float* __restrict__ gx0, float gs, float lam, Sys s, double* __restrict__ scal,
+             double* __restrict__ partials, unsigned int* __restrict__ tickets) {
+  ct::grid_dep_wait();  // before any global access (dependent launch)
+  ct::grid_dep_trigger();
   double lb = 0.0;
-  FOR_SYS(e, s) {
-    const float g = gb[e];
-    if (gx0) gx0[e] = ct::fsub(xb[e], ct::fadd(ct::fmul(gs, t[e]), ct::fmul(lam, g)));
-    lb += (double)g * (double)x0[e];
+  FOR_SYS(W, e, s) {
+    float g[kE], xv[kE];
+    ld<W>(gb, e, step, end, g);
+    ld<W>(x0, e, step, end, xv);
+    if (gx0) {
+      float tv[kE], bv[kE];
+      ld<W>(xb, e, step, end, bv);
+      ld<W>(t, e, step, end, tv);
+      EACH(j) bv[j] = ct::fsub(bv[j], ct::fadd(ct::fmul(gs, tv[j]), ct::fmul(lam, g[j])));
+      st<W>(gx0, e, step, end, bv);
+    }
+    lb += ct::dot_group(g, xv);
   }
   double v[1] = {lb}, out[1];
   if (sys_reduce<1>(v, partials, tickets, s, out)) sys_scal(scal, s, sy)[C_LAMB] -= out[0];
@@ -258,7 +455,7 @@ struct Plan {
 
 // Tape: P[K], AP[K], R[K+1] (none with recompute), then the scalars.
 // Workspace: reduction area, projector scratch, sinogram, t and the
-// backward's rb, pb, xb, apb, gb; with recompute also P, AP, R and x.
+// backward's rb, pb, apb; with recompute also P, AP, R and x.
 Plan plan_of(const ct_cg_block_desc* d) {
   Plan P;
   const size_t n = (size_t)d->geom.rows * d->geom.cols;
@@ -277,7 +474,7 @@ Plan plan_of(const ct_cg_block_desc* d) {
              ct::round_up((size_t)d->nsys * 4 * P.s.nb * sizeof(double), 256);
   P.ws_proj = ct::round_up(std::max<size_t>(std::max(P.p2.fwd_bytes, P.p2.adj_ws_bytes), 256), 256);
   P.ws_sino = ct::round_up((size_t)d->nsys * d->geom.n_views * d->geom.det_count * sizeof(float), 256);
-  P.ws_tmp = 6 * P.vec;
+  P.ws_tmp = 4 * P.vec;
   P.ws_recompute = d->recompute ? vectors + P.vec : 0;
   P.ws_total = P.ws_red + P.ws_proj + P.ws_sino + P.ws_tmp + P.ws_recompute;
   return P;
@@ -297,7 +494,7 @@ struct Bufs {
   double* partials;
   float* proj_ws;
   float* sino;
-  float *t, *rb, *pb, *xb, *apb, *gb;
+  float *t, *rb, *pb, *apb;
   float *P, *AP, *R, *x;  // iterates: the tape's, or the workspace's with recompute
   double* scal;
 };
@@ -312,14 +509,10 @@ Bufs bufs(const ct_cg_block_desc* d, const Plan& P, void* tape, void* ws, float*
   q += P.ws_proj;
   B.sino = reinterpret_cast<float*>(q);
   q += P.ws_sino;
-  float* tmp[6];
-  for (int i = 0; i < 6; ++i) tmp[i] = reinterpret_cast<float*>(q + i * P.vec);
-  B.t = tmp[0];
-  B.rb = tmp[1];
-  B.pb = tmp[2];
-  B.xb = tmp[3];
-  B.apb = tmp[4];
-  B.gb = tmp[5];
+  B.t = reinterpret_cast<float*>(q);
+  B.rb = reinterpret_cast<float*>(q + P.vec);
+  B.pb = reinterpret_cast<float*>(q + 2 * P.vec);
+  B.apb = reinterpret_cast<float*>(q + 3 * P.vec);
   q += P.ws_tmp;
   char* vec = d->recompute ? q : static_cast<char*>(tape);
   const int K = d->maxiter;
@@ -335,49 +528,43 @@ float* at(float* base, const Plan& P, int k) {
   return reinterpret_cast<float*>(reinterpret_cast<char*>(base) + (size_t)k * P.vec);
 }
 
-// t = H^T H v for the batch (forward projection, then adjoint with its view
-// splits summed in order).
-ct_status gram(const ct_cg_block_desc* d, const Plan& P, const Bufs& B, const float* v, float* t, cudaStream_t s) {
-  CT_TRY(ct::proj2d_fwd_launch(&d->geom, P.p2, v, B.sino, d->nsys, B.proj_ws, s, nullptr));
-  CT_TRY(ct::proj2d_adj_launch(&d->geom, P.p2, B.sino, t, B.proj_ws, d->nsys, s, nullptr));
-  if (P.p2.nsplit > 1) CT_TRY(ct::proj2d_sum_splits(B.proj_ws, t, (size_t)d->nsys * P.s.n, P.p2.nsplit, s));
+// t = H^T H v for the batch: forward projection, then the adjoint, whose view
+// splits the next pass sums.  v is the output of one of this file's kernels
+// (dependent) or the caller's.
+ct_status gram(const ct_cg_block_desc* d, const Plan& P, const Bufs& B, const float* v, Gram& t, cudaStream_t s,
+               bool dependent) {
+  CT_TRY(ct::proj2d_fwd_launch(&d->geom, P.p2, v, B.sino, d->nsys, B.proj_ws, s, nullptr, dependent));
+  CT_TRY(ct::proj2d_adj_launch(&d->geom, P.p2, B.sino, B.t, B.proj_ws, d->nsys, s, nullptr, true));
+  t = Gram{P.p2.nsplit > 1 ? B.proj_ws : B.t, P.p2.nsplit, (size_t)d->nsys * P.s.n};
   return CT_OK;
 }
 
-dim3 grid_of(const Plan& P) { return dim3((unsigned)P.s.nb, (unsigned)P.s.nsys, 1); }
+// A pass over all systems in its W = 4 form where `vec`, else in its W = 1 form.
+template <class... K, class... A>
+ct_status pass(const char* name, const Plan& P, cudaStream_t s, bool dependent, int vec, void (*k4)(K...),
+               void (*k1)(K...), A... args) {
+  const dim3 g((unsigned)P.s.nb, (unsigned)P.s.nsys, 1);
+  return ct::cuda_check(ct::launch_k(vec ? k4 : k1, g, dim3(NT), 0, s, dependent, args...), name);
+}
+#define PASS(k, dependent, vec, ...) CT_TRY(pass(#k, P, s, dependent, vec, k<4>, k<1>, __VA_ARGS__))
 
 ct_status forward(const ct_cg_block_desc* d, const Plan& P, const Bufs& B, const float* b, float lam,
                   const float* x0, cudaStream_t s) {
-  const size_t nbytes = (size_t)d->nsys * P.s.n * sizeof(float);
   const float gs = d->gram_scale;
-  const dim3 g = grid_of(P);
-  const float* ax0 = nullptr;
-  if (x0) {
-    CT_TRY(ct::cuda_check(cudaMemcpyAsync(B.x, x0, nbytes, cudaMemcpyDeviceToDevice, s), "x0 copy"));
-    CT_TRY(gram(d, P, B, x0, B.t, s));
-    k_cgb_axpy<<<g, NT, 0, s>>>(B.t, x0, B.t, gs, lam, P.s);  // A x0, in place of t
-    CT_TRY(ct::launch_check("k_cgb_axpy"));
-    ax0 = B.t;
-  } else {
-    CT_TRY(ct::cuda_check(cudaMemsetAsync(B.x, 0, nbytes, s), "x0 zero"));
-  }
+  const int vec = ct::quad_ok(P.s.n, b, x0, B.x);  // the tape and workspace vectors are 256-B aligned
+  Gram t{};
+  if (x0) CT_TRY(gram(d, P, B, x0, t, s, false));
   const int K = d->maxiter;
-  k_cgb_init<<<g, NT, 0, s>>>(b, ax0, at(B.R, P, 0), K > 0 ? at(B.P, P, 0) : B.pb, P.s, B.scal, B.partials,
-                              B.tickets);
-  CT_TRY(ct::launch_check("k_cgb_init"));
+  PASS(k_cgb_init, x0 != nullptr, vec, b, t, x0, B.x, at(B.R, P, 0), K > 0 ? at(B.P, P, 0) : B.pb, gs, lam, P.s,
+       B.scal, B.partials, B.tickets);
   for (int k = 0; k < K; ++k) {
     float* pk = at(B.P, P, k);
     float* apk = at(B.AP, P, k);
-    CT_TRY(gram(d, P, B, pk, B.t, s));
-    k_cgb_ap<<<g, NT, 0, s>>>(B.t, pk, apk, gs, lam, k, P.s, B.scal, B.partials, B.tickets);
-    CT_TRY(ct::launch_check("k_cgb_ap"));
-    k_cgb_upd<<<g, NT, 0, s>>>(B.x, at(B.R, P, k), at(B.R, P, k + 1), pk, apk, k, P.s, B.scal, B.partials,
-                               B.tickets);
-    CT_TRY(ct::launch_check("k_cgb_upd"));
-    if (k + 1 < K) {
-      k_cgb_dir<<<g, NT, 0, s>>>(at(B.R, P, k + 1), pk, at(B.P, P, k + 1), k, P.s, B.scal);
-      CT_TRY(ct::launch_check("k_cgb_dir"));
-    }
+    CT_TRY(gram(d, P, B, pk, t, s, true));
+    PASS(k_cgb_ap, true, vec, t, pk, apk, gs, lam, k, P.s, B.scal, B.partials, B.tickets);
+    PASS(k_cgb_upd, true, vec, B.x, at(B.R, P, k), at(B.R, P, k + 1), pk, apk, k, P.s, B.scal, B.partials, B.tickets);
+    if (k + 1 < K)
+      PASS(k_cgb_dir, true, vec, at(B.R, P, k + 1), pk, at(B.P, P, k + 1), k, P.s, B.scal);
   }
   return CT_OK;
 }
@@ -438,39 +625,26 @@ ct_status ct_cg_block_bwd(const ct_cg_block_desc* d, const float* gx, const floa
   CT_TRY(ct::cuda_check(cudaMemsetAsync(workspace, 0, P.ws_red, s), "reduction init"));
   const Bufs B = bufs(d, P, tape, workspace, nullptr);
   if (d->recompute) CT_TRY(forward(d, P, B, b, lam, x0, s));  // the iterates from the block's inputs
-  const size_t nbytes = (size_t)d->nsys * P.s.n * sizeof(float);
   const float gs = d->gram_scale;
-  const dim3 g = grid_of(P);
-  CT_TRY(ct::cuda_check(cudaMemcpyAsync(B.xb, gx, nbytes, cudaMemcpyDeviceToDevice, s), "xb init"));
-  CT_TRY(ct::cuda_check(cudaMemsetAsync(B.rb, 0, nbytes, s), "rb init"));
-  CT_TRY(ct::cuda_check(cudaMemsetAsync(B.pb, 0, nbytes, s), "pb init"));
+  const int vec = ct::quad_ok(P.s.n, gx, x0, gb, gx0);
   k_cgb_reset<<<1, 256, 0, s>>>(B.scal, P.s);
   CT_TRY(ct::launch_check("k_cgb_reset"));
   const int K = d->maxiter;
-  bool pending = false;  // B.t holds H^T H apb of the previous backward step
+  Gram t{};  // H^T H apb of the previous backward step
   for (int k = K - 1; k >= 0; --k) {
     const float* pk = at(B.P, P, k);
     const float* apk = at(B.AP, P, k);
-    k_cgb_b1<<<g, NT, 0, s>>>(B.pb, pending ? B.t : nullptr, B.apb, gs, lam, pk, k, P.s, B.scal, B.partials,
-                              B.tickets);
-    CT_TRY(ct::launch_check("k_cgb_b1"));
-    k_cgb_b2<<<g, NT, 0, s>>>(B.rb, B.pb, at(B.R, P, k + 1), B.xb, pk, apk, k, P.s, B.scal, B.partials, B.tickets);
-    CT_TRY(ct::launch_check("k_cgb_b2"));
-    k_cgb_b3<<<g, NT, 0, s>>>(B.rb, B.xb, B.pb, B.apb, pk, apk, k, P.s, B.scal, B.partials, B.tickets);
-    CT_TRY(ct::launch_check("k_cgb_b3"));
-    CT_TRY(gram(d, P, B, B.apb, B.t, s));
-    pending = true;
+    const int first = k == K - 1;
+    PASS(k_cgb_b1, !first, vec, B.pb, t, B.apb, gs, lam, pk, k, P.s, B.scal, B.partials, B.tickets);
+    PASS(k_cgb_b2, true, vec, B.rb, first, B.pb, at(B.R, P, k + 1), gx, pk, apk, k, P.s, B.scal, B.partials,
+         B.tickets);
+    PASS(k_cgb_b3, true, vec, B.rb, gx, B.pb, B.apb, pk, apk, k, P.s, B.scal, B.partials, B.tickets);
+    CT_TRY(gram(d, P, B, B.apb, t, s, true));
   }
-  if (pending) {
-    k_cgb_b1<<<g, NT, 0, s>>>(B.pb, B.t, B.apb, gs, lam, nullptr, -1, P.s, B.scal, B.partials, B.tickets);
-    CT_TRY(ct::launch_check("k_cgb_b1"));
-  }
-  k_cgb_rb0<<<g, NT, 0, s>>>(B.rb, B.pb, at(B.R, P, 0), gb, P.s, B.scal);
-  CT_TRY(ct::launch_check("k_cgb_rb0"));
+  PASS(k_cgb_rb0, K > 0, vec, B.rb, B.pb, t, B.apb, gs, lam, at(B.R, P, 0), gb, P.s, B.scal);
   if (x0) {
-    CT_TRY(gram(d, P, B, gb, B.t, s));
-    k_cgb_x0<<<g, NT, 0, s>>>(B.xb, B.t, gb, x0, gx0, gs, lam, P.s, B.scal, B.partials, B.tickets);
-    CT_TRY(ct::launch_check("k_cgb_x0"));
+    CT_TRY(gram(d, P, B, gb, t, s, true));
+    PASS(k_cgb_x0, true, vec, gx, t, gb, x0, gx0, gs, lam, P.s, B.scal, B.partials, B.tickets);
   }
   k_cgb_lamsum<<<1, 1, 0, s>>>(B.scal, P.s, glam);
   return ct::launch_check("k_cgb_lamsum");

@@ -129,6 +129,54 @@ struct KSum {
   __device__ __forceinline__ double value() const { return (double)s - (double)c; }
 };
 
+// <a, b> of one thread's group of N elements, to better than float64 keeps it
+// but with six float64 operations a group where converting and accumulating
+// each element takes three an element (the float64 pipe of this GPU, two
+// results a clock and SM, otherwise sets the pace of every pass with a dot).
+// Each product splits exactly into float32 value and error (the error by an
+// FMA); the values are summed with Knuth's two-sum, then their errors and the
+// two-sums' errors likewise, and what that second sum rounds off goes into a
+// third: about 2^-66 of sum |a_j b_j| is lost, 2^-53 an addition in float64.
+// Where the largest product is not in [2^-70, 2^120] -- there the float32
+// errors could underflow or the sums overflow -- the group is summed in
+// float64 element by element.
+__device__ __forceinline__ void two_sum(float& s, float b, float& e) {
+  const float t = __fadd_rn(s, b), bb = __fsub_rn(t, s);
+  e = __fadd_rn(__fsub_rn(s, __fsub_rn(t, bb)), __fsub_rn(b, bb));
+  s = t;
+}
+
+template <int N>
+__device__ __forceinline__ double dot_group(const float (&a)[N], const float (&b)[N]) {
+  float p[N], top = 0.0f;
+#pragma unroll
+  for (int j = 0; j < N; ++j) {
+    p[j] = __fmul_rn(a[j], b[j]);
+    top = fmaxf(top, fabsf(p[j]));
+  }
+  if (top >= 0x1p-70f && top <= 0x1p120f) {
+    float s = p[0], l = __fmaf_rn(a[0], b[0], -p[0]), m = 0.0f, e;
+#pragma unroll
+    for (int j = 1; j < N; ++j) {
+      two_sum(s, p[j], e);
+      float f;
+      two_sum(l, e, f);
+      m = __fadd_rn(m, f);
+      two_sum(l, __fmaf_rn(a[j], b[j], -p[j]), f);
+      m = __fadd_rn(m, f);
+    }
+    return ((double)m + (double)l) + (double)s;
+  }
+  float any = 0.0f;  // a zero group (an image's background) stays cheap; 0 times a NaN or an infinity does not pass
+#pragma unroll
+  for (int j = 0; j < N; ++j) any = __fadd_rn(any, __fadd_rn(fabsf(a[j]), fabsf(p[j])));
+  if (any == 0.0f) return 0.0;
+  double acc = 0.0;
+#pragma unroll
+  for (int j = 0; j < N; ++j) acc += (double)a[j] * (double)b[j];
+  return acc;
+}
+
 // ---------------------------------------------------------------------------
 // Deterministic float64 grid reduction of K simultaneous sums.  Every block
 // reduces its threads' values (fixed shuffle tree, warps in order) and
