@@ -566,15 +566,11 @@ __device__ __forceinline__ void lhs_pass(const float* adj, int nsplit, const flo
         for (int j = 0; j < 4; ++j) re[j] = ct::fsub(b[j], v[j]);
         st4(out, e0, re);  // r
         st4(p, e0, re);
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          acc[0] += (double)re[j] * (double)re[j];
-          acc[1] += (double)b[j] * (double)b[j];
-        }
+        acc[0] += ct::dot_group(re, re);
+        acc[1] += ct::dot_group(b, b);
       } else {
         st4(out, e0, v);  // Ap
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[0] += (double)qc[j] * (double)v[j];
+        acc[0] += ct::dot_group(qc, v);
       }
     }
   } else {
@@ -628,9 +624,12 @@ __global__ void __launch_bounds__(NT)
   const bool cached = INIT && slots[S_XCLEAN] != 0.0;
   double acc[2] = {0.0, 0.0};
   lhs_pass<ND, INIT, LdPlain>(adj, nsplit, q, sh, N, tp, out, rhs, p, lhsx, cached, vec, acc);
-  double tot[2];
-  if (ct::grid_sumk_last<NT, 2>(acc, partials, ticket, tot)) {
-    if (INIT) {
+  constexpr int KS = INIT ? 2 : 1;
+  double part[KS], tot[KS];
+#pragma unroll
+  for (int k = 0; k < KS; ++k) part[k] = acc[k];
+  if (ct::grid_sumk_last<NT, KS>(part, partials, ticket, tot)) {
+    if constexpr (INIT) {
       write_record(rp, slots);
       const double bn = sqrt(tot[1]);
       const double thr = fmax(tol * bn, atol);
@@ -916,7 +915,8 @@ __global__ void __launch_bounds__(NT, 2)
   ct::grid_dep_wait();  // before any global access (dependent launch)
   ct::grid_dep_trigger();
   using LDS = LdL2;  // state written by other blocks earlier in this launch
-  __shared__ double dec_s[2];
+  __shared__ double dec_s[3];  // ||r||^2, ||rhs||, squared threshold: one thread's float64 square root, not the block's
+  __shared__ bool done_s;
   // A block whose barrier wait runs out hands over to the graph's CG loop
   // and returns: the solve's results are void (the error word says so), and
   // the fused CG step then ends the loop on its own failed barrier, so every
@@ -957,13 +957,15 @@ __global__ void __launch_bounds__(NT, 2)
     double tot[2];
     ct::sum_partials<NT, 2>(fp + kFfInit, gridDim.x, tot, kFfK);
     if (threadIdx.x == 0) {
+      const double bn = sqrt(tot[1]);
+      const double thr = fmax(tol * bn, atol);
       dec_s[0] = tot[0];
-      dec_s[1] = tot[1];
+      dec_s[1] = bn;
+      dec_s[2] = thr * thr;
+      done_s = cg_maxiter <= 0 || !(tot[0] > thr * thr);
     }
     __syncthreads();
-    const double bn = sqrt(dec_s[1]);
-    const double thr = fmax(tol * bn, atol);
-    const bool done = cg_maxiter <= 0 || !(dec_s[0] > thr * thr);
+    const bool done = done_s;
     if (blockIdx.x == 0) {
       if (phase > 0) {  // k_rhs's total, before the record that reads it
         double d[1];
@@ -976,8 +978,8 @@ __global__ void __launch_bounds__(NT, 2)
         cg[CT_CG_PAP] = 0.0;
         cg[CT_CG_ALPHA] = 0.0;
         cg[CT_CG_BETA] = 0.0;
-        cg[CT_CG_BNORM] = bn;
-        cg[CT_CG_TOL2] = thr * thr;
+        cg[CT_CG_BNORM] = dec_s[1];
+        cg[CT_CG_TOL2] = dec_s[2];
         cg[CT_CG_ITERS] = 0.0;
         cg[CT_CG_MAXITER] = (double)cg_maxiter;
         cg[CT_CG_RAN] = 0.0;
@@ -1032,7 +1034,7 @@ __global__ void __launch_bounds__(NT, 2)
               int vec_update, int vec_dir, uint32_t max_polls, int* errflag) {
   ct::grid_dep_wait();  // before any global access (dependent launch)
   ct::grid_dep_trigger();
-  __shared__ double sum_s;
+  __shared__ float fac_s;
   // read by every block before the first barrier; block 0 writes them only after the second
   const double num = cg[CT_CG_NUM], it0 = cg[CT_CG_ITERS];
   const double tol2 = cg[CT_CG_TOL2], maxit = cg[CT_CG_MAXITER];
@@ -1054,26 +1056,29 @@ __global__ void __launch_bounds__(NT, 2)
   // Ap = lhs(p) and <p, Ap> (k_lhs_finish<PAP>)
   double acc[2] = {0.0, 0.0};
   lhs_pass<ND, false, LdPlain>(adj, nsplit, p, sh, N, tp, ap, nullptr, nullptr, nullptr, false, vec, acc);
-  ct::block_partials<NT, 2>(acc, part);
+  double t[1] = {acc[0]};
+  ct::block_partials<NT, 1>(t, part);
   if (!ct::grid_barrier(bar + 1, base + gridDim.x, max_polls, errflag, kErrBarrier)) return give_up();
-  double t[2];
-  ct::sum_partials<NT, 2>(part, gridDim.x, t);
-  if (threadIdx.x == 0) sum_s = t[0];
+  ct::sum_partials<NT, 1>(part, gridDim.x, t);
+  double pap = 0.0, alpha = 0.0;  // in thread 0: one float64 division a block
+  if (threadIdx.x == 0) {
+    pap = t[0];
+    alpha = num / pap;
+    fac_s = (float)alpha;
+  }
   __syncthreads();
-  const double pap = sum_s;
-  const double alpha = num / pap;
   // x += alpha p; r -= alpha Ap; <r, r> (k_cg_update)
-  double v2[2] = {ct::cg_update_pass(x, r, p, ap, N, (float)alpha, vec_update), 0.0};
-  ct::block_partials<NT, 2>(v2, part + 2 * NB);
+  t[0] = ct::cg_update_pass(x, r, p, ap, N, fac_s, vec_update);
+  ct::block_partials<NT, 1>(t, part + 2 * NB);
   if (!ct::grid_barrier(bar + 1, base + 2 * gridDim.x, max_polls, errflag, kErrBarrier)) return give_up();
-  ct::sum_partials<NT, 2>(part + 2 * NB, gridDim.x, t);
-  if (threadIdx.x == 0) sum_s = t[0];
+  ct::sum_partials<NT, 1>(part + 2 * NB, gridDim.x, t);
+  const double trr = t[0];  // in thread 0
+  const double beta = threadIdx.x == 0 ? trr / num : 0.0;
+  if (threadIdx.x == 0) fac_s = (float)beta;
   __syncthreads();
-  const double trr = sum_s;
-  const double beta = trr / num;
-  const double it = it0 + 1.0;
-  const bool done = !(trr > tol2) || it >= maxit;
   if (blockIdx.x == 0 && threadIdx.x == 0) {
+    const double it = it0 + 1.0;
+    const bool done = !(trr > tol2) || it >= maxit;
     cg[CT_CG_PAP] = pap;
     cg[CT_CG_ALPHA] = alpha;
     cg[CT_CG_NUM] = trr;
@@ -1086,7 +1091,7 @@ __global__ void __launch_bounds__(NT, 2)
   }
   // p = r + beta p (k_cg_direction): the direction update still runs in the
   // step that finds CG done (reference order)
-  ct::cg_direction_pass(p, r, N, (float)beta, vec_dir);
+  ct::cg_direction_pass(p, r, N, fac_s, vec_dir);
 }
 
 // ---------------------------------------------------------------------------

@@ -48,11 +48,11 @@ __device__ __forceinline__ double* rec(double* scal, const Sys& s, int sy, int k
 
 // Reduction of K (<= 4) sums over the blocks of one system (grid = (nb, nsys),
 // nb <= 64); true in thread 0 of the system's last block.  The block's first
-// warp finishes alone, both over the block's warps and, in the last block,
-// over the blocks' partials, in fixed shuffle trees: no thread adds a row of
-// float64 values one after the other and no second block-wide barrier stands
-// between the ticket and the result (as block_reduce has it for larger grids;
-// with that form the 16 images below take 2.88 instead of 2.82 ms).
+// warp adds the threads' values as ct::block_reduce does and finishes alone: no
+// block-wide barrier stands between the ticket and the result, and the last
+// block's sum over the partials is that warp's too (16 images below: 2.82 ms
+// with per-warp shuffle trees against 2.88 with grid_reduce_last as it was,
+// 2.80 with the adds in one warp).
 template <int K>
 __device__ __forceinline__ void warp_sums(double (&v)[K]) {
 #pragma unroll
@@ -65,23 +65,19 @@ __device__ __forceinline__ void warp_sums(double (&v)[K]) {
 template <int K>
 __device__ __forceinline__ bool sys_reduce(double (&v)[K], double* partials, unsigned int* tickets, const Sys& s,
                                            double (&out)[K]) {
-  constexpr int NW = NT / 32;
-  __shared__ double red[K][NW];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  warp_sums<K>(v);
-  if (lane == 0) {
+  __shared__ double red[K][NT];
+  const int lane = threadIdx.x;
 #pragma unroll
-    for (int k = 0; k < K; ++k) red[k][warp] = v[k];
-  }
+  for (int k = 0; k < K; ++k) red[k][threadIdx.x] = v[k];
   __syncthreads();
-  if (warp != 0) return false;
+  if (threadIdx.x >= 32) return false;
   double* part = partials + (size_t)blockIdx.y * 4 * s.nb;
 #pragma unroll
   for (int k = 0; k < K; ++k) {
-    v[k] = red[k][lane & (NW - 1)];
-#pragma unroll
-    for (int o = NW / 2; o > 0; o >>= 1) v[k] += __shfl_xor_sync(0xffffffffu, v[k], o);
+    const double* r = red[k] + lane;
+    v[k] = ((r[0] + r[32]) + (r[64] + r[96])) + ((r[128] + r[160]) + (r[192] + r[224]));
   }
+  warp_sums<K>(v);
   int last = 0;
   if (lane == 0) {
 #pragma unroll
@@ -110,7 +106,7 @@ __device__ __forceinline__ bool sys_reduce(double (&v)[K], double* partials, uns
 // whole image of 256^2 (32 blocks); dots go through ct::dot_group.
 // H^T H v is taken as the adjoint left it: the view splits are summed here, in
 // split order, instead of by a pass of their own.  16 images of 256^2, 6 steps,
-// forward and backward: 3.24 -> 2.82 ms with the projections, which did not
+// forward and backward: 3.24 -> 2.80 ms with the projections, which did not
 // change (3.00 ms with each element's dot term converted to float64); one image
 // of 256^2 0.95 -> 0.68 ms, odd sizes (5 x 255^2, W = 1) 1.27 -> 1.04 ms.
 constexpr int kE = 8;

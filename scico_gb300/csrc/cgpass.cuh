@@ -30,8 +30,8 @@ __device__ __forceinline__ double cg_update_pass(float* x, float* r, const float
       for (int j = 0; j < 4; ++j) {
         xv[j] = fadd(cgp_at4(x4, j), fmul(af, cgp_at4(p4, j)));
         rv[j] = fsub(cgp_at4(r4, j), fmul(af, cgp_at4(a4, j)));
-        rr += (double)rv[j] * (double)rv[j];
       }
+      rr += dot_group(rv, rv);
       cgp_st4(x, e0, make_float4(xv[0], xv[1], xv[2], xv[3]));
       cgp_st4(r, e0, make_float4(rv[0], rv[1], rv[2], rv[3]));
     };

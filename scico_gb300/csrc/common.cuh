@@ -117,7 +117,7 @@ __device__ __forceinline__ void boxcar2d(float px, float width, float inv_width,
 // terms within a few units of rounding, as a float64 accumulation would,
 // without float64 arithmetic per element (the float64 pipe of this GPU runs
 // at a small fraction of the float32 rate).  The CG dot products, which
-// steer the iteration, stay float64 per element.
+// steer the iteration, keep float64's accuracy per element (dot_group).
 struct KSum {
   float s = 0.0f, c = 0.0f;
   __device__ __forceinline__ void add(float v) {
@@ -179,7 +179,7 @@ __device__ __forceinline__ double dot_group(const float (&a)[N], const float (&b
 
 // ---------------------------------------------------------------------------
 // Deterministic float64 grid reduction of K simultaneous sums.  Every block
-// reduces its threads' values (fixed shuffle tree, warps in order) and
+// reduces its threads' values (in a fixed tree) and
 // writes K partials to partials[K*blockIdx.x + k]; the last block to finish
 // (integer ticket, so which block it is does not affect the value) sums the
 // partials with all its threads in a fixed pattern.  The ticket is reset by
@@ -187,23 +187,25 @@ __device__ __forceinline__ double dot_group(const float (&a)[N], const float (&b
 // without host involvement.  Returns true in thread 0 of the last block,
 // with `out` holding the K totals.
 // ---------------------------------------------------------------------------
+// The block's sums: every thread's value goes through shared memory and the
+// first warp adds them (eight a lane, then a shuffle tree), 13 warp-wide float64
+// additions a sum where a shuffle tree in each warp and a row of their totals
+// takes 48: the float64 pipe serves two lanes a clock, so these additions, not
+// their latency, set the time (with dot_group and one thread's divisions: a
+// CG step of the 512^2 / 360-view solve 120 -> 114 us, 88 of them projections).
+// The sums are valid in the first warp.
 template <int NT, int K>
-__device__ __forceinline__ void block_reduce(double (&v)[K], double (*red)[NT / 32]) {
+__device__ __forceinline__ void block_reduce(double (&v)[K], double (*red)[NT]) {
+  static_assert(NT == 256, "eight values a lane of the first warp");
 #pragma unroll
-  for (int k = 0; k < K; ++k)
-    for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_xor_sync(0xffffffffu, v[k], o);
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  if (lane == 0) {
-#pragma unroll
-    for (int k = 0; k < K; ++k) red[k][warp] = v[k];
-  }
+  for (int k = 0; k < K; ++k) red[k][threadIdx.x] = v[k];
   __syncthreads();
-  if (threadIdx.x == 0) {
+  if (threadIdx.x < 32) {
 #pragma unroll
     for (int k = 0; k < K; ++k) {
-      double s = 0.0;
-      for (int w = 0; w < NT / 32; ++w) s += red[k][w];
-      v[k] = s;
+      const double* r = red[k] + threadIdx.x;
+      v[k] = ((r[0] + r[32]) + (r[64] + r[96])) + ((r[128] + r[160]) + (r[192] + r[224]));
+      for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_xor_sync(0xffffffffu, v[k], o);
     }
   }
   __syncthreads();
@@ -216,7 +218,7 @@ __device__ __forceinline__ void block_reduce(double (&v)[K], double (*red)[NT / 
 // them).
 template <int NT, int K>
 __device__ __forceinline__ void block_partials(double (&v)[K], double* partials) {
-  __shared__ double red[K][NT / 32];
+  __shared__ double red[K][NT];
   block_reduce<NT, K>(v, red);
   if (threadIdx.x == 0) {
 #pragma unroll
@@ -229,7 +231,7 @@ __device__ __forceinline__ void block_partials(double (&v)[K], double* partials)
 template <int NT, int K>
 __device__ __forceinline__ void sum_partials(const double* partials, unsigned int nblocks, double (&out)[K],
                                              unsigned int stride = K) {
-  __shared__ double red[K][NT / 32];
+  __shared__ double red[K][NT];
   double acc[K];
 #pragma unroll
   for (int k = 0; k < K; ++k) acc[k] = 0.0;

@@ -21,19 +21,6 @@ ct_status red_ws(void* ws, size_t bytes, const char* who, RedWs& r) {
   return CT_OK;
 }
 
-// Two simultaneous float64 grid sums; the last block gets both totals.
-template <int NT>
-__device__ __forceinline__ bool grid_sum2_last(double a, double b, double* partials,
-                                               unsigned int* ticket, double& ta, double& tb) {
-  double v[2] = {a, b}, out[2];
-  const bool last = ct::grid_reduce_last<NT, 2>(v, partials, ticket, out);
-  if (last) {
-    ta = out[0];
-    tb = out[1];
-  }
-  return last;
-}
-
 constexpr int NT = ct::kReduceThreads;
 
 // Quad path: with n % 4 == 0 and every array 16-B aligned a thread moves
@@ -65,19 +52,19 @@ __global__ void __launch_bounds__(NT)
         a1 = ld4(a, e0 + stride);
         b1 = ld4(b, e0 + stride);
       }
-#pragma unroll
-      for (int j = 0; j < 4; ++j) acc += (double)at4(a0, j) * (double)at4(b0, j);
+      const float u0[4] = {a0.x, a0.y, a0.z, a0.w}, v0[4] = {b0.x, b0.y, b0.z, b0.w};
+      acc += ct::dot_group(u0, v0);
       if (two) {
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc += (double)at4(a1, j) * (double)at4(b1, j);
+        const float u1[4] = {a1.x, a1.y, a1.z, a1.w}, v1[4] = {b1.x, b1.y, b1.z, b1.w};
+        acc += ct::dot_group(u1, v1);
       }
     }
   } else {
     for (size_t e = (size_t)blockIdx.x * NT + threadIdx.x; e < n; e += (size_t)gridDim.x * NT)
       acc += (double)a[e] * (double)b[e];
   }
-  double t0, t1;
-  if (grid_sum2_last<NT>(acc, 0.0, partials, ticket, t0, t1)) *out = t0;
+  double v[1] = {acc}, t[1];
+  if (ct::grid_reduce_last<NT, 1>(v, partials, ticket, t)) *out = t[0];
 }
 
 __global__ void __launch_bounds__(NT)
@@ -89,14 +76,14 @@ __global__ void __launch_bounds__(NT)
   if (vec) {
     for (size_t e0 = 4 * ((size_t)blockIdx.x * NT + threadIdx.x); e0 < n; e0 += 4 * (size_t)gridDim.x * NT) {
       const float4 b4 = ld4(b, e0), a4 = ld4(Ax, e0);
-      float re[4];
+      float re[4], be[4];
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        const float be = at4(b4, j);
-        re[j] = ct::fsub(be, at4(a4, j));
-        rr += (double)re[j] * (double)re[j];
-        bb += (double)be * (double)be;
+        be[j] = at4(b4, j);
+        re[j] = ct::fsub(be[j], at4(a4, j));
       }
+      rr += ct::dot_group(re, re);
+      bb += ct::dot_group(be, be);
       const float4 r4 = make_float4(re[0], re[1], re[2], re[3]);
       st4(r, e0, r4);
       st4(p, e0, r4);
@@ -111,8 +98,9 @@ __global__ void __launch_bounds__(NT)
       bb += (double)be * (double)be;
     }
   }
-  double trr, tbb;
-  if (grid_sum2_last<NT>(rr, bb, partials, ticket, trr, tbb)) {
+  double v[2] = {rr, bb}, t[2];
+  if (ct::grid_reduce_last<NT, 2>(v, partials, ticket, t)) {
+    const double trr = t[0], tbb = t[1];
     const double bn = sqrt(tbb);
     const double thr = fmax(tol * bn, atol);
     s[CT_CG_NUM] = trr;
@@ -150,8 +138,9 @@ __global__ void __launch_bounds__(NT)
   const double alpha = alpha_s;
   const float af = (float)alpha;
   const double rr = ct::cg_update_pass(x, r, p, Ap, n, af, vec);
-  double trr, t1;
-  if (grid_sum2_last<NT>(rr, 0.0, partials, ticket, trr, t1)) {
+  double v[1] = {rr}, t[1];
+  if (ct::grid_reduce_last<NT, 1>(v, partials, ticket, t)) {
+    const double trr = t[0];
     const double num_old = s[CT_CG_NUM];
     s[CT_CG_ALPHA] = alpha;
     s[CT_CG_NUM] = trr;
