@@ -9,6 +9,7 @@ namespace ct {
 struct Proj2dPlan {
   // forward: 32-row x 256-column strips, views per CTA, bins per tile / strip
   int tiles_i, n_chunks, n_strips, L, LS, cspan, vpc, fwd_groups;
+  int fwd_big, fwd_vps;  // view groups of vpc views, views per CTA of the groups after them
   size_t fwd_bytes, fwd_smem;
   // adjoint: 16x64 tiles, view splits, staged window length
   int adj_gx, adj_gy, nsplit, per_split, W, adj_ni;  // adj_ni: images per CTA

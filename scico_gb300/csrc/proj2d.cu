@@ -49,7 +49,6 @@ constexpr int kT = 32;          // forward tile edge: rows = lanes, columns = re
 constexpr int kCW = 256;        // forward strip width (8 tiles)
 constexpr int kFW = 8;          // warps of a forward CTA (one tile each)
 constexpr int kSms = 152;
-constexpr int kFwdTargetCtas = 12 * kSms;
 constexpr int kLSDefault = 47;  // partial-row stride when projected pixels are at most one bin wide
 constexpr int kGL = 16;         // strips read per round by a forward gather warp
 constexpr int kAI = 64;         // adjoint tile rows
@@ -260,7 +259,8 @@ struct FwdArgs {
   const float* views;
   int rows, cols, nv;
   int L, LS, cspan;
-  int n_chunks, vpc;
+  int n_chunks, n_strips, batch;
+  int vpc, big, vps;    // views per CTA of the first `big` view groups, and of the rest
   int tensor;           // 1 = strip tiles by tensor-map loads (the kernel's map parameter)
   uint32_t max_polls;   // poll limit of the strip-copy wait
   int* errflag;
@@ -304,9 +304,8 @@ struct FwdViewSmem {
 // otherwise compute the same values for its tile).  A span that does not fit
 // the partial rows or the strip's bins (impossible for a table from
 // ct_proj2d_views) sets bit 0 of the error word and skips the tile.
-__device__ __forceinline__ void fwd_view_params(const FwdArgs& a, FwdViewSmem* vs, int i0, int c0, int ch) {
-  const int vbeg = blockIdx.y * a.vpc;
-  const int nvw = min(a.nv, vbeg + a.vpc) - vbeg;
+__device__ __forceinline__ void fwd_view_params(const FwdArgs& a, FwdViewSmem* vs, int i0, int c0, int ch, int vbeg,
+                                                int nvw) {
   const int t = threadIdx.x;
   if (t >= nvw * kFW) return;
   const int vi = t / kFW, w = t - vi * kFW;
@@ -335,7 +334,7 @@ __device__ __forceinline__ void fwd_view_params(const FwdArgs& a, FwdViewSmem* v
   }
 }
 
-// grid = (n_strips, view groups, batch), block = 256.  LSC: the partial-row
+// One CTA per (view group, image, strip), strips fastest, long runs of views first; block = 256.  LSC: the partial-row
 // stride as a compile-time constant (its default-geometry value, so the row
 // sums address with immediates), or 0 for a.LS.
 template <int LSC>
@@ -354,13 +353,13 @@ __global__ void __launch_bounds__(kFW * 32, 3)
   uint64_t* bar = reinterpret_cast<uint64_t*>(vs + 1);
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int s = blockIdx.x;
+  const int u = blockIdx.x / a.n_strips, s = blockIdx.x - u * a.n_strips;
+  const int grp = u / a.batch, b = u - grp * a.batch;
   const int ti = s / a.n_chunks, ch = s - ti * a.n_chunks;
   const int i0 = ti * kT, c0 = ch * kCW;
-  const int b = blockIdx.z;
 
-  const int vbeg = blockIdx.y * a.vpc;
-  const int vend = min(a.nv, vbeg + a.vpc);
+  const int vbeg = grp < a.big ? grp * a.vpc : a.big * a.vpc + (grp - a.big) * a.vps;
+  const int vend = min(a.nv, vbeg + (grp < a.big ? a.vpc : a.vps));
 
   // ---- stage the strip's tiles (zero outside the image) ---------------------
   // Tiles that start right of the image are not loaded: their warps have
@@ -377,7 +376,7 @@ __global__ void __launch_bounds__(kFW * 32, 3)
       ct::mbar_arrive_expect_tx(bar, (uint32_t)(ntl * kT * kT * 4));
       for (int w = 0; w < ntl; ++w) ct::tensor_g2s_3d(tiles + w * kT * kT, &tmap, c0 + w * kT, i0, b, bar);
     }
-    fwd_view_params(a, vs, i0, c0, ch);
+    fwd_view_params(a, vs, i0, c0, ch, vbeg, vend - vbeg);
     if (!ct::mbar_wait_bounded(bar, 0, a.max_polls)) {
       timed_out = 1;
       if (tid == 0) atomicOr(a.errflag, 2);
@@ -394,13 +393,13 @@ __global__ void __launch_bounds__(kFW * 32, 3)
       const int gi = i0 + r, gj = c0 + w * kT + c;
       tiles[w * kT * kT + swz(r, c)] = (gi < a.rows && gj < a.cols) ? __ldg(im + (size_t)gi * a.cols + gj) : 0.0f;
     }
-    fwd_view_params(a, vs, i0, c0, ch);
+    fwd_view_params(a, vs, i0, c0, ch, vbeg, vend - vbeg);
   }
   if (__syncthreads_or(timed_out)) {
     // The strip is not known to be complete: skip the work and leave zeros
     // in this CTA's strip bins, so the gather reads defined values.
     for (int vi = warp; vi < vend - vbeg; vi += kFW) {
-      float* po = a.part + (((size_t)b * gridDim.x + s) * a.nv + vbeg + vi) * a.cspan;
+      float* po = a.part + (((size_t)b * a.n_strips + s) * a.nv + vbeg + vi) * a.cspan;
       const int n = min(vs->strip[vi].y, a.cspan);
       for (int k = lane; k < n; k += 32) po[k] = 0.0f;
     }
@@ -507,7 +506,7 @@ __global__ void __launch_bounds__(kFW * 32, 3)
   float* acc = part + warp * kT * LS;
   for (int vi = warp; vi < vend - vbeg; vi += kFW) {
     const float* tb = tbins + (size_t)vi * kFW * a.L;
-    float* po = a.part + (((size_t)b * gridDim.x + s) * a.nv + vbeg + vi) * a.cspan;
+    float* po = a.part + (((size_t)b * a.n_strips + s) * a.nv + vbeg + vi) * a.cspan;
     const int n = min(vs->strip[vi].y, a.cspan);
     for (int k = lane; k < n; k += 32) acc[k] = 0.0f;
     __syncwarp();
@@ -920,15 +919,29 @@ Proj2dPlan proj2d_plan_sched(const ct_geom2d* g, int batch, Sched2d sc) {
   p.LS = p.L;
   while ((p.LS & 31) != 15 && (p.LS & 31) != 17) ++p.LS;
   p.cspan = (int)floorf((float)(kCW - 1) * mw + 1.01f) + 3;
-  const long work = (long)p.n_strips * g->n_views * batch;
-  // Views per CTA: about kFwdTargetCtas CTAs, each with its staging to pay; a
-  // problem of at most eight rounds of single views instead takes one round of
-  // the SMs' three CTAs (200^2 x 500 views: 27.5 us at 2, 22.0 us at 8; 256^2 x
-  // 180: 14.9 us at 2, 13.9 us at 4; 384^2 x 270 stays: 37.0 us at 4, 39.5 us at 16).
+  // Views per CTA.  A problem of at most eight rounds of single views over the
+  // SMs' three CTAs takes one round (200^2 x 500 views: 27.5 us at 2 views, 22.0 us
+  // at 8; 256^2 x 180: 14.9 us at 2, 13.9 us at 4).  A larger one takes long runs of
+  // even length, which stage a strip seldom, and then about one round of CTAs with
+  // runs a third as long, so that the SMs end together.  Against one length and
+  // about 1824 CTAs: 512^2 x 360 60.4 -> 58.7 us, 501^2 68.5 -> 64.0 us, 640^2 x 270
+  // 78.3 -> 72.8 us, 450^2 x 300 58.8 -> 52.7 us, 16 x 256^2 x 180 112.1 -> 109.5 us.
+  // Runs of 12 under 20 rounds: 384^2 x 270 33.8 us (16: 34.0), 512^2 x 129 27.0 us
+  // (28.9).  Images of at most two tile columns keep even runs: their CTAs, two busy
+  // warps of eight, are mostly staging (300 x 64^2 x 45: 82.2 us, tapered 87.4 us).
   const long round = 3L * kSms;
-  const long vpc = work <= 8 * round ? (work + round - 1) / round : (work + kFwdTargetCtas - 1) / kFwdTargetCtas;
-  p.vpc = sc.vpc > 0 ? std::min(sc.vpc, kMaxVpc) : (int)std::min<long>(kMaxVpc, std::max<long>(2, vpc));
-  p.fwd_groups = (g->n_views + p.vpc - 1) / p.vpc;
+  const long per_view = (long)p.n_strips * batch, work = per_view * g->n_views;
+  const bool large = work > 8 * round;
+  const long vpc = large ? (work >= 20 * round ? 16 : 12) : std::max<long>(2, (work + round - 1) / round);
+  p.vpc = sc.vpc > 0 ? std::min(sc.vpc, kMaxVpc) : (int)std::min<long>(kMaxVpc, vpc);
+  const bool taper = large && g->cols > 2 * kT;
+  p.fwd_vps = taper ? std::max(1, p.vpc / 3) : p.vpc;
+  const long small = taper ? (round + per_view - 1) / per_view : 0;  // groups of short runs
+  const long rest = std::max(0L, g->n_views - small * p.fwd_vps);  // views in long runs, of even length
+  const long n_big = (rest + p.vpc - 1) / p.vpc;
+  if (sc.vpc <= 0 && n_big > 0) p.vpc = (int)std::max<long>(p.fwd_vps, (rest + n_big - 1) / n_big);
+  p.fwd_big = (int)std::min<long>(n_big, g->n_views / p.vpc);
+  p.fwd_groups = p.fwd_big + (g->n_views - p.fwd_big * p.vpc + p.fwd_vps - 1) / p.fwd_vps;
   p.fwd_bytes = round_up((size_t)batch * p.n_strips * g->n_views * p.cspan * sizeof(float), 256);
   p.fwd_smem = fwd_smem_bytes(p.LS, p.L);
   p.W = (int)floorf((float)(std::max(kAI, kAJ) - 1) * mw + 1.01f) + 3;
@@ -1065,7 +1078,11 @@ ct_status proj2d_fwd_launch(const ct_geom2d* g, const Proj2dPlan& p, const float
   a.LS = p.LS;
   a.cspan = p.cspan;
   a.n_chunks = p.n_chunks;
+  a.n_strips = p.n_strips;
+  a.batch = batch;
   a.vpc = p.vpc;
+  a.big = p.fwd_big;
+  a.vps = p.fwd_vps;
   CUtensorMap tmap;
   memset(&tmap, 0, sizeof(tmap));
   a.tensor = encode_image_map(&tmap, img, g->rows, g->cols, batch) ? 1 : 0;
@@ -1073,7 +1090,7 @@ ct_status proj2d_fwd_launch(const ct_geom2d* g, const Proj2dPlan& p, const float
   a.errflag = errflag_ptr();
   a.skip = skip;
   if (!a.errflag) return fail(CT_ERR_CUDA, "proj2d: error-word address unavailable");
-  dim3 g1(p.n_strips, p.fwd_groups, batch);
+  dim3 g1((unsigned)p.n_strips * p.fwd_groups * batch);
   auto strips = p.LS == kLSDefault ? k_proj2d_fwd_strips<kLSDefault> : k_proj2d_fwd_strips<0>;
   ct_status st = cuda_check(launch_k(strips, g1, dim3(kFW * 32), p.fwd_smem, s, dependent, a, tmap),
                             "k_proj2d_fwd_strips");

@@ -56,3 +56,19 @@ def test_reduced_scratch(cuda):
         assert st == (_lib.CT_OK if ok else _lib.CT_ERR_WORKSPACE)
         if ok:
             assert _rel(out, want) <= 2e-6
+
+
+@pytest.mark.parametrize("shape,nv,batch", [((70, 100), 60, 100), ((300, 200), 91, 8), ((33, 66), 7, 900), ((40, 70), 1, 2000),
+                                            ((64, 64), 45, 90), ((500, 257), 200, 1), ((90, 80), 23, 120)], ids=str)
+def test_forward_runs_of_views(cuda, shape, nv, batch):
+    """Long and short runs of views a CTA (large problems) against one round of even runs: no sum depends on the
+    runs, so each image's projections are the same bits as alone, and each view's as in a scan of a few views."""
+    ang = np.linspace(0, np.pi, nv, endpoint=False)
+    A = linop.XRayTransform2D(shape, ang)
+    x = torch.rand((batch,) + shape, generator=torch.Generator().manual_seed(nv)).to(cuda)
+    got = A.project(x if batch > 1 else x[0]).reshape((batch,) + A.output_shape)
+    for k in {0, batch // 2, batch - 1} if batch > 1 else ():
+        assert torch.equal(got[k], A.project(x[k].contiguous()))
+    few = sorted({0, nv // 2, nv - 2, nv - 1} - {-1})
+    B = linop.XRayTransform2D(shape, ang[few])
+    assert torch.equal(got[-1][few], B.project(x[-1].contiguous()))
