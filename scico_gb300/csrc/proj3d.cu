@@ -883,13 +883,40 @@ __global__ void __launch_bounds__(256) k_p3_gen_march(const float* __restrict__ 
   }
 }
 
-__global__ void k_p3_sum_splits(const float* __restrict__ part, float* __restrict__ out, size_t n,
-                                int nsplit, size_t stride) {
-  for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < n;
-       e += (size_t)gridDim.x * blockDim.x) {
-    float s = 0.0f;
-    for (int k = 0; k < nsplit; ++k) s += part[(size_t)k * stride + e];
-    out[e] = s;
+// out[e] = sum over the view splits, in split order.  A stream of nsplit + 1
+// volumes: W = 4 elements an access where the volume's size and both arrays allow
+// it, four splits loaded before they are added (2 splits of 256^3: 71.6 us with
+// single elements, 26.1 us; the back projection 1541 -> 1501 us).
+template <int W>
+__global__ void __launch_bounds__(256) k_p3_sum_splits(const float* __restrict__ part, float* __restrict__ out,
+                                                       size_t n, int nsplit) {
+  constexpr int kAhead = 4;
+  for (size_t e = W * ((size_t)blockIdx.x * 256 + threadIdx.x); e < n; e += W * (size_t)gridDim.x * 256) {
+    float acc[W] = {};
+    for (int k = 0; k < nsplit; k += kAhead) {
+      float v[kAhead][W];
+#pragma unroll
+      for (int u = 0; u < kAhead; ++u) {
+        if (k + u >= nsplit) break;
+        const float* q = part + (size_t)(k + u) * n + e;
+        if constexpr (W == 4) {
+          const float4 f = __ldcs(reinterpret_cast<const float4*>(q));
+          v[u][0] = f.x, v[u][1] = f.y, v[u][2] = f.z, v[u][3] = f.w;
+        } else {
+          v[u][0] = __ldcs(q);
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < kAhead; ++u) {
+        if (k + u >= nsplit) break;
+#pragma unroll
+        for (int j = 0; j < W; ++j) acc[j] += v[u][j];
+      }
+    }
+    if constexpr (W == 4)
+      *reinterpret_cast<float4*>(out + e) = make_float4(acc[0], acc[1], acc[2], acc[3]);
+    else
+      out[e] = acc[0];
   }
 }
 
@@ -1077,6 +1104,14 @@ Proj3dPlan proj3d_plan_sched(const ct_geom3d* g, Sched3d sc) {
   p.adj_ws_bytes = ns_ws > 1 ? round_up(sizeof(float) * (size_t)ns_ws * S * NJ * NK, 256) : 0;
   p.adj_ws_bytes = std::max(p.adj_ws_bytes, std::max(p.adj_bytes, std::max(p.adj_least, p.adj_tune)));
   return p;
+}
+
+ct_status sum_splits(const float* part, float* out, size_t n, int nsplit, cudaStream_t s) {
+  const int vec = quad_ok(n, part, out);
+  const size_t per = vec ? 1024 : 256;
+  const int blocks = (int)std::min<size_t>((n + per - 1) / per, 16 * 1024);
+  (vec ? k_p3_sum_splits<4> : k_p3_sum_splits<1>)<<<blocks, 256, 0, s>>>(part, out, n, nsplit);
+  return launch_check("k_p3_sum_splits");
 }
 
 // Schedules recorded by ct_proj3d_autotune, keyed by the geometry's sizes
@@ -1420,9 +1455,7 @@ ct_status ct_proj3d_adj(const ct_geom3d* g, const float* proj, float* vol, int32
     st = proj3d_adj_launch(g, p, proj + b * proj_n, vol + b * vol_n, part, s, nullptr);
     if (st != CT_OK) return st;
     if (p.nsplit > 1) {
-      const int blocks = (int)std::min<size_t>((vol_n + 255) / 256, 4096);
-      k_p3_sum_splits<<<blocks, 256, 0, s>>>(part, vol + b * vol_n, vol_n, p.nsplit, vol_n);
-      st = launch_check("k_p3_sum_splits");
+      st = sum_splits(part, vol + b * vol_n, vol_n, p.nsplit, s);
       if (st != CT_OK) return st;
     }
   }
@@ -1508,9 +1541,7 @@ ct_status ct_proj3d_autotune(const ct_geom3d* g, float* vol, float* proj, void* 
           [&] {
             ct_status r = proj3d_adj_launch(g, p, proj, vol, part, s, nullptr);
             if (r != CT_OK || p.nsplit == 1) return r;
-            const int blocks = (int)std::min<size_t>((vol_n + 255) / 256, 4096);
-            k_p3_sum_splits<<<blocks, 256, 0, s>>>(part, vol, vol_n, p.nsplit, vol_n);
-            return launch_check("k_p3_sum_splits");
+            return sum_splits(part, vol, vol_n, p.nsplit, s);
           },
           us);
       if (st != CT_OK) return st;

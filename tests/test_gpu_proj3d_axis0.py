@@ -25,6 +25,7 @@ CASES = [
     dict(shape=(131, 34, 18), det=(131, 40), nv=66),
     dict(shape=(40, 20, 22), det=(44, 31), nv=7),  # rows off the slices (offset 2)
     dict(shape=(260, 16, 17), det=(260, 25), nv=40),
+    dict(shape=(33, 21, 19), det=(33, 29), nv=80),  # view splits of a volume that is no whole number of quads
 ]
 
 
