@@ -785,26 +785,62 @@ __global__ void __launch_bounds__(kAdjThreads, 3) k_proj2d_adj_two(const AdjArgs
 // out[e] = sum_s part[s*stride + e] in split order; with a mask (of n_img
 // pixels, one per image of the batch), times `scale` where it is set and 0
 // where it is not (out may be part when there is one split).  Latency-bound:
-// kSumU splits are loaded before they are added.
+// kSumU splits are loaded before they are added, W elements an access (4 from
+// the size on where that still leaves a thread for every slot of the SMs:
+// back projection of 4 x 300^2 x 200 views 27.5 -> 26.8 us, 768^2 x 180 45.7 ->
+// 44.9 us, 1024^2 x 360 136.3 -> 134.1 us; below it single elements, 384^2 x 270
+// 20.0 against 20.6 us, 256^2 x 180 11.2 against 11.5 us).
 constexpr int kSumU = 8;
-template <bool MASK>
+template <bool MASK, int W>
 __global__ void __launch_bounds__(256) k_sum_splits(const float* part, float* out, size_t n, int nsplit, size_t stride,
                                                     const uint8_t* __restrict__ mask, size_t n_img, float scale) {
-  for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < n;
-       e += (size_t)gridDim.x * blockDim.x) {
-    float s = 0.0f;
+  for (size_t e = W * ((size_t)blockIdx.x * blockDim.x + threadIdx.x); e < n; e += W * (size_t)gridDim.x * blockDim.x) {
+    float s[W] = {};
     int k = 0;
+    auto load = [&](int at, float (&v)[W]) {
+      const float* q = part + (size_t)at * stride + e;
+      if constexpr (W == 4) {
+        const float4 f = *reinterpret_cast<const float4*>(q);
+        v[0] = f.x, v[1] = f.y, v[2] = f.z, v[3] = f.w;
+      } else {
+        v[0] = *q;
+      }
+    };
     for (; k + kSumU <= nsplit; k += kSumU) {
-      float v[kSumU];
+      float v[kSumU][W];
 #pragma unroll
-      for (int u = 0; u < kSumU; ++u) v[u] = part[(size_t)(k + u) * stride + e];
+      for (int u = 0; u < kSumU; ++u) load(k + u, v[u]);
 #pragma unroll
-      for (int u = 0; u < kSumU; ++u) s += v[u];
+      for (int u = 0; u < kSumU; ++u)
+#pragma unroll
+        for (int j = 0; j < W; ++j) s[j] += v[u][j];
     }
-    for (; k < nsplit; ++k) s += part[(size_t)k * stride + e];
-    if (MASK) s = ct::fmul(mask[n_img == n ? e : e % n_img] ? scale : 0.0f, s);
-    out[e] = s;
+    for (; k < nsplit; ++k) {
+      float v[W];
+      load(k, v);
+#pragma unroll
+      for (int j = 0; j < W; ++j) s[j] += v[j];
+    }
+    if constexpr (MASK) {
+#pragma unroll
+      for (int j = 0; j < W; ++j) s[j] = ct::fmul(mask[n_img == n ? e + j : (e + j) % n_img] ? scale : 0.0f, s[j]);
+    }
+    if constexpr (W == 4)
+      *reinterpret_cast<float4*>(out + e) = make_float4(s[0], s[1], s[2], s[3]);
+    else
+      out[e] = s[0];
   }
+}
+
+template <bool MASK>
+ct_status sum_splits(const float* part, float* out, size_t n, int nsplit, const uint8_t* mask, size_t n_img, float scale,
+                     cudaStream_t s) {
+  const bool quads = n >= 2048 * (size_t)kSms && ct::quad_ok(n, part, out);
+  const size_t per = quads ? 1024 : 256;
+  const int blocks = (int)std::min<size_t>((n + per - 1) / per, 4096);
+  (quads ? k_sum_splits<MASK, 4> : k_sum_splits<MASK, 1>)<<<blocks, 256, 0, s>>>(part, out, n, nsplit, n, mask, n_img,
+                                                                                scale);
+  return ct::launch_check("k_sum_splits");
 }
 
 // Device error word of the library's device checks (bit 0: forward tile
@@ -1033,9 +1069,7 @@ bool sched_lookup(const ct_geom2d* g, int batch, SchedVal& out) {
 uint32_t proj2d_wait_polls() { return g_wait_polls.load(std::memory_order_relaxed); }
 
 ct_status proj2d_sum_splits(const float* part, float* out, size_t n, int nsplit, cudaStream_t s) {
-  const int blocks = (int)std::min<size_t>((n + 255) / 256, 4096);
-  k_sum_splits<false><<<blocks, 256, 0, s>>>(part, out, n, nsplit, n, nullptr, n, 1.0f);
-  return launch_check("k_sum_splits");
+  return sum_splits<false>(part, out, n, nsplit, nullptr, n, 1.0f, s);
 }
 
 Proj2dPlan proj2d_plan(const ct_geom2d* g, int batch) {
@@ -1183,9 +1217,7 @@ static ct_status adj_call(const char* who, const ct_geom2d* g, const float* sino
   if (st != CT_OK || (p.nsplit == 1 && !mask)) return st;
   const size_t n_img = (size_t)g->rows * g->cols, n = (size_t)batch * n_img;
   if (!mask) return ct::proj2d_sum_splits(part, img, n, p.nsplit, s);
-  const int blocks = (int)std::min<size_t>((n + 255) / 256, 4096);
-  k_sum_splits<true><<<blocks, 256, 0, s>>>(p.nsplit == 1 ? img : part, img, n, p.nsplit, n, mask, n_img, scale);
-  return ct::launch_check("k_sum_splits");
+  return sum_splits<true>(p.nsplit == 1 ? img : part, img, n, p.nsplit, mask, n_img, scale, s);
 }
 
 ct_status ct_proj2d_adj(const ct_geom2d* g, const float* sino, float* img, int32_t batch,

@@ -23,6 +23,8 @@ def _rel(a, b):
 
 @pytest.mark.parametrize("shape,nv,batch,kw", [
     ((64, 64), 33, 2, {}), ((65, 63), 40, 3, {}), ((130, 200), 96, 5, {}), ((128, 96), 180, 16, {}),
+    ((301, 300), 64, 4, {}), ((303, 303), 40, 4, {}),  # the split sum in quads, and too odd for them
+   
     ((40, 30), 64, 7, dict(det_count=20)), ((50, 50), 48, 4, dict(y0=-3.0e6, det_count=71)),
     ((64, 70), 17, 2, dict(dx=0.4))], ids=str)
 def test_batch_matches_single(cuda, shape, nv, batch, kw):
