@@ -451,7 +451,7 @@ struct Plan {
 
 // Tape: P[K], AP[K], R[K+1] (none with recompute), then the scalars.
 // Workspace: reduction area, projector scratch, sinogram, t and the
-// backward's rb, pb, apb; with recompute also P, AP, R and x.
+// backward's rb, pb, apb, xb (where a gradient is written over gx); with recompute also P, AP, R and x.
 Plan plan_of(const ct_cg_block_desc* d) {
   Plan P;
   const size_t n = (size_t)d->geom.rows * d->geom.cols;
@@ -470,7 +470,7 @@ Plan plan_of(const ct_cg_block_desc* d) {
              ct::round_up((size_t)d->nsys * 4 * P.s.nb * sizeof(double), 256);
   P.ws_proj = ct::round_up(std::max<size_t>(std::max(P.p2.fwd_bytes, P.p2.adj_ws_bytes), 256), 256);
   P.ws_sino = ct::round_up((size_t)d->nsys * d->geom.n_views * d->geom.det_count * sizeof(float), 256);
-  P.ws_tmp = 4 * P.vec;
+  P.ws_tmp = 5 * P.vec;
   P.ws_recompute = d->recompute ? vectors + P.vec : 0;
   P.ws_total = P.ws_red + P.ws_proj + P.ws_sino + P.ws_tmp + P.ws_recompute;
   return P;
@@ -490,7 +490,7 @@ struct Bufs {
   double* partials;
   float* proj_ws;
   float* sino;
-  float *t, *rb, *pb, *apb;
+  float *t, *rb, *pb, *apb, *xb;
   float *P, *AP, *R, *x;  // iterates: the tape's, or the workspace's with recompute
   double* scal;
 };
@@ -509,6 +509,7 @@ Bufs bufs(const ct_cg_block_desc* d, const Plan& P, void* tape, void* ws, float*
   B.rb = reinterpret_cast<float*>(q + P.vec);
   B.pb = reinterpret_cast<float*>(q + 2 * P.vec);
   B.apb = reinterpret_cast<float*>(q + 3 * P.vec);
+  B.xb = reinterpret_cast<float*>(q + 4 * P.vec);
   q += P.ws_tmp;
   char* vec = d->recompute ? q : static_cast<char*>(tape);
   const int K = d->maxiter;
@@ -622,6 +623,15 @@ ct_status ct_cg_block_bwd(const ct_cg_block_desc* d, const float* gx, const floa
   const Bufs B = bufs(d, P, tape, workspace, nullptr);
   if (d->recompute) CT_TRY(forward(d, P, B, b, lam, x0, s));  // the iterates from the block's inputs
   const float gs = d->gram_scale;
+  const size_t nbytes = (size_t)d->nsys * P.s.n * sizeof(float);
+  auto over = [&](const float* p) {
+    const char *u = reinterpret_cast<const char*>(gx), *w = reinterpret_cast<const char*>(p);
+    return p && u < w + nbytes && w < u + nbytes;
+  };
+  if (over(gb) || over(gx0)) {  // gx is read to the end
+    CT_TRY(ct::cuda_check(cudaMemcpyAsync(B.xb, gx, nbytes, cudaMemcpyDeviceToDevice, s), "gx copy"));
+    gx = B.xb;
+  }
   const int vec = ct::quad_ok(P.s.n, gx, x0, gb, gx0);
   k_cgb_reset<<<1, 256, 0, s>>>(B.scal, P.s);
   CT_TRY(ct::launch_check("k_cgb_reset"));

@@ -71,3 +71,35 @@ def test_cg_block_scale(cuda, power):
     assert _rel(gbs, gb) < 1e-6
     assert _rel(gls / c, gl) < 1e-6
     assert float((gx0s - gx0).norm() / w.norm()) < 1e-6
+
+
+def test_cg_block_gradient_over_its_input(cuda):
+    """ct_cg_block_bwd with a gradient written over gx: the bits of separate arrays."""
+    import ctypes
+
+    from scico_gb300 import _device, _lib
+
+    A = linop.XRayTransform2D((40, 36), np.linspace(0, np.pi, 20, endpoint=False))
+    gen = torch.Generator().manual_seed(8)
+    b, x0, w = (torch.randn((2, 40, 36), generator=gen).to(cuda) for _ in range(3))
+    d = _lib.CgBlockDesc(A.geometry(), 2, 3, 0, 1.0 / 1600.0)
+    tb, wb = _lib.c_size_t(), _lib.c_size_t()
+    at = ctypes.addressof
+    _lib.call("ct_cg_block_workspace", at(d), at(tb), at(wb))
+    tape, ws = _device.workspace(tb.value), _device.workspace(wb.value)
+    x = torch.empty_like(b)
+    st = _device.stream()
+    _lib.call("ct_cg_block_fwd", at(d), b.data_ptr(), 20.0, x0.data_ptr(), x.data_ptr(), tape.data_ptr(),
+              tape.numel(), ws.data_ptr(), ws.numel(), st)
+
+    def grads(gx, gb, gx0):
+        gl = torch.zeros(1, dtype=torch.float64, device=cuda)
+        _lib.call("ct_cg_block_bwd", at(d), gx.data_ptr(), b.data_ptr(), 20.0, x0.data_ptr(), tape.data_ptr(),
+                  tape.numel(), gb.data_ptr(), gx0.data_ptr(), gl.data_ptr(), ws.data_ptr(), ws.numel(), st)
+        return gb, gx0, gl
+
+    want = grads(w, torch.empty_like(w), torch.empty_like(w))
+    for over in (0, 1):
+        g = w.clone()
+        got = grads(g, g if over == 0 else torch.empty_like(w), g if over == 1 else torch.empty_like(w))
+        assert all(torch.equal(a, c) for a, c in zip(got, want))
