@@ -216,18 +216,18 @@ __device__ __forceinline__ void block_reduce(double (&v)[K], double (*red)[NT]) 
 // grid's partials, summed with all threads of one block in a fixed pattern;
 // valid in thread 0.  The partials are read through L2 (other blocks wrote
 // them).
+// stride: doubles per block in `partials` (K when the block's partials are
+// exactly these K sums; larger when they are K of a wider set).
 template <int NT, int K>
-__device__ __forceinline__ void block_partials(double (&v)[K], double* partials) {
+__device__ __forceinline__ void block_partials(double (&v)[K], double* partials, unsigned int stride = K) {
   __shared__ double red[K][NT];
   block_reduce<NT, K>(v, red);
   if (threadIdx.x == 0) {
 #pragma unroll
-    for (int k = 0; k < K; ++k) partials[(size_t)K * blockIdx.x + k] = v[k];
+    for (int k = 0; k < K; ++k) partials[(size_t)stride * blockIdx.x + k] = v[k];
   }
 }
 
-// stride: doubles per block in `partials` (K when the block's partials are
-// exactly these K sums; larger when they are K of a wider set).
 template <int NT, int K>
 __device__ __forceinline__ void sum_partials(const double* partials, unsigned int nblocks, double (&out)[K],
                                              unsigned int stride = K) {
