@@ -70,17 +70,20 @@ ct_status make_fd(const ct_fd_desc* d, FdParams& p, const char* who) {
 // memory; what cost the time before was index arithmetic (two 64-bit divisions
 // an element) and one element in flight per thread.
 //
-// Rows of at least a warp (k_fd_rows): a warp takes up to kFdU elements a
-// lane of one row (the last axis), so the position along the other axes, and
-// with it the offset to the neighbour and the test for the line's end, is the
-// same for the whole warp and costs nothing per element.  32-bit accesses of
-// whole warps: rows of odd length are as common as multiples of four, and they
-// fill the sectors either way.  Shorter rows (k_fd_*_flat) would leave lanes
-// idle: there a thread takes kFdU elements of the flat array kFdT apart and
-// finds their coordinates with two 32-bit multiply-high divisions.
+// Rows of a whole number of quads in aligned arrays (k_fd_*_quads): a thread
+// takes four elements of a row, whose coordinates cost two 32-bit multiply-high
+// divisions a quad, and its six loads are all in flight.  Other rows of at
+// least a warp (k_fd_rows): a warp takes up to kFdU elements a lane of one
+// row (the last axis), so the position along the other axes, and with it the
+// offset to the neighbour and the test for the line's end, is the same for
+// the whole warp and costs nothing per element.  Shorter ones (k_fd_*_flat) would
+// leave lanes idle: there a thread takes kFdU elements of the flat array
+// kFdT apart.  A copied end's second term is behind a branch that few threads
+// take: as a select it cost the adjoint more than its loads (192^3 in quads 22.3 us).
 // 192^3, three axes (forward / adjoint): 177 / 150 us with the divisions of
-// k_fd_fwd / k_fd_adj, 43 / 62 us flat, 19 / 29 us by rows; 26 us is a
-// copy of the three output arrays.
+// k_fd_fwd / k_fd_adj, 43 / 62 us flat, 18.8 / 27.7 us by rows, 17.4 / 19.9 us
+// in quads (113 MB each: 17 us of measured bandwidth); 300 x 200 x 100 17.7 /
+// 21.5 by rows, 12.7 / 13.7 in quads; 100 x 100 x 20 3.7 / 4.2 flat, 2.0 / 2.1.
 // ---------------------------------------------------------------------------
 constexpr int kFdT = 256;  // threads of a block
 constexpr int kFdU = 4;    // elements per thread
@@ -342,22 +345,21 @@ __device__ __forceinline__ void fd_adj_row(const float* __restrict__ d, float* _
   float acc[U];
 #pragma unroll
   for (int k = 0; k < NB; ++k) {
-    const int a = q.axis[k];
-    const int ca = (int)(a == 1 ? r.c1 : r.c0), na = a == 2 ? n2 : (a == 1 ? q.n[1] : q.n[0]);
-    const bool row_cp = a != 2 && (fwd ? ca == 0 : ca == na - 1);
+    float v[U];
 #pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const bool cp = !wrap && !q.zero && (a == 2 ? (fwd ? c + 32 * u == 0 : c + 32 * u == n2 - 1) : row_cp);
-      float v;
-      if (fwd) {
-        v = ct::fsub(dc[k][u], dn[k][u]);
-        if (cp) v = ct::fadd(ct::fsub(0.0f, dc[k][u]), v);  // position 0 first
-      } else {
-        v = ct::fsub(dn[k][u], dc[k][u]);
-        if (cp) v = ct::fadd(v, dc[k][u]);  // then the position past the end: d[n-1] - 0
+    for (int u = 0; u < U; ++u) v[u] = fwd ? ct::fsub(dc[k][u], dn[k][u]) : ct::fsub(dn[k][u], dc[k][u]);
+    if (!wrap && !q.zero) {  // a copied end: position 0 first, or then the position past the end (d[n-1] - 0)
+      const int a = q.axis[k];
+      const int ca = (int)(a == 1 ? r.c1 : r.c0), na = a == 1 ? q.n[1] : q.n[0];
+      if (a == 2 || (fwd ? ca == 0 : ca == na - 1)) {
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+          if (a != 2 || (fwd ? c + 32 * u == 0 : c + 32 * u == n2 - 1))
+            v[u] = fwd ? ct::fadd(ct::fsub(0.0f, dc[k][u]), v[u]) : ct::fadd(v[u], dc[k][u]);
       }
-      acc[u] = k == 0 ? v : ct::fadd(acc[u], v);
     }
+#pragma unroll
+    for (int u = 0; u < U; ++u) acc[u] = k == 0 ? v[u] : ct::fadd(acc[u], v[u]);
   }
 #pragma unroll
   for (int u = 0; u < U; ++u)
@@ -382,6 +384,107 @@ __global__ void __launch_bounds__(kFdT) k_fd_rows(const float* __restrict__ src,
   }
 }
 
+// Quads (rows of a whole number of them, 16-byte aligned arrays): a thread takes four consecutive elements, its
+// neighbours along the last axis from the quad itself and one more element.
+template <int NB, int MODE>
+__global__ void __launch_bounds__(kFdT) k_fd_fwd_quads(const float* __restrict__ x, float* __restrict__ out, const FdSame q) {
+  constexpr bool back = MODE == 2, wrap = MODE == 0;
+  const uint32_t e = 4 * (blockIdx.x * (uint32_t)kFdT + threadIdx.x);
+  if (e >= q.count) return;
+  int c[3];
+  fd_coords(q, e, c);
+  const float* __restrict__ xp = x + (size_t)blockIdx.y * q.count + e;
+  const float4 x4 = __ldg(reinterpret_cast<const float4*>(xp));
+  const float xc[4] = {x4.x, x4.y, x4.z, x4.w};
+  float xn[NB][4];
+#pragma unroll
+  for (int k = 0; k < NB; ++k) {
+    const int a = q.axis[k];
+    if (a == 2) {
+      const bool end = back ? c[2] == 0 : c[2] + 4 == q.n[2];
+      const int at = back ? (end ? (wrap ? q.n[2] - 1 : 0) : -1) : (end ? (wrap ? 4 - q.n[2] : 3) : 4);
+      float far = __ldg(xp + at);
+      if (!wrap && end && q.zero) far = 0.0f;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) xn[k][j] = back ? (j > 0 ? xc[j > 0 ? j - 1 : 0] : far) : (j < 3 ? xc[j < 3 ? j + 1 : 3] : far);
+    } else {
+      const int ca = a == 1 ? c[1] : c[0], na = a == 1 ? q.n[1] : q.n[0];
+      const bool end = back ? ca == 0 : ca == na - 1;
+      const ptrdiff_t sd = (ptrdiff_t)q.stride[k];
+      const float4 f = __ldg(reinterpret_cast<const float4*>(xp + (end ? (wrap ? -(ptrdiff_t)ca * sd : 0) : (back ? -sd : sd))));
+      xn[k][0] = f.x, xn[k][1] = f.y, xn[k][2] = f.z, xn[k][3] = f.w;
+      if (!wrap && end && q.zero) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) xn[k][j] = 0.0f;
+      }
+    }
+  }
+  float* __restrict__ op = out + (size_t)blockIdx.y * NB * q.count + e;
+#pragma unroll
+  for (int k = 0; k < NB; ++k) {
+    float v[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) v[j] = back ? ct::fsub(xc[j], xn[k][j]) : ct::fsub(xn[k][j], xc[j]);
+    *reinterpret_cast<float4*>(op + (size_t)k * q.count) = make_float4(v[0], v[1], v[2], v[3]);
+  }
+}
+
+template <int NB, int MODE>
+__global__ void __launch_bounds__(kFdT) k_fd_adj_quads(const float* __restrict__ d, float* __restrict__ x, const FdSame q) {
+  constexpr bool fwd = MODE == 2, wrap = MODE == 0;
+  const uint32_t e = 4 * (blockIdx.x * (uint32_t)kFdT + threadIdx.x);
+  if (e >= q.count) return;
+  int c[3];
+  fd_coords(q, e, c);
+  const float* __restrict__ dp = d + (size_t)blockIdx.y * NB * q.count + e;
+  float dc[NB][4], dn[NB][4];
+#pragma unroll
+  for (int k = 0; k < NB; ++k) {
+    const float* __restrict__ dk = dp + (size_t)k * q.count;
+    const int a = q.axis[k];
+    const float4 f = __ldg(reinterpret_cast<const float4*>(dk));
+    dc[k][0] = f.x, dc[k][1] = f.y, dc[k][2] = f.z, dc[k][3] = f.w;
+    if (a == 2) {
+      const bool off = fwd ? c[2] + 4 == q.n[2] : c[2] == 0;
+      float far = __ldg(dk + (off ? (wrap ? q.n[2] - 1 : 0) : (fwd ? 4 : -1)));
+      if (!wrap && off) far = 0.0f;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) dn[k][j] = fwd ? (j < 3 ? dc[k][j < 3 ? j + 1 : 3] : far) : (j > 0 ? dc[k][j > 0 ? j - 1 : 0] : far);
+    } else {
+      const int ca = a == 1 ? c[1] : c[0], na = a == 1 ? q.n[1] : q.n[0];
+      const bool off = fwd ? ca == na - 1 : ca == 0;
+      const ptrdiff_t sd = (ptrdiff_t)q.stride[k];
+      const float4 g = __ldg(reinterpret_cast<const float4*>(dk + (off ? (wrap ? (ptrdiff_t)(na - 1) * sd : 0) : (fwd ? sd : -sd))));
+      dn[k][0] = g.x, dn[k][1] = g.y, dn[k][2] = g.z, dn[k][3] = g.w;
+      if (!wrap && off) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) dn[k][j] = 0.0f;
+      }
+    }
+  }
+  float acc[4];
+#pragma unroll
+  for (int k = 0; k < NB; ++k) {
+    float v[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) v[j] = fwd ? ct::fsub(dc[k][j], dn[k][j]) : ct::fsub(dn[k][j], dc[k][j]);
+    if (!wrap && !q.zero) {  // a copied end: position 0 first, or then the position past the end (d[n-1] - 0)
+      const int a = q.axis[k];
+      const int ca = a == 2 ? (fwd ? c[2] : c[2] + 3) : (a == 1 ? c[1] : c[0]);
+      const int na = a == 2 ? q.n[2] : (a == 1 ? q.n[1] : q.n[0]);
+      if (fwd ? ca == 0 : ca == na - 1) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          if (a != 2 || j == (fwd ? 0 : 3))
+            v[j] = fwd ? ct::fadd(ct::fsub(0.0f, dc[k][j]), v[j]) : ct::fadd(v[j], dc[k][j]);
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) acc[j] = k == 0 ? v[j] : ct::fadd(acc[j], v[j]);
+  }
+  *reinterpret_cast<float4*>(x + (size_t)blockIdx.y * q.count + e) = make_float4(acc[0], acc[1], acc[2], acc[3]);
+}
+
 // Launch of the same-shape kernels.
 template <bool ADJ, int NB, int U>
 void fd_rows_launch(const float* src, float* dst, const FdSame& q, dim3 g, cudaStream_t s) {
@@ -395,6 +498,17 @@ void fd_rows_launch(const float* src, float* dst, const FdSame& q, dim3 g, cudaS
 
 template <bool ADJ, int NB>
 ct_status fd_same_launch(const float* src, float* dst, const FdSame& q, int batch, cudaStream_t s) {
+  if (q.n[2] % 4 == 0 && ct::aligned(src, 16) && ct::aligned(dst, 16)) {
+    const dim3 g((q.count / 4 + kFdT - 1) / kFdT, batch);
+    if constexpr (ADJ) {
+      auto f = q.mode == 0 ? k_fd_adj_quads<NB, 0> : (q.mode == 1 ? k_fd_adj_quads<NB, 1> : k_fd_adj_quads<NB, 2>);
+      f<<<g, kFdT, 0, s>>>(src, dst, q);
+    } else {
+      auto f = q.mode == 0 ? k_fd_fwd_quads<NB, 0> : (q.mode == 1 ? k_fd_fwd_quads<NB, 1> : k_fd_fwd_quads<NB, 2>);
+      f<<<g, kFdT, 0, s>>>(src, dst, q);
+    }
+    return ct::launch_check("k_fd_quads");
+  }
   if (q.n[2] >= 32) {
     const dim3 g((q.units + kFdT / 32 - 1) / (kFdT / 32), batch);
     switch (q.per_lane) {

@@ -19,7 +19,8 @@ pytestmark = pytest.mark.gpu
 
 MODES = [dict(append=0), dict(append=1), dict(prepend=0), dict(prepend=1), dict(circular=True)]
 SHAPES = [((1023,), None), ((1025,), None), ((1, 7), None), ((33, 31), (1, 0)), ((7, 1, 151), None),
-          ((5, 37, 29), (2, 0)), ((16, 64, 4), (0, 1, 2)), ((5, 37, 29), (1,))]
+          ((5, 37, 29), (2, 0)), ((16, 64, 4), (0, 1, 2)), ((5, 37, 29), (1,)),
+          ((1024,), None), ((12, 40), (1, 0)), ((3, 5, 260), None), ((6, 9, 8), (2, 0)), ((1, 3, 4), None)]  # whole quads
 
 
 @pytest.mark.parametrize("kw", MODES, ids=str)
@@ -39,6 +40,18 @@ def test_same_shape_differences(cuda, shape, axes, kw):
         np.testing.assert_array_equal(y[b], np.stack(ref))
         want = ctref.fd_adj(d[b], shape, axes=ax, **kw)
         np.testing.assert_array_equal(back[b], want)
+
+
+@pytest.mark.parametrize("kw", MODES, ids=str)
+@pytest.mark.parametrize("shape", [(6, 40), (3, 5, 64)], ids=str)
+def test_differences_off_a_quad_boundary(cuda, shape, kw):
+    """Arrays that start off a 16-byte boundary: the bits of aligned ones."""
+    D, n = linop.FiniteDifference(shape, **kw), int(np.prod(shape))
+    v = torch.from_numpy(np.random.default_rng(n).standard_normal((1 + len(shape)) * n).astype(np.float32)).to(cuda)
+    x, d = v[:n].clone().view((1,) + shape), v[n:].clone().view((1, len(shape)) + shape)
+    xs, ds = (torch.empty(t.numel() + 1, device=cuda)[1:].view(t.shape).copy_(t) for t in (x, d))
+    assert xs.is_contiguous() and xs.data_ptr() % 16
+    assert torch.equal(D._eval(xs), D._eval(x)) and torch.equal(D._adj(ds), D._adj(d))
 
 
 @pytest.mark.parametrize("ncomp", [1, 2, 3, 4])
