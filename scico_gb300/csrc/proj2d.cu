@@ -21,7 +21,7 @@
 //   No atomics: the result is bit-reproducible.
 // Adjoint (A^T), k_proj2d_adj: pixel-driven gather with the same weights.  A
 //   CTA owns a 64x64 pixel tile; per run of 32 views it stages the tile's
-//   detector windows in shared memory as (y[k] - y[k+1], y[k+1]) pairs (zero outside
+//   detector windows in shared memory as (y[k], y[k+1]) pairs (zero outside
 //   the detector), then each thread accumulates its 4 x 4 pixels over the
 //   views in view order.  Small images split the views into a fixed number
 //   of runs whose partial images are summed in run order.
@@ -599,33 +599,26 @@ struct AdjArgs {
 };
 
 // One view's contribution to this thread's pixels of NI images.  Fast path: the
-// window entries of key k, (y[k] - y[k+1], y[k+1]) with the images side by
-// side, live at shared address off + 8 NI (kMagicBits + k) for the float bits
-// kMagicBits + k of kMagic + k.  The Px, floor and distance steps of two pixels
-// run as paired instructions (bit-identical to the scalar form); the column
-// products Pdx1 * j are shared by the thread's rows and the weights by the images.
-// A pixel adds y[k+1] + w (y[k] - y[k+1]): one multiply-add rounded at y's
-// size and one addition at the sum's, where w y[k] + (1 - w) y[k+1] took 1 - w
-// and two roundings at the sum's: 512^2 x 360 views 37.9 -> 35.3 us, 768^2 x 180
-// 45.0 -> 42.0 us, error against 64 bits 9.0e-8 -> 8.8e-8 at 512^2 (with the sums
-// unpaired 35.6 us, and 256^2 11.1 -> 11.5 us).
+// window pairs of key k (images side by side) live at shared address
+// off + 8 NI (kMagicBits + k) for the float bits kMagicBits + k of kMagic + k.
+// The Px, floor, distance and 1 - w steps of two pixels run as paired
+// instructions (bit-identical to the scalar form); the column products Pdx1 * j
+// are shared by the thread's rows and the weights by the images.
 template <int NI>
-__device__ __forceinline__ void ld_window(uint32_t at, float (&d)[NI], float (&y)[NI]) {
-  if constexpr (NI == 1) {
-    const float2 v = ld_shared2(at);
-    d[0] = v.x;
-    y[0] = v.y;
-  } else {
+__device__ __forceinline__ void ld_window(uint32_t at, float2 (&y)[NI]) {
+  if constexpr (NI == 1)
+    y[0] = ld_shared2(at);
+  else
     asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
-                 : "=f"(d[0]), "=f"(d[1]), "=f"(y[0]), "=f"(y[1])
+                 : "=f"(y[0].x), "=f"(y[0].y), "=f"(y[1].x), "=f"(y[1].y)
                  : "r"(at));
-  }
 }
 
 template <int NI>
 __device__ __forceinline__ void adj_view_fast2(const float4 pv, uint32_t off, const float (&fi)[kAR],
                                                const float (&fj)[kAPX], float (&acc)[NI][kAR][kAPX]) {
   const unsigned long long M2 = pk2(kMagic, kMagic), M12 = pk2(kMagic - 1.0f, kMagic - 1.0f);
+  const unsigned long long one2 = pk2(1.0f, 1.0f);
   float pj[kAPX];
 #pragma unroll
   for (int q = 0; q < kAPX; ++q) pj[q] = ct::fmul(pv.z, fj[q]);
@@ -642,24 +635,24 @@ __device__ __forceinline__ void adj_view_fast2(const float4 pv, uint32_t off, co
       upk2(t2, t0, t1);
       upk2(d2, d0, d1);
       const float w0 = __saturatef(ct::fmul(d0, pv.w)), w1 = __saturatef(ct::fmul(d1, pv.w));
-      float d0v[NI], b0v[NI], d1v[NI], b1v[NI];
-      ld_window<NI>(off + 8u * NI * (uint32_t)__float_as_int(t0), d0v, b0v);
-      ld_window<NI>(off + 8u * NI * (uint32_t)__float_as_int(t1), d1v, b1v);
-      float(&ua)[kAPX] = acc[0][r], (&ub)[kAPX] = acc[NI - 1][r];
-      const float p0 = fmaf(d0v[0], w0, b0v[0]), p1 = fmaf(d1v[0], w1, b1v[0]);
-      if constexpr (NI == 1) {  // pairs of columns
-        upk2(fadd2(pk2(ua[2 * h], ua[2 * h + 1]), pk2(p0, p1)), ua[2 * h], ua[2 * h + 1]);
-      } else {  // pairs of images
-        const float q0 = fmaf(d0v[NI - 1], w0, b0v[NI - 1]), q1 = fmaf(d1v[NI - 1], w1, b1v[NI - 1]);
-        upk2(fadd2(pk2(ua[2 * h], ub[2 * h]), pk2(p0, q0)), ua[2 * h], ub[2 * h]);
-        upk2(fadd2(pk2(ua[2 * h + 1], ub[2 * h + 1]), pk2(p1, q1)), ua[2 * h + 1], ub[2 * h + 1]);
+      float o0, o1;
+      upk2(fsub2(one2, pk2(w0, w1)), o0, o1);
+      float2 y0[NI], y1[NI];
+      ld_window<NI>(off + 8u * NI * (uint32_t)__float_as_int(t0), y0);
+      ld_window<NI>(off + 8u * NI * (uint32_t)__float_as_int(t1), y1);
+#pragma unroll
+      for (int n = 0; n < NI; ++n) {
+        acc[n][r][2 * h] = fmaf(y0[n].x, w0, acc[n][r][2 * h]);
+        acc[n][r][2 * h] = fmaf(y0[n].y, o0, acc[n][r][2 * h]);
+        acc[n][r][2 * h + 1] = fmaf(y1[n].x, w1, acc[n][r][2 * h + 1]);
+        acc[n][r][2 * h + 1] = fmaf(y1[n].y, o1, acc[n][r][2 * h + 1]);
       }
     }
   }
 }
 
 template <int NI>
-__device__ __forceinline__ void adj_view_gen(const float4 pv, float width, int base, const float* __restrict__ wy,
+__device__ __forceinline__ void adj_view_gen(const float4 pv, float width, int base, const float2* __restrict__ wy,
                                              const float (&fi)[kAR], const float (&fj)[kAPX],
                                              float (&acc)[NI][kAR][kAPX]) {
 #pragma unroll
@@ -671,9 +664,13 @@ __device__ __forceinline__ void adj_view_gen(const float4 pv, float width, int b
       int key;
       float w;
       weight_floor(px, width, pv.w, base, key, w);
-      const float* y = wy + 2 * NI * key;
+      const float o = ct::fsub(1.0f, w);
 #pragma unroll
-      for (int n = 0; n < NI; ++n) acc[n][r][q] = ct::fadd(acc[n][r][q], fmaf(y[n], w, y[NI + n]));
+      for (int n = 0; n < NI; ++n) {
+        const float2 y = wy[key * NI + n];
+        acc[n][r][q] = fmaf(y.x, w, acc[n][r][q]);
+        acc[n][r][q] = fmaf(y.y, o, acc[n][r][q]);
+      }
     }
   }
 }
@@ -689,8 +686,8 @@ __device__ __forceinline__ void adj_tile(const AdjArgs& a) {
   ct::grid_dep_trigger();
   if (a.skip && *a.skip != 0.0) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  float* sy = reinterpret_cast<float*>(smem_raw);                   // [kAVC][W][2][NI]
-  float4* sp = reinterpret_cast<float4*>(sy + kAVC * a.W * 2 * NI);  // [kAVC] pxmin, pd0, pd1, 1/width
+  float2* sy = reinterpret_cast<float2*>(smem_raw);             // [kAVC][W][NI]
+  float4* sp = reinterpret_cast<float4*>(sy + kAVC * a.W * NI);  // [kAVC] pxmin, pd0, pd1, 1/width
   float* sw = reinterpret_cast<float*>(sp + kAVC);              // [kAVC] width
   int* sb = reinterpret_cast<int*>(sw + kAVC);                  // [kAVC] window base
   int* sf = sb + kAVC;                                          // [kAVC] 1 = fast floor, -1 = skip
@@ -737,29 +734,22 @@ __device__ __forceinline__ void adj_tile(const AdjArgs& a) {
         f = -1;
       }
       sf[tid] = f;
-      so[tid] = ct::smem_u32(sy + tid * a.W * 2 * NI) - 8u * NI * (uint32_t)(kMagicBits + base);
+      so[tid] = ct::smem_u32(sy + tid * a.W * NI) - 8u * NI * (uint32_t)(kMagicBits + base);
     }
     __syncthreads();
     for (int v = warp; v < n; v += kWarps) {
       const float* yr = yb + (size_t)(a0 + v) * a.det;
       const int base = sb[v];
-      float* wy = sy + v * a.W * 2 * NI;
+      float2* wy = sy + v * a.W * NI;
       for (int k = lane; k < a.W; k += 32) {
         const int bin = base + k;
         const bool in0 = (unsigned)bin < (unsigned)a.det, in1 = (unsigned)(bin + 1) < (unsigned)a.det;
-        float y0[NI], y1[NI];
 #pragma unroll
         for (int m = 0; m < NI; ++m) {
           const bool image = NI == 1 || b + m < a.batch;
           const float* q = yr + m * sino_n + bin;
-          y0[m] = image && in0 ? __ldg(q) : 0.0f;
-          y1[m] = image && in1 ? __ldg(q + 1) : 0.0f;
+          wy[k * NI + m] = make_float2(image && in0 ? __ldg(q) : 0.0f, image && in1 ? __ldg(q + 1) : 0.0f);
         }
-        if constexpr (NI == 1)
-          *reinterpret_cast<float2*>(wy + 2 * k) = make_float2(ct::fsub(y0[0], y1[0]), y1[0]);
-        else
-          *reinterpret_cast<float4*>(wy + 4 * k) =
-              make_float4(ct::fsub(y0[0], y1[0]), ct::fsub(y0[1], y1[1]), y1[0], y1[1]);
       }
     }
     __syncthreads();
@@ -768,7 +758,7 @@ __device__ __forceinline__ void adj_tile(const AdjArgs& a) {
       if (f == 1)
         adj_view_fast2<NI>(sp[v], so[v], fi, fj, acc);
       else if (f == 0)
-        adj_view_gen<NI>(sp[v], sw[v], sb[v], sy + v * a.W * 2 * NI, fi, fj, acc);
+        adj_view_gen<NI>(sp[v], sw[v], sb[v], sy + v * a.W * NI, fi, fj, acc);
     }
   }
   auto store = [&](int m) {
