@@ -1007,7 +1007,8 @@ Proj2dPlan proj2d_plan_sched(const ct_geom2d* g, int batch, Sched2d sc) {
   // 180 45.8 us at 9, 44.2 us at 8; two images a CTA against one: 16 x 256^2 x 180
   // 57 against 75 us, 2 x 512^2 x 360 54 against 75 us, 4 x 300^2 x 200 28 against 35 us.
   {
-    const int first = sc.ns > 0 ? ns : std::min(2, ns), most = sc.ns > 0 || ns == 1 ? ns : ns_max;
+    // at least three quarters of the splits that fill the SMs, so that no sum gets much longer
+    const int first = sc.ns > 0 ? ns : std::min(ns, std::max(2, (3 * ns + 3) / 4)), most = sc.ns > 0 || ns == 1 ? ns : ns_max;
     double least = 1e300;
     for (int ni = 1; ni <= std::min(batch, 2); ++ni) {
       if (adj_smem_bytes(p.W, ni) > 70 * 1024 && ni > 1) break;

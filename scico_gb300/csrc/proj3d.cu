@@ -537,7 +537,7 @@ __global__ void __launch_bounds__(256) k_p3_ax0_rows(const float* __restrict__ a
 // of shared reads per interaction instead of the 8 of one (y[c], y[c+1]) pair
 // each, which bound the version before (lane = pixel, 32 slices of
 // accumulators).  Weights and row offsets come from a table that a warp makes
-// for its pixels, half a warp per view.  256^3 x 360 views: 2258 -> 1544 us (two view
+// for its pixels, half a warp per view.  256^3 x 360 views: 2258 -> 1494 us (two view
 // splits), of issue slots (19 a pixel and view) and shared reads alike.
 // ---------------------------------------------------------------------------
 constexpr int kAdjTile = 16;   // tile edge (pixels)
@@ -1043,8 +1043,14 @@ Proj3dPlan proj3d_plan_sched(const ct_geom3d* g, Sched3d sc) {
     };
     auto lanes = [&](int k) { return cost(4, k) <= std::min(cost(2, k), cost(1, k)) ? 4 : (cost(2, k) <= cost(1, k) ? 2 : 1); };
     const int most = std::max(1, V / (2 * kAdjViews));
+    ns_max = std::max(1, V / 16);
+    // the scratch that a call has always needed (32 x 16 pixel tiles of 32 slices)
+    const long old_ctas = (long)((NK + 31) / 32) * ((NJ + 15) / 16) * (p.Spad / 32);
+    const int old_ns = std::min(old_ctas < 304 ? (int)((304 + old_ctas - 1) / old_ctas) : 1, ns_max);
+    // and no fewer splits than those, so that no sum gets longer (134 x 200 x 72, 64
+    // views: one split instead of two has 1.7 times the error against 64 bits)
     double least = 1e300;
-    for (int k = 1; k <= std::min(16, most); ++k) {
+    for (int k = std::min({16, most, old_ns}); k <= std::min(16, most); ++k) {
       const double c = cost(lanes(k), k);
       if (c < 0.98 * least) {
         least = c;
@@ -1052,10 +1058,6 @@ Proj3dPlan proj3d_plan_sched(const ct_geom3d* g, Sched3d sc) {
       }
     }
     p.adj_sl = lanes(sc.ns > 0 ? std::min(sc.ns, most) : ns);
-    ns_max = std::max(1, V / 16);
-    // the scratch that a call has always needed (32 x 16 pixel tiles of 32 slices)
-    const long old_ctas = (long)((NK + 31) / 32) * ((NJ + 15) / 16) * (p.Spad / 32);
-    const int old_ns = std::min(old_ctas < 304 ? (int)((304 + old_ctas - 1) / old_ctas) : 1, ns_max);
     least_scratch(old_ns, std::min(kMaxSplits3d, ns_max));
     ns_max = most;
   } else {
