@@ -84,7 +84,9 @@ typedef struct ct_geom2d {
   float max_width;   /* max_width_out of ct_proj2d_views for the table */
 } ct_geom2d;
 
-/* Workspace bytes that ct_proj2d_fwd / ct_proj2d_adj need for `batch`. */
+/* Workspace bytes that ct_proj2d_fwd / ct_proj2d_adj use for `batch` under any
+ * schedule.  An adjoint given less runs with fewer view splits, down to a least
+ * size (zero where one split is enough); below it CT_ERR_WORKSPACE. */
 ct_status ct_proj2d_workspace(const ct_geom2d* g, int32_t batch,
                               size_t* fwd_bytes, size_t* adj_bytes);
 
@@ -266,7 +268,10 @@ typedef struct ct_geom3d {
   const uint16_t* order;   /* device, n_views*CT_PROJ3D_ORDER (AXIS0)   */
 } ct_geom3d;
 
-/* Workspace bytes that ct_proj3d_fwd / ct_proj3d_adj need for `batch`. */
+/* Workspace bytes that ct_proj3d_fwd / ct_proj3d_adj use for `batch` under any
+ * schedule.  Calls given less run with fewer tile groups or view splits, down to a
+ * least size; below it CT_ERR_WORKSPACE.  A GENERAL forward needs none: without
+ * (or with too little) it runs its slower kernel. */
 ct_status ct_proj3d_workspace(const ct_geom3d* g, int32_t batch,
                               size_t* fwd_bytes, size_t* adj_bytes);
 
@@ -274,9 +279,10 @@ ct_status ct_proj3d_workspace(const ct_geom3d* g, int32_t batch,
  * proj[b] = A vol[b]  (XRayTransform3D.project / _project / _project_single,
  * _xray3d.py:95-159; weights _calc_weights :206-266).  vol (batch, n0, n1, n2)
  * -> proj (batch, n_views, rows, cols).  The reference scatters four taps
- * per voxel with mode="drop"; here every detector pixel gathers its taps
- * (GENERAL) or each slice's column contributions are accumulated by one
- * owner in a fixed order (AXIS0): no atomics, deterministic.
+ * per voxel with mode="drop"; here windows of voxels scatter into their own
+ * detector tiles, which are then gathered per pixel (GENERAL), or each slice's
+ * column contributions are accumulated by one owner in a fixed order (AXIS0): no
+ * atomics, deterministic.
  */
 ct_status ct_proj3d_fwd(const ct_geom3d* g, const float* vol, float* proj,
                         int32_t batch, void* workspace, size_t workspace_bytes,
@@ -415,7 +421,8 @@ ct_status ct_l21_norm(const float* v, int32_t ncomp, int64_t n,
  * overlap in time (issue them on one stream). */
 size_t ct_reduce_workspace(void);
 
-/* *out_dev (float64, device) = sum a[i] b[i], products and sums in float64,
+/* *out_dev (float64, device) = sum a[i] b[i] to float64's accuracy (exact
+ * float32 splittings of groups of products, or products and sums in float64),
  * fixed summation order. */
 ct_status ct_dot(const float* a, const float* b, int64_t n, double* out_dev,
                  void* workspace, size_t workspace_bytes, ct_stream_t stream);
