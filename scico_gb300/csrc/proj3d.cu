@@ -988,17 +988,14 @@ Proj3dPlan proj3d_plan_sched(const ct_geom3d* g, Sched3d sc) {
     auto fwd_best = [&](int G, Proj3dPlan& q) {
       double best = 1e300;
       for (int sl = 4; sl >= 1; sl /= 2)
-        for (int nw = 16; nw >= 4; nw /= 2)
-          {
-            if (getenv("X_SL") && sl != atoi(getenv("X_SL"))) continue;
-            if (getenv("X_NW") && nw != atoi(getenv("X_NW"))) continue;
-            const double c = fwd_cost(sl, nw, G);
-            if (c < 0.98 * best) {
-              best = c;
-              q.fwd_sl = sl;
-              q.fwd_nw = nw;
-            }
+        for (int nw = 16; nw >= 4; nw /= 2) {
+          const double c = fwd_cost(sl, nw, G);
+          if (c < 0.98 * best) {
+            best = c;
+            q.fwd_sl = sl;
+            q.fwd_nw = nw;
           }
+        }
       return best;
     };
     p.G = std::min(std::max(sc.G, 1), g_max);
