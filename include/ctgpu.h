@@ -268,6 +268,17 @@ typedef struct ct_geom3d {
   const uint16_t* order;   /* device, n_views*CT_PROJ3D_ORDER (AXIS0)   */
 } ct_geom3d;
 
+/*
+ * Which kernel a GENERAL forward with scratch takes for each view of a host table
+ * (views_out of ct_proj3d_views): taken_out[v] = 0 the march over detector pixels
+ * (voxels too coarse or fine for a window's tile, matrix rows so nearly parallel
+ * that float32 does not place the windows), 1 the windows, 2 the windows over a
+ * copy of the volume with axis 2 outermost.  The device decides by the same
+ * test; host code only.  No reference counterpart.
+ */
+ct_status ct_proj3d_window_views(const float* views, int32_t n_views,
+                                 const int32_t* shape, int32_t* taken_out);
+
 /* Workspace bytes that ct_proj3d_fwd / ct_proj3d_adj use for `batch` under any
  * schedule.  Calls given less run with fewer tile groups or view splits, down to a
  * least size; below it CT_ERR_WORKSPACE.  A GENERAL forward needs none: without

@@ -206,6 +206,7 @@ _SIGNATURES = {
     "ct_proj2d_schedule_clear": (None, []),
     "ct_fbp_filter": (ctypes.c_int, [P, P, c_int32, c_int32, P]),
     "ct_proj3d_views": (ctypes.c_int, [P, c_int32, P, P, P, P, P, P]),
+    "ct_proj3d_window_views": (ctypes.c_int, [P, c_int32, P, P]),
     "ct_proj3d_workspace": (ctypes.c_int, [P, c_int32, P, P]),
     "ct_proj3d_fwd": (ctypes.c_int, [P, P, P, c_int32, P, c_size_t, P]),
     "ct_proj3d_adj": (ctypes.c_int, [P, P, P, c_int32, P, c_size_t, P]),

@@ -88,9 +88,27 @@ inline int quad_ok(size_t n, const P*... ptrs) {
 // same IEEE operations, in the same order, as the reference's float32
 // expressions, so the compiler may not contract a*b+c into an FMA there.
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ float fmul(float a, float b) { return __fmul_rn(a, b); }
-__device__ __forceinline__ float fadd(float a, float b) { return __fadd_rn(a, b); }
-__device__ __forceinline__ float fsub(float a, float b) { return __fsub_rn(a, b); }
+__host__ __device__ __forceinline__ float fmul(float a, float b) {
+#ifdef __CUDA_ARCH__
+  return __fmul_rn(a, b);
+#else
+  return a * b;
+#endif
+}
+__host__ __device__ __forceinline__ float fadd(float a, float b) {
+#ifdef __CUDA_ARCH__
+  return __fadd_rn(a, b);
+#else
+  return a + b;
+#endif
+}
+__host__ __device__ __forceinline__ float fsub(float a, float b) {
+#ifdef __CUDA_ARCH__
+  return __fsub_rn(a, b);
+#else
+  return a - b;
+#endif
+}
 
 // Detector position of pixel (i, j) for one view:
 // (Pxmin + Pdx0*i) + Pdx1*j, each operation rounded to float32

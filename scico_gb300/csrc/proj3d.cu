@@ -948,6 +948,16 @@ ct_status proj3d_check(const ct_geom3d* g, const char* who) {
 constexpr int kMaxSplits3d = 4;
 constexpr size_t kGenScratch = 96u << 20;  // bytes of GENERAL forward tiles per launch
 
+// Windows of one view of a GENERAL forward: a bound over the marching axes.
+int gen_windows_bound(const int32_t* n) {
+  long nwin = 0;
+  for (int ax = 0; ax < 3; ++ax) {
+    const long na = n[ax], np = n[ax == 0 ? 1 : 0], nq = n[ax == 2 ? 1 : 2];
+    nwin = std::max(nwin, ((np + na) / kWin + 2) * ((nq + na) / kWin + 2));
+  }
+  return (int)std::min<long>(nwin, 1 << 20);
+}
+
 // The AXIS0 span bounds need max |M[1][1]| and |M[1][2]|; ct_proj3d_views
 // guarantees both <= 1, so the bounds are fixed.
 Proj3dPlan proj3d_plan_sched(const ct_geom3d* g, Sched3d sc) {
@@ -1075,16 +1085,10 @@ Proj3dPlan proj3d_plan_sched(const ct_geom3d* g, Sched3d sc) {
     const long old_ctas = (long)(((double)S * NJ * NK + 255) / 256);
     const int old_ns = std::min(old_ctas < 4L * sms ? (int)((4L * sms + old_ctas - 1) / old_ctas) : 1, ns_max);
     least_scratch(old_ns, std::min(kMaxSplits3d, ns_max));
-    // forward: windows of a view (bound over the marching axes), plane segments
-    // until two warps a slot are there, views per launch until the tiles of a
-    // launch pass kGenScratch (they are read back from L2)
-    const int n3[3] = {S, NJ, NK};
-    long nwin = 0;
-    for (int ax = 0; ax < 3; ++ax) {
-      const long na = n3[ax], np = n3[ax == 0 ? 1 : 0], nq = n3[ax == 2 ? 1 : 2];
-      nwin = std::max(nwin, ((np + na) / kWin + 2) * ((nq + na) / kWin + 2));
-    }
-    p.nwin = (int)std::min<long>(nwin, 1 << 20);
+    // forward: windows of a view, plane segments until two warps a slot are
+    // there, views per launch until the tiles of a launch pass kGenScratch (they
+    // are read back from L2)
+    p.nwin = gen_windows_bound(g->shape);
     const long warps = std::max(1L, p.nwin / 4L * V), target = 40L * sms;
     p.nseg = (int)std::min<long>(std::max(1L, (target + warps - 1) / warps),
                                  std::max(1, std::min(S, std::min(NJ, NK)) / 8));
@@ -1379,6 +1383,21 @@ ct_status ct_proj3d_views(const float* matrices, int32_t n_views, const int32_t*
       for (int p = 0; p < CT_PROJ3D_ORDER; ++p)
         order_out[(size_t)v * CT_PROJ3D_ORDER + p] = (uint16_t)key[p].second;
     }
+  }
+  return CT_OK;
+}
+
+ct_status ct_proj3d_window_views(const float* views, int32_t n_views, const int32_t* shape, int32_t* taken_out) {
+  if (!views || !shape || !taken_out) return ct::fail(CT_ERR_INVALID_ARG, "ct_proj3d_window_views: null argument");
+  if (n_views <= 0) return ct::fail(CT_ERR_SHAPE, "ct_proj3d_window_views: n_views=%d", n_views);
+  for (int q = 0; q < 3; ++q)
+    if (shape[q] <= 0) return ct::fail(CT_ERR_SHAPE, "ct_proj3d_window_views: shape[%d]=%d", q, shape[q]);
+  const int nwin = ct::gen_windows_bound(shape);
+  for (int v = 0; v < n_views; ++v) {
+    const float* m = views + (size_t)v * CT_VIEW3D_STRIDE;
+    if (!(m[8] == 0.0f || m[8] == 1.0f || m[8] == 2.0f))
+      return ct::fail(CT_ERR_INVALID_ARG, "ct_proj3d_window_views: view %d is not of ct_proj3d_views", v);
+    taken_out[v] = !ct::gen_view_fits(m, shape[0], shape[1], shape[2], nwin) ? 0 : (m[8] == 2.0f ? 2 : 1);
   }
   return CT_OK;
 }

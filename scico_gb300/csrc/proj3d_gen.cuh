@@ -135,7 +135,17 @@ struct GenView {
   float i00, i01, i10, i11;  // (1 / kWin) inverse of the (p, q) columns
 };
 
-__device__ __forceinline__ int gen_shift(float d, int ia) { return (int)floorf(fadd(fmul(d, (float)ia), 0.5f)); }
+__host__ __device__ __forceinline__ float gen_div(float a, float b) {
+#ifdef __CUDA_ARCH__
+  return __fdiv_rn(a, b);
+#else
+  return a / b;
+#endif
+}
+
+__host__ __device__ __forceinline__ int gen_shift(float d, int ia) {
+  return (int)floorf(fadd(fmul(d, (float)ia), 0.5f));
+}
 
 __device__ __forceinline__ void gen_tile_base(const GenView& g, int I, int J, int& b0, int& b1) {
   const float x = (float)(kWin * I), y = (float)(kWin * J);
@@ -143,13 +153,14 @@ __device__ __forceinline__ void gen_tile_base(const GenView& g, int I, int J, in
   b1 = (int)floorf(fadd(g.b1, fadd(fmul(g.mp1, x), fmul(g.mq1, y))));
 }
 
-// By all 32 lanes of one warp; valid in every lane.
-__device__ GenView gen_view(const float* __restrict__ m, int n0, int n1, int n2, int nwin) {
-  const int lane = threadIdx.x & 31;
-  GenView g;
+// Everything of a view's plan but phases and LD; returns the tests of `ok` that
+// concern the view as a whole.
+__host__ __device__ inline bool gen_view_base(GenView& g, const float* m, int n0, int n1, int n2, int nwin) {
+  auto pick = [&](int k) { return k == 0 ? n0 : (k == 1 ? n1 : n2); };
+  auto least = [](int a, int b) { return a < b ? a : b; };
+  auto most = [](int a, int b) { return a > b ? a : b; };
   g.ax = (int)m[8];
   const int p = g.ax == 0 ? 1 : 0, q = g.ax == 2 ? 1 : 2;
-  auto pick = [&](int k) { return k == 0 ? n0 : (k == 1 ? n1 : n2); };
   g.na = pick(g.ax);
   g.np = pick(p);
   g.nq = pick(q);
@@ -162,24 +173,31 @@ __device__ GenView gen_view(const float* __restrict__ m, int n0, int n1, int n2,
   g.c0 = m[3];
   g.c1 = m[7];
   const float det = fsub(fmul(g.mp0, g.mq1), fmul(g.mq0, g.mp1));
-  g.dp = -__fdiv_rn(fsub(fmul(g.mq1, g.ma0), fmul(g.mq0, g.ma1)), det);
-  g.dq = -__fdiv_rn(fsub(fmul(g.mp0, g.ma1), fmul(g.mp1, g.ma0)), det);
+  g.dp = -gen_div(fsub(fmul(g.mq1, g.ma0), fmul(g.mq0, g.ma1)), det);
+  g.dq = -gen_div(fsub(fmul(g.mp0, g.ma1), fmul(g.mp1, g.ma0)), det);
   const float w = 1.0f / kWin;
-  g.i00 = __fdiv_rn(fmul(w, g.mq1), det);
-  g.i01 = -__fdiv_rn(fmul(w, g.mq0), det);
-  g.i10 = -__fdiv_rn(fmul(w, g.mp1), det);
-  g.i11 = __fdiv_rn(fmul(w, g.mp0), det);
+  g.i00 = gen_div(fmul(w, g.mq1), det);
+  g.i01 = -gen_div(fmul(w, g.mq0), det);
+  g.i10 = -gen_div(fmul(w, g.mp1), det);
+  g.i11 = gen_div(fmul(w, g.mp0), det);
   // coordinates small enough for the slack, a sane shear
   const float r0 = fabsf(g.ma0) * g.na + fabsf(g.mp0) * g.np + fabsf(g.mq0) * g.nq + fabsf(g.c0);
   const float r1 = fabsf(g.ma1) * g.na + fabsf(g.mp1) * g.np + fabsf(g.mq1) * g.nq + fabsf(g.c1);
   bool ok = r0 < 32768.0f && r1 < 32768.0f && fabsf(g.dp) < 1.01f && fabsf(g.dq) < 1.01f;
+  // the gather's window index of a pixel, off by less than its margin of 0.01:
+  // the terms that cancel in it, each good to a few units of rounding
+  // (nearly parallel matrix rows make them many times the index)
+  const float P = (float)g.np + (float)g.na, Q = (float)g.nq + (float)g.na;
+  const float y0 = fabsf(g.mp0) * P + fabsf(g.mq0) * Q, y1 = fabsf(g.mp1) * P + fabsf(g.mq1) * Q;
+  ok = ok && 0x1p-20f * (fabsf(g.i00) * y0 + fabsf(g.i01) * y1) <= 0.01f &&
+       0x1p-20f * (fabsf(g.i10) * y0 + fabsf(g.i11) * y1) <= 0.01f;
   // shift range over the planes, window ranges
   const int ep = ok ? gen_shift(g.dp, g.na - 1) : 0, eq = ok ? gen_shift(g.dq, g.na - 1) : 0;
   auto fdiv = [](int a) { return a >= 0 ? a / kWin : -((-a + kWin - 1) / kWin); };
-  g.I0 = fdiv(-max(0, ep));
-  g.nI = fdiv(g.np - 1 - min(0, ep)) - g.I0 + 1;
-  g.J0 = fdiv(-max(0, eq));
-  g.nJ = fdiv(g.nq - 1 - min(0, eq)) - g.J0 + 1;
+  g.I0 = fdiv(-most(0, ep));
+  g.nI = fdiv(g.np - 1 - least(0, ep)) - g.I0 + 1;
+  g.J0 = fdiv(-most(0, eq));
+  g.nJ = fdiv(g.nq - 1 - least(0, eq)) - g.J0 + 1;
   ok = ok && (long long)g.nI * g.nJ <= nwin;
   // footprint of a window: its voxels' left positions span
   // [min, max] of kWin (mp x + mq y), x, y in [0, 1] (half a voxel of shift
@@ -195,24 +213,49 @@ __device__ GenView gen_view(const float* __restrict__ m, int n0, int n1, int n2,
   const float l1 = fadd(fmul(fw, fminf(g.mp1, 0.0f)), fmul(fw, fminf(g.mq1, 0.0f)));
   g.b0 = fadd(fadd(fadd(g.c0, fmul(0.5f, g.ma0)), -0.25f - kTileSlack), l0);
   g.b1 = fadd(fadd(fadd(g.c1, fmul(0.5f, g.ma1)), -0.25f - kTileSlack), l1);
-  // the voxels of a step sit 2 apart: displacements (2 di, 2 dj), half plane; two
-  // share a slot only where both components stay below one pixel
-  bool any = false, even = false, both = false;
-  for (int k = lane; k < 15 * 8; k += 32) {
-    const int dj = k / 15, di = k % 15 - 7;
-    if (dj == 0 && di <= 0) continue;
-    const float x = 2.0f * di, y = 2.0f * dj;
-    const float d0 = fabsf(fadd(fmul(g.mp0, x), fmul(g.mq0, y))), d1 = fabsf(fadd(fmul(g.mp1, x), fmul(g.mq1, y)));
-    const bool bad = !(fmaxf(d0, d1) >= 1.0f + 2.0f * kTileSlack);
-    any = any || bad;
-    even = even || (bad && ((di + dj) & 1) == 0);
-    both = both || (bad && (di & 1) == 0 && (dj & 1) == 0);
+  return ok;
+}
+
+// Plane ia's shift keeps its voxels inside the tile: the windows' footprint moves
+// by at most half a voxel either way, as e0 and e1 allow, and a quarter of the
+// slack.  The shears are quotients of differences, which nearly parallel matrix rows
+// leave few digits of; over the planes that adds up to whole pixels.
+__host__ __device__ inline bool gen_plane_fits(const GenView& g, int ia) {
+  const float sp = (float)gen_shift(g.dp, ia), sq = (float)gen_shift(g.dq, ia), xa = (float)ia;
+  const float d0 = fadd(fmul(g.ma0, xa), fadd(fmul(g.mp0, sp), fmul(g.mq0, sq)));
+  const float d1 = fadd(fmul(g.ma1, xa), fadd(fmul(g.mp1, sp), fmul(g.mq1, sq)));
+  return fabsf(d0) <= fadd(fmul(0.5f, fadd(fabsf(g.mp0), fabsf(g.mq0))), 0.25f * kTileSlack) &&
+         fabsf(d1) <= fadd(fmul(0.5f, fadd(fabsf(g.mp1), fabsf(g.mq1))), 0.25f * kTileSlack);
+}
+
+// The voxels of a step sit 2 apart: displacements (2 di, 2 dj), half plane, number k
+// of kLattice; two share a slot only where both components stay below one pixel.
+// Returns 0 where they cannot, else 1, + 2 where di + dj is even, + 4 where both are.
+constexpr int kLattice = 15 * 8;
+__host__ __device__ inline int gen_lattice(const GenView& g, int k) {
+  const int dj = k / 15, di = k % 15 - 7;
+  if (dj == 0 && di <= 0) return 0;
+  const float x = 2.0f * di, y = 2.0f * dj;
+  const float d0 = fabsf(fadd(fmul(g.mp0, x), fmul(g.mq0, y))), d1 = fabsf(fadd(fmul(g.mp1, x), fmul(g.mq1, y)));
+  if (fmaxf(d0, d1) >= 1.0f + 2.0f * kTileSlack) return 0;
+  return 1 + (((di + dj) & 1) == 0 ? 2 : 0) + ((di & 1) == 0 && (dj & 1) == 0 ? 4 : 0);
+}
+
+// By all 32 lanes of one warp; valid in every lane.
+__device__ GenView gen_view(const float* __restrict__ m, int n0, int n1, int n2, int nwin) {
+  const int lane = threadIdx.x & 31;
+  GenView g;
+  bool ok = gen_view_base(g, m, n0, n1, n2, nwin);
+  if (ok) {  // the same in every lane
+    bool fits = true;
+    for (int ia = lane; ia < g.na; ia += 32) fits = fits && gen_plane_fits(g, ia);
+    ok = __all_sync(0xffffffffu, fits);
   }
-  any = __any_sync(0xffffffffu, any);
-  even = __any_sync(0xffffffffu, even);
-  both = __any_sync(0xffffffffu, both);
-  g.phases = !any ? 1 : (!even ? 2 : 4);
-  ok = ok && !both;
+  int shared = 0;
+  for (int k = lane; k < kLattice; k += 32) shared |= gen_lattice(g, k);
+  shared = __reduce_or_sync(0xffffffffu, shared);
+  g.phases = !(shared & 1) ? 1 : (!(shared & 2) ? 2 : 4);
+  ok = ok && !(shared & 4);
   // row stride: lane = (candidate, starting phase); the bank groups that eight
   // lanes in a row along q meet
   const int cand = lane & 7;
@@ -237,6 +280,17 @@ __device__ GenView gen_view(const float* __restrict__ m, int n0, int n1, int n2,
   g.LD = g.T1 + (cost & 7);
   g.ok = ok ? 1 : 0;
   return g;
+}
+
+// gen_view's `ok` on the host (the table as ct_proj3d_views wrote it).
+inline bool gen_view_fits(const float* m, int n0, int n1, int n2, int nwin) {
+  GenView g;
+  if (!gen_view_base(g, m, n0, n1, n2, nwin)) return false;
+  for (int ia = 0; ia < g.na; ++ia)
+    if (!gen_plane_fits(g, ia)) return false;
+  for (int k = 0; k < kLattice; ++k)
+    if (gen_lattice(g, k) & 4) return false;
+  return true;
 }
 
 struct GenFwdArgs {
