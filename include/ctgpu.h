@@ -302,7 +302,9 @@ ct_status ct_proj3d_fwd(const ct_geom3d* g, const float* vol, float* proj,
 /*
  * vol[b] = A^T proj[b]  (XRayTransform3D.back_project / _back_project /
  * _back_project_single, :161-204).  Voxel-driven gather with the forward's
- * weights, views summed in a fixed order.
+ * weights (GENERAL: an axis at a time, so the product of the two is rounded in
+ * another order), views summed in a fixed order.  A pixel of weight 0 adds
+ * nothing, however large; one that is not finite reaches the voxels that read it.
  */
 ct_status ct_proj3d_adj(const ct_geom3d* g, const float* proj, float* vol,
                         int32_t batch, void* workspace, size_t workspace_bytes,

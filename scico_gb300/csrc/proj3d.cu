@@ -10,7 +10,10 @@
 //   (ul0,   ul1+1) t0*(0.5-t1)*4    (ul0+1, ul1+1) (0.5-t0)*(0.5-t1)*4
 // each zeroed when its detector pixel is out of range.  Every kernel here
 // evaluates these expressions with the same float32 operations in the same
-// order (no contraction), so forward and adjoint use bit-identical weights.
+// order (no contraction) up to to_next, so forward and adjoint place every voxel
+// alike and agree bit for bit in each axis's two weights; the GENERAL adjoint
+// multiplies a pixel by the one and then the other (rounded after each) instead
+// of by their rounded product.
 //
 // Two geometry kinds (ct_proj3d_views classifies):
 //  * AXIS0 -- rotation about volume axis 0, slice i on detector row

@@ -337,11 +337,6 @@ __global__ void __launch_bounds__(256) k_p3_gen_setup(const float* __restrict__ 
   }
 }
 
-__device__ __forceinline__ float4 lds128(uint32_t a) {
-  float4 v;
-  asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a) : "memory");
-  return v;
-}
 __device__ __forceinline__ void lds_pairs(uint32_t a, unsigned long long& x, unsigned long long& y) {
   asm volatile("ld.shared.v2.b64 {%0, %1}, [%2];" : "=l"(x), "=l"(y) : "r"(a) : "memory");
 }
@@ -567,20 +562,33 @@ __global__ void __launch_bounds__(kGatherWarps * 32) k_p3_gen_gather(const GenFw
 // brick of kBrick^3 voxels, a thread a column of kBrick along axis 0, and runs
 // over the views in order.  Per view it stages the detector tile that the
 // brick's footprints can touch, one view ahead and zero off the detector, as
-// float4s of two rows' first difference and second pixel (y[r][c] - y[r][c+1],
-// y[r+1][c] - y[r+1][c+1], y[r][c+1], y[r+1][c+1]), so that a voxel is one 16-byte
-// shared load and three multiply-adds between columns and rows, rounded at y's
-// size, then one addition to its sum, without tests, divisions or conversions.  The rows'
+// float4s of a slot's four pixels, (y[r][c], y[r+1][c]) and (y[r][c+1], y[r+1][c+1]),
+// so that a voxel is one 16-byte shared load, w0 y0 + w1 y1 between columns and then
+// rows, and one addition to its sum, without tests, divisions or conversions.
+// Each product and sum is rounded at the size of the voxel's own taps, and a pixel of
+// weight 0 adds nothing, however large (an interpolation from differences of the
+// pixels, three operations less, would round at the size of the larger).  The rows'
 // stride is 1 or 7 modulo 8 by the sign of the two steps along axis 2, so that
 // eight neighbouring lanes walk monotonically over the eight 16-byte bank
 // groups.  Views whose tile does not fit (voxels above ~1.3 detector pixels)
 // gather from global memory.  Bound by the FP32 pipe (some 23 operations a voxel
 // and view).  97 x 128 x 111 voxels, 60 views: one voxel a thread with four
 // scalar gathers 238 us; bricks with the four weights formed and four multiply-adds
-// into the sum 163 us; this 147 us, and a third of the error against 64 bits less
+// into the sum 163 us; this 157 us, and a third of the error against 64 bits less
 // (1.8e-7 -> 1.2e-7).
 // ---------------------------------------------------------------------------
 constexpr int kBrick = 16;
+
+// A voxel's value between the columns (y[r][c], y[r+1][c]), (y[r][c+1], y[r+1][c+1])
+// and then the rows, with the weights 2 min(t, 0.5) and 1 less it of each axis's first
+// and second pixel.
+__device__ __forceinline__ float gen_interp(unsigned long long y0, unsigned long long y1, float t0, float t1) {
+  const float s0 = __saturatef(fadd(t0, t0)), s1 = __saturatef(fadd(t1, t1));
+  const float o0 = __saturatef(fmaf(-2.0f, t0, 1.0f)), o1 = __saturatef(fmaf(-2.0f, t1, 1.0f));
+  float r0, r1;
+  g_upk(g_fma(y0, g_pk(s1, s1), g_mul(y1, g_pk(o1, o1))), r0, r1);
+  return fmaf(r0, s0, fmul(r1, o0));
+}
 constexpr int kAdjSlots = 1024;  // float4 slots of a staged tile
 constexpr int kAdjChunk = 32;    // views whose tiles are laid out at once
 
@@ -642,7 +650,7 @@ __global__ void __launch_bounds__(256, 3) k_p3_gen_adj(const float* __restrict__
 #pragma unroll
     for (int k = 0; k < kStage; ++k)
       if (tid + 256 * k < n)
-        sy[buf][tid + 256 * k] = make_float4(fsub(st[k].x, st[k].y), fsub(st[k].z, st[k].w), st[k].y, st[k].w);
+        sy[buf][tid + 256 * k] = make_float4(st[k].x, st[k].z, st[k].y, st[k].w);
   };
 
   for (int vc = vs; vc < ve; vc += kAdjChunk) {
@@ -703,11 +711,9 @@ __global__ void __launch_bounds__(256, 3) k_p3_gen_adj(const float* __restrict__
             int u0, u1;
             float t0, t1;
             foot_edges(g_add(g_add(g_add(A, P), Q), cc), u0, u1, t0, t1);
-            // 2 min(t, 0.5), the weight of the first of the two pixels
-            const float s0 = __saturatef(fadd(t0, t0)), s1 = __saturatef(fadd(t1, t1));
-            const float4 y = lds128(origin + ld16 * (uint32_t)u0 + 16u * (uint32_t)u1);
-            const float r0 = fmaf(y.x, s1, y.z), r1 = fmaf(y.y, s1, y.w);  // the two rows between their columns
-            v[h] = fmaf(fsub(r0, r1), s0, r1);
+            unsigned long long y0, y1;
+            lds_pairs(origin + ld16 * (uint32_t)u0 + 16u * (uint32_t)u1, y0, y1);
+            v[h] = gen_interp(y0, y1, t0, t1);
           }
           g_upk(g_add(g_pk(acc[k], acc[k + 1]), g_pk(v[0], v[1])), acc[k], acc[k + 1]);
         }
@@ -720,13 +726,13 @@ __global__ void __launch_bounds__(256, 3) k_p3_gen_adj(const float* __restrict__
           float t0, t1;
           edge3(px3(m0, t.m[1], t.m[2], t.m[3], x0, x1, x2), u0, t0);
           edge3(px3(m4, t.m[5], t.m[6], t.m[7], x0, x1, x2), u1, t1);
-          const float s0 = fsub(0.5f, t0), s1 = fsub(0.5f, t1);
           const bool r0 = u0 >= 0 && u0 < R, r1 = u0 + 1 >= 0 && u0 + 1 < R;
           const bool c0 = u1 >= 0 && u1 < C, c1 = u1 + 1 >= 0 && u1 + 1 < C;
-          if (r0 && c0) acc[k] = fmaf(__ldg(y + (size_t)u0 * C + u1), fmul(fmul(t0, t1), 4.0f), acc[k]);
-          if (r1 && c0) acc[k] = fmaf(__ldg(y + (size_t)(u0 + 1) * C + u1), fmul(fmul(s0, t1), 4.0f), acc[k]);
-          if (r0 && c1) acc[k] = fmaf(__ldg(y + (size_t)u0 * C + u1 + 1), fmul(fmul(t0, s1), 4.0f), acc[k]);
-          if (r1 && c1) acc[k] = fmaf(__ldg(y + (size_t)(u0 + 1) * C + u1 + 1), fmul(fmul(s0, s1), 4.0f), acc[k]);
+          const float y00 = r0 && c0 ? __ldg(y + (size_t)u0 * C + u1) : 0.0f;
+          const float y10 = r1 && c0 ? __ldg(y + (size_t)(u0 + 1) * C + u1) : 0.0f;
+          const float y01 = r0 && c1 ? __ldg(y + (size_t)u0 * C + u1 + 1) : 0.0f;
+          const float y11 = r1 && c1 ? __ldg(y + (size_t)(u0 + 1) * C + u1 + 1) : 0.0f;
+          acc[k] = fadd(acc[k], gen_interp(g_pk(y00, y10), g_pk(y01, y11), t0, t1));
         }
       }
       if (next) stage_store((vi + 1) & 1, tv[vi + 1]);
