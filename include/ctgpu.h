@@ -282,7 +282,10 @@ ct_status ct_proj3d_window_views(const float* views, int32_t n_views,
 /* Workspace bytes that ct_proj3d_fwd / ct_proj3d_adj use for `batch` under any
  * schedule.  Calls given less run with fewer tile groups or view splits, down to a
  * least size; below it CT_ERR_WORKSPACE.  A GENERAL forward needs none: without
- * (or with too little) it runs its slower kernel. */
+ * (or with too little) it runs its slower kernel.  The last of its bytes, the
+ * volume's size rounded up to 256, serve the views that ct_proj3d_window_views
+ * reports as 2; a call without them runs the slower kernel for those alone.  Where
+ * that reports 0 for every view, no scratch is the best choice. */
 ct_status ct_proj3d_workspace(const ct_geom3d* g, int32_t batch,
                               size_t* fwd_bytes, size_t* adj_bytes);
 

@@ -61,9 +61,10 @@ struct Proj3dPlan {
   // AXIS0 forward: slices padded to 64, tiles, tile groups, slices a lane
   // and warps (views) a CTA
   int Spad = 0, tiles_k = 0, n_tiles = 0, G = 1, fwd_sl = 4, fwd_nw = 16;
-  // GENERAL forward: windows of a view (bound), segments of the planes, views per launch
+  // GENERAL forward: windows of a view (bound; 0: the march alone), segments of the
+  // planes, views per launch
   int nwin = 0, nseg = 1, gen_views = 1;
-  size_t gen_plan = 0, gen_turn = 0;  // bytes of the views' plans and of the turned volume
+  size_t gen_plan = 0, gen_tiles = 0, gen_turn = 0;  // bytes of the views' plans, their tiles and the turned volume
   // adjoint view splits (both kinds)
   int nsplit = 1, per_split = 0;
   int adj_sl = 4;        // AXIS0 adjoint: slices a lane

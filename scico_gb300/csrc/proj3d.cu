@@ -949,16 +949,34 @@ ct_status proj3d_check(const ct_geom3d* g, const char* who) {
 
 // Most adjoint view splits the tuner tries.
 constexpr int kMaxSplits3d = 4;
-constexpr size_t kGenScratch = 96u << 20;  // bytes of GENERAL forward tiles per launch
+constexpr size_t kGenScratch = 96u << 20;       // bytes of GENERAL forward tiles per launch
+constexpr size_t kGenScratchView = 1024u << 20;  // the most that one view's tiles may take (or the volume's size)
 
-// Windows of one view of a GENERAL forward: a bound over the marching axes.
-int gen_windows_bound(const int32_t* n) {
-  long nwin = 0;
+// Windows of a view of a GENERAL forward (a bound over the marching axes; 0: no
+// windows, the march), segments of its planes until two warps a slot are there, and
+// the bytes of one view's tiles.  Flat volumes thousands of voxels wide have so many windows that their
+// tiles would outgrow the volume itself: those march.
+struct GenTiles {
+  int nwin = 0, nseg = 1;
+  size_t per_view = 0;
+};
+GenTiles gen_tiles(const int32_t* n, int V) {
+  GenTiles t;
+  double nwin = 0;
   for (int ax = 0; ax < 3; ++ax) {
     const long na = n[ax], np = n[ax == 0 ? 1 : 0], nq = n[ax == 2 ? 1 : 2];
-    nwin = std::max(nwin, ((np + na) / kWin + 2) * ((nq + na) / kWin + 2));
+    nwin = std::max(nwin, (double)((np + na) / kWin + 2) * (double)((nq + na) / kWin + 2));
   }
-  return (int)std::min<long>(nwin, 1 << 20);
+  const size_t most = std::max(kGenScratchView, sizeof(float) * (size_t)n[0] * n[1] * n[2]);
+  if (nwin * sizeof(float) * kTilePix > (double)most) return t;
+  t.nwin = (int)nwin;
+  const long warps = std::max(1L, t.nwin / 4L * V), target = 40L * std::max(1, sm_count());
+  t.nseg = (int)std::min<long>(std::max(1L, (target + warps - 1) / warps),
+                               std::max(1, std::min({n[0], n[1], n[2]}) / 8));
+  const size_t one = sizeof(float) * (size_t)t.nwin * kTilePix;
+  t.nseg = (int)std::min<size_t>(t.nseg, std::max<size_t>(1, most / one));
+  t.per_view = one * t.nseg;
+  return t;
 }
 
 // The AXIS0 span bounds need max |M[1][1]| and |M[1][2]|; ct_proj3d_views
@@ -1088,18 +1106,18 @@ Proj3dPlan proj3d_plan_sched(const ct_geom3d* g, Sched3d sc) {
     const long old_ctas = (long)(((double)S * NJ * NK + 255) / 256);
     const int old_ns = std::min(old_ctas < 4L * sms ? (int)((4L * sms + old_ctas - 1) / old_ctas) : 1, ns_max);
     least_scratch(old_ns, std::min(kMaxSplits3d, ns_max));
-    // forward: windows of a view, plane segments until two warps a slot are
-    // there, views per launch until the tiles of a launch pass kGenScratch (they
-    // are read back from L2)
-    p.nwin = gen_windows_bound(g->shape);
-    const long warps = std::max(1L, p.nwin / 4L * V), target = 40L * sms;
-    p.nseg = (int)std::min<long>(std::max(1L, (target + warps - 1) / warps),
-                                 std::max(1, std::min(S, std::min(NJ, NK)) / 8));
-    const size_t per_view = sizeof(float) * (size_t)p.nseg * p.nwin * kTilePix;
-    p.gen_views = (int)std::max<size_t>(1, std::min<size_t>(std::min(V, 65535), kGenScratch / per_view));
-    p.gen_plan = round_up(sizeof(GenView) * (size_t)V, 256);
-    p.gen_turn = round_up(sizeof(float) * (size_t)S * NJ * NK, 256);
-    p.fwd_bytes = p.fwd_ws_bytes = p.gen_plan + p.gen_turn + round_up((size_t)p.gen_views * per_view, 256);
+    // forward: views per launch until the tiles of a launch pass kGenScratch (they
+    // are read back from L2); the turned volume last, so that a call can go without it
+    const GenTiles t = gen_tiles(g->shape, V);
+    p.nwin = t.nwin;
+    p.nseg = t.nseg;
+    if (p.nwin > 0) {
+      p.gen_views = (int)std::max<size_t>(1, std::min<size_t>(std::min(V, 65535), kGenScratch / t.per_view));
+      p.gen_plan = round_up(sizeof(GenView) * (size_t)V, 256);
+      p.gen_tiles = round_up((size_t)p.gen_views * t.per_view, 256);
+      p.gen_turn = round_up(sizeof(float) * (size_t)S * NJ * NK, 256);
+      p.fwd_bytes = p.fwd_ws_bytes = p.gen_plan + p.gen_tiles + p.gen_turn;
+    }
   }
   ns = std::min(ns, ns_max);
   const int ns_ws = std::max(ns, std::min(kMaxSplits3d, ns_max));
@@ -1234,14 +1252,14 @@ ct_status proj3d_fwd_launch(const ct_geom3d* g, const Proj3dPlan& p, const float
                                              g->row_offset, skip);
     return launch_check("k_p3_ax0_rows");
   }
-  GenView* plan = static_cast<GenView*>(ws);
-  if (ws) {
+  GenView* plan = p.nwin > 0 ? static_cast<GenView*>(ws) : nullptr;
+  if (plan) {
     GenFwdArgs a;
-    float* turned = reinterpret_cast<float*>(static_cast<char*>(ws) + p.gen_plan);
+    float* turned = p.gen_turn ? reinterpret_cast<float*>(static_cast<char*>(ws) + p.gen_plan + p.gen_tiles) : nullptr;
     a.vol = vol;
     a.vol_t = turned;
     a.plan = plan;
-    a.part = reinterpret_cast<float*>(static_cast<char*>(ws) + p.gen_plan + p.gen_turn);
+    a.part = reinterpret_cast<float*>(static_cast<char*>(ws) + p.gen_plan);
     a.proj = proj;
     a.n0 = S;
     a.n1 = NJ;
@@ -1251,7 +1269,7 @@ ct_status proj3d_fwd_launch(const ct_geom3d* g, const Proj3dPlan& p, const float
     a.nwin = p.nwin;
     a.nseg = p.nseg;
     a.skip = skip;
-    const unsigned turn_blocks = (unsigned)((S * (long)NJ + 31) / 32) * (unsigned)((NK + 31) / 32);
+    const unsigned turn_blocks = !turned ? 0 : (unsigned)((S * (long)NJ + 31) / 32) * (unsigned)((NK + 31) / 32);
     k_p3_gen_setup<<<(V + 7) / 8 + turn_blocks, 256, 0, s>>>(g->views, plan, vol, turned, S, NJ, NK, V, p.nwin, skip);
     ct_status st = launch_check("k_p3_gen_setup");
     if (st != CT_OK) return st;
@@ -1269,7 +1287,7 @@ ct_status proj3d_fwd_launch(const ct_geom3d* g, const Proj3dPlan& p, const float
   }
   // with windows, few blocks a view: most find it taken
   const int full = (int)(((long)R * C + 255) / 256);
-  dim3 grid(ws ? std::min(full, std::max(16, 16 * sm_count() / V)) : full, V);
+  dim3 grid(plan ? std::min(full, std::max(16, 16 * sm_count() / V)) : full, V);
   k_p3_gen_march<<<grid, 256, 0, s>>>(vol, proj, g->views, S, NJ, NK, R, C, plan, skip);
   return launch_check("k_p3_gen_march");
 }
@@ -1395,7 +1413,7 @@ ct_status ct_proj3d_window_views(const float* views, int32_t n_views, const int3
   if (n_views <= 0) return ct::fail(CT_ERR_SHAPE, "ct_proj3d_window_views: n_views=%d", n_views);
   for (int q = 0; q < 3; ++q)
     if (shape[q] <= 0) return ct::fail(CT_ERR_SHAPE, "ct_proj3d_window_views: shape[%d]=%d", q, shape[q]);
-  const int nwin = ct::gen_windows_bound(shape);
+  const int nwin = ct::gen_tiles(shape, n_views).nwin;
   for (int v = 0; v < n_views; ++v) {
     const float* m = views + (size_t)v * CT_VIEW3D_STRIDE;
     if (!(m[8] == 0.0f || m[8] == 1.0f || m[8] == 2.0f))
@@ -1433,8 +1451,11 @@ ct_status ct_proj3d_fwd(const ct_geom3d* g, const float* vol, float* proj, int32
       fewer.ns = p.nsplit;
       p = proj3d_plan_sched(g, fewer);
     }
-  } else if (workspace_bytes < p.fwd_bytes || !aligned(workspace, 256))
+  } else if (workspace_bytes < p.fwd_bytes - p.gen_turn || !aligned(workspace, 256)) {
     workspace = nullptr;  // GENERAL runs without scratch, slower
+  } else if (workspace_bytes < p.fwd_bytes) {
+    p.gen_turn = 0;  // views that march along axis 2 without their copy of the volume, slower
+  }
   if (st != CT_OK) return st;
   st = proj3d_prepare(g, p);
   if (st != CT_OK) return st;

@@ -242,10 +242,10 @@ __host__ __device__ inline int gen_lattice(const GenView& g, int k) {
 }
 
 // By all 32 lanes of one warp; valid in every lane.
-__device__ GenView gen_view(const float* __restrict__ m, int n0, int n1, int n2, int nwin) {
+__device__ GenView gen_view(const float* __restrict__ m, int n0, int n1, int n2, int nwin, bool turned) {
   const int lane = threadIdx.x & 31;
   GenView g;
-  bool ok = gen_view_base(g, m, n0, n1, n2, nwin);
+  bool ok = gen_view_base(g, m, n0, n1, n2, nwin) && (turned || g.ax != 2);
   if (ok) {  // the same in every lane
     bool fits = true;
     for (int ia = lane; ia < g.na; ia += 32) fits = fits && gen_plane_fits(g, ia);
@@ -306,8 +306,9 @@ struct GenFwdArgs {
 };
 
 // What a forward needs before its windows: the views' plans (the first
-// ceil(V / 8) blocks, a warp per view) and the volume with axis 2 outermost,
-// out[k][r] = in[r][k] (rows = n0 n1), a 32 x 32 piece per further block.
+// ceil(V / 8) blocks, a warp per view) and, where a view marches along axis 2, the
+// volume with that axis outermost, out[k][r] = in[r][k] (rows = n0 n1), a 32 x 32
+// piece per further block.  out null: no copy, and no windows for those views.
 __global__ void __launch_bounds__(256) k_p3_gen_setup(const float* __restrict__ views, GenView* __restrict__ plan,
                                                       const float* __restrict__ in, float* __restrict__ out, int n0,
                                                       int n1, int n2, int V, int nwin, const double* skip) {
@@ -316,10 +317,13 @@ __global__ void __launch_bounds__(256) k_p3_gen_setup(const float* __restrict__ 
   if (blockIdx.x < plan_blocks) {
     const int v = blockIdx.x * 8 + (threadIdx.x >> 5);
     if (v >= V) return;
-    const GenView g = gen_view(views + (size_t)v * kVT, n0, n1, n2, nwin);
+    const GenView g = gen_view(views + (size_t)v * kVT, n0, n1, n2, nwin, out != nullptr);
     if ((threadIdx.x & 31) == 0) plan[v] = g;
     return;
   }
+  int along = 0;
+  for (int v = threadIdx.x; v < V; v += 256) along |= views[(size_t)v * kVT + 8] == 2.0f;
+  if (!__syncthreads_or(along)) return;
   __shared__ float t[32][33];
   const int rows = n0 * n1;
   const unsigned piece = blockIdx.x - plan_blocks, nk = (n2 + 31) / 32, br = piece / nk, bk = piece - br * nk;

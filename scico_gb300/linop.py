@@ -621,6 +621,10 @@ class XRayTransform3D(LinearOperator):
         self._dev_tables = None
         self._geom = None
         self._ws_bytes: dict = {}
+        # what a general forward's scratch is for: views by windows, and of those any along axis 2
+        self._window_views = (False, False)
+        if self.kind == "general":
+            self._window_views = (self._any_windows(), bool((self.view_table[:, 8] == 2).any()))
         super().__init__(
             input_shape=self.input_shape,
             input_dtype=np.float32,
@@ -663,6 +667,35 @@ class XRayTransform3D(LinearOperator):
             got = self._ws_bytes[key] = (int(fwd.value), int(adj.value))
         return got
 
+    def _any_windows(self) -> bool:
+        """Whether the general forward's windows take any view (most often the first)."""
+        shape = np.asarray(self.input_shape, dtype=np.int32)
+        taken = np.zeros(len(self.matrices), dtype=np.int32)
+        for a, b in ((0, 1), (1, len(taken))):
+            if b > a:
+                _lib.call("ct_proj3d_window_views", self.view_table[a:].ctypes.data, b - a, shape.ctypes.data,
+                          taken[a:].ctypes.data)
+            if taken.any():
+                return True
+        return False
+
+    def _fwd_scratch(self, batch: int) -> Optional[torch.Tensor]:
+        """Scratch of :meth:`project`: for a general geometry only what its views use
+        (the copy of the volume serves views that march along axis 2, nothing serves
+        views that no window takes), and none where that much memory is not free."""
+        nbytes, _ = self.workspace_bytes(batch)
+        if self.kind != "general":
+            return _device.workspace(nbytes)
+        windows, along2 = self._window_views
+        if not windows or nbytes == 0:
+            return None
+        if not along2:
+            nbytes -= -(-4 * math.prod(self.input_shape) // 256) * 256
+        try:
+            return _device.workspace(nbytes)
+        except torch.cuda.OutOfMemoryError:
+            return None
+
     def autotune(self, reps: int = 5) -> dict:
         """Measure the 3D projector's launch schedules for this geometry
         (AXIS0 forward tile groups, adjoint view splits) and record the
@@ -701,10 +734,9 @@ class XRayTransform3D(LinearOperator):
         t, batch, has_batch = self._batched(im, self.input_shape, "volume")
         g = self.geometry()
         out = _device.empty(((batch,) if has_batch else ()) + self.output_shape)
-        fwd_bytes, _ = self.workspace_bytes(batch)
-        ws = _device.workspace(fwd_bytes)
+        ws = self._fwd_scratch(batch)
         _lib.call("ct_proj3d_fwd", _lib.ctypes.addressof(g), t.data_ptr(), out.data_ptr(), batch,
-                  ws.data_ptr(), ws.numel(), _device.stream())
+                  ws.data_ptr() if ws is not None else None, ws.numel() if ws is not None else 0, _device.stream())
         return out
 
     def back_project(self, proj) -> torch.Tensor:
