@@ -182,12 +182,13 @@ typedef struct ct_proj2d_schedule {
 } ct_proj2d_schedule;
 
 /*
- * Autotuner: times the forward for each candidate views-per-CTA and the
- * adjoint (with its split sum) for the split counts 1, 2, 4, 8, ... on
- * `stream` with CUDA events (one untimed call, then `reps` timed calls
- * each), and records the fastest forward and, among adjoint timings within
- * 3 % of the fastest, the fewest splits (so the choice, which sets the
- * adjoint's summation order, does not flip between runs on noise) in a
+ * Autotuner: times the forward for the planner's runs of views and each candidate
+ * views-per-CTA and the adjoint (with its split sum) for the split counts 1, 2, 4,
+ * 8, ... and the planner's own on `stream` with CUDA events (one untimed call, then
+ * `reps` timed calls each), and records the fastest forward and, among adjoint
+ * timings of the former counts within 3 % of the fastest, the fewest splits (so
+ * the choice, which sets the adjoint's summation order, does not flip between runs
+ * on noise), or the planner's count where that is faster by more than 10 %, in a
  * process-wide table (guarded by a mutex) keyed by the geometry's sizes and
  * batch.  Every later call on that
  * geometry (ct_proj2d_fwd/adj, the fused solvers) uses the recorded
@@ -329,10 +330,11 @@ typedef struct ct_proj3d_schedule {
 /*
  * Autotuner of the 3D projector: times the AXIS0 forward for tile-group
  * counts 1..8 (GENERAL geometries have no forward schedule) and the adjoint
- * with its split sum for 1, 2 and 4 view splits, on `stream` with CUDA
- * events (one untimed call, then `reps` timed ones each), and records the
- * fastest forward and, among adjoint timings within 3 % of the fastest, the
- * fewest splits, in a process-wide table (mutex-guarded) keyed by the
+ * with its split sum for 1, 2 and 4 view splits and the planner's own count, on
+ * `stream` with CUDA events (one untimed call, then `reps` timed ones each), and
+ * records the fastest forward and, among adjoint timings of 1, 2 and 4 within 3 %
+ * of the fastest, the fewest splits, or the planner's count where that is faster by
+ * more than 10 %, in a process-wide table (mutex-guarded) keyed by the
  * geometry's sizes and kind.  Later calls on that geometry (ct_proj3d_fwd /
  * adj, the fused 3D solver) use the recorded schedule; results change only
  * in summation order.  `vol` and `proj` are scratch arrays of the

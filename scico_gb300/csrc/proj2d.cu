@@ -1282,8 +1282,8 @@ ct_status ct_proj2d_autotune(const ct_geom2d* g, int32_t batch, float* img, floa
   if (st != CT_OK) return st;
   float* ws = static_cast<float*>(workspace);
 
-  // forward: views per CTA
-  static const int kVpcCand[] = {2, 3, 4, 5, 6, 7, 8, 10, 12, 16};
+  // forward: views per CTA, the planner's own runs (0) and single lengths; the results do not depend on it
+  static const int kVpcCand[] = {0, 2, 3, 4, 5, 6, 7, 8, 10, 12, 16};
   ct::Sched2d best;
   float best_f = 0.0f;
   for (int vpc : kVpcCand) {
@@ -1292,21 +1292,25 @@ ct_status ct_proj2d_autotune(const ct_geom2d* g, int32_t batch, float* img, floa
     float us = 0.0f;
     st = time_calls([&] { return ct::proj2d_fwd_launch(g, p, img, sino, batch, ws, s, nullptr); }, reps, s, us);
     if (st != CT_OK) return st;
-    if (best.vpc == 0 || us < best_f) {
-      best.vpc = p.vpc;
+    if (vpc == 0 || us < best_f) {
+      best.vpc = vpc;
       best_f = us;
     }
   }
-  // adjoint: view splits (the split sum included, as ct_proj2d_adj runs it)
+  // adjoint: 1, 2, 4, 8, .. view splits and the planner's own count (the split sum
+  // included, as ct_proj2d_adj runs it)
   const long ctas = (long)p0.adj_gx * p0.adj_gy * batch;
   const int ns_max = ct::max_splits(g, ctas);
   const size_t n = (size_t)batch * g->rows * g->cols;
-  // Split counts 1, 2, 4, 8, ...: neighbours far enough apart in time that
-  // the choice does not flip between runs on noise (the split count sets the
-  // adjoint's summation order, and with it the rounding a caller sees).
-  // Timings within kTie of the fastest count as ties and go to the fewest
-  // splits (less split memory).
-  constexpr float kTie = 1.03f;
+  auto time_adj = [&](const ct::Proj2dPlan& p, float& us) {
+    return time_calls(
+        [&] {
+          ct_status r = ct::proj2d_adj_launch(g, p, sino, img, ws, batch, s, nullptr);
+          if (r != CT_OK || p.nsplit == 1) return r;
+          return ct::proj2d_sum_splits(ws, img, n, p.nsplit, s);
+        },
+        reps, s, us);
+  };
   std::vector<std::pair<int, float>> cand;
   int last = 0;
   for (int ns = 1; ns <= ns_max; ns *= 2) {
@@ -1314,33 +1318,22 @@ ct_status ct_proj2d_autotune(const ct_geom2d* g, int32_t batch, float* img, floa
     if (p.nsplit == last) continue;  // same split count as the previous candidate
     last = p.nsplit;
     float us = 0.0f;
-    st = time_calls(
-        [&] {
-          ct_status r = ct::proj2d_adj_launch(g, p, sino, img, ws, batch, s, nullptr);
-          if (r != CT_OK || p.nsplit == 1) return r;
-          return ct::proj2d_sum_splits(ws, img, n, p.nsplit, s);
-        },
-        reps, s, us);
+    st = time_adj(p, us);
     if (st != CT_OK) return st;
     cand.emplace_back(p.nsplit, us);
   }
-  float fastest = cand.front().second;
-  for (const auto& c : cand) fastest = std::min(fastest, c.second);
-  float best_a = 0.0f;
-  for (const auto& c : cand) {
-    if (c.second <= kTie * fastest) {
-      best.ns = c.first;
-      best_a = c.second;
-      break;
-    }
-  }
+  float own = 0.0f, best_a = 0.0f;
+  st = time_adj(p0, own);
+  if (st != CT_OK) return st;
+  best.ns = ct::tuned_splits(cand, own, best_a);
   {
     std::lock_guard<std::mutex> lk(ct::g_sched_mu);
     ct::g_sched[ct::sched_key(g, batch)] = ct::SchedVal{best, best_f, best_a};
   }
   if (chosen) {
-    chosen->views_per_cta = best.vpc;
-    chosen->adj_splits = best.ns;
+    const ct::Proj2dPlan p = ct::proj2d_plan_sched(g, batch, best);
+    chosen->views_per_cta = p.vpc;
+    chosen->adj_splits = p.nsplit;
     chosen->fwd_us = best_f;
     chosen->adj_us = best_a;
     chosen->tuned = 1;

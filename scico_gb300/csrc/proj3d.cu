@@ -1572,6 +1572,16 @@ ct_status ct_proj3d_autotune(const ct_geom3d* g, float* vol, float* proj, void* 
     pick(cand, best.G, best_f);
   }
   {
+    // 1, 2 and 4 view splits and the planner's own count
+    auto time_adj = [&](const Proj3dPlan& p, float& us) {
+      return timed(
+          [&] {
+            ct_status r = proj3d_adj_launch(g, p, proj, vol, part, s, nullptr);
+            if (r != CT_OK || p.nsplit == 1) return r;
+            return sum_splits(part, vol, vol_n, p.nsplit, s);
+          },
+          us);
+    };
     std::vector<std::pair<int, float>> cand;
     int last = 0;
     for (int ns = 1; ns <= kMaxSplits3d; ns *= 2) {
@@ -1579,17 +1589,14 @@ ct_status ct_proj3d_autotune(const ct_geom3d* g, float* vol, float* proj, void* 
       if (p.nsplit == last) continue;
       last = p.nsplit;
       float us = 0.0f;
-      st = timed(
-          [&] {
-            ct_status r = proj3d_adj_launch(g, p, proj, vol, part, s, nullptr);
-            if (r != CT_OK || p.nsplit == 1) return r;
-            return sum_splits(part, vol, vol_n, p.nsplit, s);
-          },
-          us);
+      st = time_adj(p, us);
       if (st != CT_OK) return st;
       cand.emplace_back(p.nsplit, us);
     }
-    pick(cand, best.ns, best_a);
+    float own = INFINITY;  // where the scratch given does not hold the planner's count, it is not a choice
+    if (workspace_bytes >= p0.adj_bytes) st = time_adj(p0, own);
+    if (st != CT_OK) return st;
+    best.ns = tuned_splits(cand, own, best_a);
   }
   {
     std::lock_guard<std::mutex> lk(g_sched3_mu);

@@ -1,0 +1,61 @@
+"""The autotuners leave no geometry slower than its untuned plan where the
+planner's own split count lies between the tuners' counts: sizes at which the
+best of 1, 2, 4, .. splits is 20 to 40 % slower.  Timed as replayed graphs, the
+fastest of several; the tuners' rule allows 10 %, the timing 5 % more."""
+
+import numpy as np
+import pytest
+import torch
+
+from scico_gb300 import _lib, linop
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(autouse=True)
+def clear_schedules():
+    for clear in (_lib.load().ct_proj2d_schedule_clear, _lib.load().ct_proj3d_schedule_clear):
+        clear()
+    yield
+    for clear in (_lib.load().ct_proj2d_schedule_clear, _lib.load().ct_proj3d_schedule_clear):
+        clear()
+
+
+def _us(fn):
+    fn()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        for _ in range(20):
+            fn()
+    best = float("inf")
+    for _ in range(8):
+        a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        a.record()
+        graph.replay()
+        b.record()
+        b.synchronize()
+        best = min(best, a.elapsed_time(b) * 50.0)
+    return best
+
+
+def _op2(n, nv):
+    return linop.XRayTransform2D((n, n), np.linspace(0, np.pi, nv, endpoint=False))
+
+
+def _op3(shape, nv):
+    det = (shape[0], int(np.hypot(*shape[1:])) + 1)
+    M = linop.XRayTransform3D.matrices_from_euler_angles(shape, det, "X", np.linspace(0, np.pi, nv, endpoint=False)[:, None])
+    return linop.XRayTransform3D(shape, M, det)
+
+
+@pytest.mark.parametrize("make,args", [(_op2, (96, 50)), (_op3, ((64, 64, 64), 90)), (_op3, ((48, 60, 70), 120))],
+                         ids=["2d-96", "3d-64", "3d-48x60x70"])
+def test_tuned_is_not_slower_than_untuned(cuda, make, args):
+    H = make(*args)
+    x, y = torch.rand(H.input_shape, device=cuda), torch.rand(H.output_shape, device=cuda)
+    fwd, adj = _us(lambda: H.project(x)), _us(lambda: H.back_project(y))
+    H.autotune()
+    assert H.schedule()["tuned"]
+    assert _us(lambda: H.project(x)) <= 1.15 * fwd
+    assert _us(lambda: H.back_project(y)) <= 1.15 * adj
