@@ -35,7 +35,6 @@
 #include <algorithm>
 #include <atomic>
 #include <cmath>
-#include <cstdlib>
 #include <map>
 #include <mutex>
 #include <tuple>
@@ -55,8 +54,8 @@ constexpr int kWalkGroup = 4;   // walk entries tested together for a new bin
 
 static_assert(kTileJ * kTileK == kOrd, "order table covers one tile");
 
-// Device error word of the 3D kernels' internal checks (bit 0: forward
-// accumulator span, bit 1: adjoint window span).
+// Device error word of the 3D kernels' internal checks (bit 0: forward tile
+// span, bit 1: adjoint window span).
 __device__ int g_proj3d_err = 0;
 
 int* errflag3_ptr() {
@@ -120,10 +119,11 @@ struct Ax0FwdArgs {
   const uint16_t* order;
   int S, NJ, NK, V, C, Spad;
   int tiles_k, n_tiles, G;
+  int* errflag;
   const double* skip;  // device flag: return at once when non-zero (may be null)
 };
 
-// Bin range of one 16x32 tile for one view.  Every operation of the rounded
+// Bin range of one 16x16 tile for one view.  Every operation of the rounded
 // Px is monotone in each pixel index, so the tile's extremes are at corner
 // pixels; floor(left) of those, widened by one bin below and two above
 // (room for the second tap and the carried bin), gives [lo, hi).
@@ -307,7 +307,7 @@ __global__ void __launch_bounds__(NW * 32, SL == 4 ? 1 : 2) k_p3_ax0_fwd(const A
   __shared__ int2 tlist[256];                                     // tile origins (j0, k0)
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int g = blockIdx.x, i0 = blockIdx.y * 32 * SL, v = blockIdx.z * NW + warp;
-  const bool live = v < a.V;  // warp-uniform
+  bool live = v < a.V;  // warp-uniform
   float2* tabw = tab + warp * kOrd;
   unsigned char* binw = bins + warp * kOrd;
   const uint32_t sv_s = (uint32_t)__cvta_generic_to_shared(sv);
@@ -330,6 +330,12 @@ __global__ void __launch_bounds__(NW * 32, SL == 4 ? 1 : 2) k_p3_ax0_fwd(const A
     const uint16_t* q = a.order + (size_t)v * kOrd;
 #pragma unroll
     for (int u = 0; u < kOrd / 64; ++u) ord[u] = __ldg(q + 64 * u + lane) | (unsigned)__ldg(q + 64 * u + 32 + lane) << 16;
+    // a tile's bins are kept in 8 bits (at most 36 for |m| <= 1, which ct_proj3d_views
+    // sees to); a view of another table that needs more is left out: zeros
+    if (!(15.0f * (fabsf(m11) + fabsf(m12)) <= 250.0f)) {
+      if (lane == 0) atomicOr(a.errflag, 1);
+      live = false;
+    }
   }
 
   const int per = (a.n_tiles + a.G - 1) / a.G, nrun = min(per, a.n_tiles - g * per);
@@ -1240,6 +1246,7 @@ ct_status proj3d_fwd_launch(const ct_geom3d* g, const Proj3dPlan& p, const float
     a.tiles_k = p.tiles_k;
     a.n_tiles = p.n_tiles;
     a.G = p.G;
+    a.errflag = errflag3_ptr();
     a.skip = skip;
     with_fwd(p, [&](auto* kernel, size_t bytes, int slices) {
       const dim3 grid(p.G, (S + slices - 1) / slices, (V + p.fwd_nw - 1) / p.fwd_nw);
