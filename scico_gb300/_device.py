@@ -18,6 +18,13 @@ _reduce_ws: dict[tuple[int, int], torch.Tensor] = {}
 _devices: dict[int, torch.device] = {}
 
 
+# The device index and the raw stream handle without the objects around them, which
+# cost more than a small projection's launches; torch's public calls where a release
+# does not have these names.
+_device_index = getattr(torch._C, "_cuda_getDevice", None) or torch.cuda.current_device
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+
+
 def require_cuda() -> torch.device:
     """Return the current CUDA device; raise if there is none (no CPU path)."""
     if not _devices:
@@ -27,7 +34,7 @@ def require_cuda() -> torch.device:
                 "there is no CPU fallback"
             )
         torch.cuda.current_device()  # initialises CUDA
-    index = torch._C._cuda_getDevice()
+    index = _device_index()
     dev = _devices.get(index)
     if dev is None:
         dev = _devices[index] = torch.device("cuda", index)
@@ -36,7 +43,8 @@ def require_cuda() -> torch.device:
 
 def stream() -> int:
     """Handle of the current torch CUDA stream (passed to the C ABI)."""
-    return torch._C._cuda_getCurrentRawStream(require_cuda().index)
+    index = require_cuda().index
+    return torch.cuda.current_stream(index).cuda_stream if _raw_stream is None else _raw_stream(index)
 
 
 def to_device(x, shape=None, name: str = "array") -> torch.Tensor:
