@@ -1579,7 +1579,9 @@ ct_status ct_proj3d_autotune(const ct_geom3d* g, float* vol, float* proj, void* 
     pick(cand, best.G, best_f);
   }
   {
-    // 1, 2 and 4 view splits and the planner's own count
+    // 1, 2 and 4 view splits and the planner's own count, of those what the scratch
+    // given holds (a call may always have had less than the counts of now need)
+    const size_t scratch = workspace && aligned(workspace, 256) ? workspace_bytes : 0;
     auto time_adj = [&](const Proj3dPlan& p, float& us) {
       return timed(
           [&] {
@@ -1593,15 +1595,15 @@ ct_status ct_proj3d_autotune(const ct_geom3d* g, float* vol, float* proj, void* 
     int last = 0;
     for (int ns = 1; ns <= kMaxSplits3d; ns *= 2) {
       const Proj3dPlan p = proj3d_plan_sched(g, Sched3d{0, ns});
-      if (p.nsplit == last) continue;
+      if (p.nsplit == last || p.adj_bytes > scratch) continue;
       last = p.nsplit;
       float us = 0.0f;
       st = time_adj(p, us);
       if (st != CT_OK) return st;
       cand.emplace_back(p.nsplit, us);
     }
-    float own = INFINITY;  // where the scratch given does not hold the planner's count, it is not a choice
-    if (workspace_bytes >= p0.adj_bytes) st = time_adj(p0, own);
+    float own = INFINITY;
+    if (p0.adj_bytes <= scratch) st = time_adj(p0, own);
     if (st != CT_OK) return st;
     best.ns = tuned_splits(cand, own, best_a);
   }
