@@ -92,6 +92,7 @@ struct Proj3dPlan {
   // adjoint view splits (both kinds)
   int nsplit = 1, per_split = 0;
   int adj_sl = 4;        // AXIS0 adjoint: slices a lane
+  bool adj_voxels = false;  // GENERAL adjoint: a voxel per thread
   size_t adj_least = 0, adj_tune = 0;  // scratch below which an adjoint / its tuning is refused
   size_t fwd_bytes = 0, adj_bytes = 0;
   size_t fwd_least = 0;  // AXIS0: forward scratch below which a call is refused

@@ -1095,23 +1095,38 @@ Proj3dPlan proj3d_plan_sched(const ct_geom3d* g, Sched3d sc) {
     least_scratch(old_ns, std::min(kMaxSplits3d, ns_max));
     ns_max = most;
   } else {
-    // adjoint: the view splits (up to 16, each costs a pass over its partial
-    // volume) with the fewest rounds of the SMs' three CTAs per view
-    const long ctas = (long)((S + kBrick - 1) / kBrick) * ((NJ + kBrick - 1) / kBrick) * ((NK + kBrick - 1) / kBrick);
-    double least = 1e300;
-    for (int k = 1; k <= 16; ++k) {
-      const double cost = std::ceil((double)ctas * k / (3.0 * sms)) / k * (1.0 + 0.02 * (k - 1));
-      if (cost < 0.98 * least) {
-        least = cost;
-        ns = k;
-      }
-    }
     ns_max = std::max(1, V / 8);
     // the scratch that a call has always needed (a voxel per thread, four CTAs
     // of 256 an SM); one with no more runs the splits that fit (ct_proj3d_adj)
     const long old_ctas = (long)(((double)S * NJ * NK + 255) / 256);
     const int old_ns = std::min(old_ctas < 4L * sms ? (int)((4L * sms + old_ctas - 1) / old_ctas) : 1, ns_max);
     least_scratch(old_ns, std::min(kMaxSplits3d, ns_max));
+    // Bricks, or a voxel per thread where there are too few bricks to keep the SMs
+    // busy, and the view splits, by the us of the busiest SM: a view costs a brick
+    // 1.2, each further brick beside it (three an SM) 0.55; a voxel's chain 0.28 a view, or
+    // the rate of 4e-6 a voxel and view; splits a pass over the partial volumes.  Within
+    // 10 % of the best measured choice for volumes of 8^3 to 128^3 with 3 to 180
+    // views (16^3, 6 views: 9.6 us in bricks, 2.5 us by voxels; 40^3, 20 views 15.9 and 8.5;
+    // 64^3, 20 views 13.6 and 24.0; 4 x 256 x 256, 8 views 17.2 and 11.7).  Bricks need
+    // a lead: voxels of more than a pixel, which only the device sees, cost them up
+    // to three times as much.
+    ns_max = std::max(1, V / 2);
+    const double voxels = (double)S * NJ * NK;
+    const long bricks = (long)((S + kBrick - 1) / kBrick) * ((NJ + kBrick - 1) / kBrick) * ((NK + kBrick - 1) / kBrick);
+    auto split_us = [&](int k) { return k > 1 ? 2.0 + 7e-7 * voxels * (k + 1) : 0.0; };
+    auto brick_us = [&](int k) {
+      const long c = (bricks * k + sms - 1) / sms, part = c % 3;
+      return ((V + k - 1) / k) * ((c / 3) * 2.3 + (part ? 0.65 + 0.55 * part : 0.0)) + split_us(k);
+    };
+    auto voxel_us = [&](int k) { return std::max(0.28 * ((V + k - 1) / k), 4e-6 * voxels * V) + split_us(k); };
+    int nb = 1, nv = old_ns;  // a voxel per thread: no fewer splits than a call has always had
+    for (int k = 2; k <= std::min(16, ns_max); ++k)
+      if (brick_us(k) < 0.98 * brick_us(nb)) nb = k;
+    for (int k = old_ns + 1; k <= std::min(16, V / 4); ++k)
+      if (voxel_us(k) < 0.98 * voxel_us(nv)) nv = k;
+    if (sc.ns > 0) nb = nv = std::min(sc.ns, ns_max);
+    p.adj_voxels = voxel_us(nv) < 1.25 * brick_us(nb);
+    ns = p.adj_voxels ? nv : nb;
     // forward: views per launch until the tiles of a launch pass kGenScratch (they
     // are read back from L2); the turned volume last, so that a call can go without it
     const GenTiles t = gen_tiles(g->shape, V);
@@ -1331,6 +1346,11 @@ ct_status proj3d_adj_launch(const ct_geom3d* g, const Proj3dPlan& p, const float
     else
       k_p3_ax0_adj<1><<<grid, kAdjWarps * 32, adj3_smem(1), s>>>(a);
     return launch_check("k_p3_ax0_adj");
+  }
+  if (p.adj_voxels) {
+    k_p3_gen_adj_voxels<<<dim3((unsigned)((vol_n + 255) / 256), p.nsplit), 256, 0, s>>>(
+        proj, dst, g->views, S, NJ, NK, V, R, C, p.per_split, vol_n, skip);
+    return launch_check("k_p3_gen_adj_voxels");
   }
   const dim3 grid((unsigned)((NK + kBrick - 1) / kBrick) * ((NJ + kBrick - 1) / kBrick) * ((S + kBrick - 1) / kBrick), p.nsplit);
   k_p3_gen_adj<<<grid, 256, 0, s>>>(proj, dst, g->views, S, NJ, NK, V, R, C, p.per_split, vol_n,
