@@ -78,7 +78,7 @@ ct_status make_fd(const ct_fd_desc* d, FdParams& p, const char* who) {
 // offset to the neighbour and the test for the line's end, is the same for
 // the whole warp and costs nothing per element.  Shorter ones (k_fd_*_flat) would
 // leave lanes idle: there a thread takes kFdU elements of the flat array
-// kFdT apart.  A copied end's second term is behind a branch that few threads
+// kFdT apart, or one (one_each: 17 x 19 x 23 2.9 / 3.9 -> 1.9 / 2.1 us).  A copied end's second term is behind a branch that few threads
 // take: as a select it cost the adjoint more than its loads (192^3 in quads 22.3 us).
 // 192^3, three axes (forward / adjoint): 177 / 150 us with the divisions of
 // k_fd_fwd / k_fd_adj, 43 / 62 us flat, 18.8 / 27.7 us by rows, 17.4 / 19.9 us
@@ -87,6 +87,10 @@ ct_status make_fd(const ct_fd_desc* d, FdParams& p, const char* who) {
 // ---------------------------------------------------------------------------
 constexpr int kFdT = 256;  // threads of a block
 constexpr int kFdU = 4;    // elements per thread
+
+// One element a thread where the SMs hold a thread for each (eight CTAs of 256 an
+// SM): there a thread's second element only lengthens the launch.
+bool one_each(size_t n) { return n <= (size_t)ct::sm_count() * 8 * 256; }
 
 // Division of 31-bit unsigned numbers by a fixed divisor: q = (mulhi(e, m) + e) >> s.
 struct FastDiv {
@@ -157,14 +161,14 @@ __device__ __forceinline__ void fd_coords(const FdSame& q, uint32_t e, int (&c)[
 
 // out[k][e] = (next) - (this) along axis k, next the circular neighbour or the
 // extended sample at the end (append), or (this) - (previous) (prepend).
-template <int NB>
+template <int NB, int U>
 __global__ void __launch_bounds__(kFdT) k_fd_fwd_flat(const float* __restrict__ x, float* __restrict__ out, const FdSame q) {
   x += (size_t)blockIdx.y * q.count;
   out += (size_t)blockIdx.y * NB * q.count;
-  const uint32_t e0 = blockIdx.x * (uint32_t)(kFdT * kFdU) + threadIdx.x;
-  float xc[kFdU], xn[kFdU][NB];
+  const uint32_t e0 = blockIdx.x * (uint32_t)(kFdT * U) + threadIdx.x;
+  float xc[U], xn[U][NB];
 #pragma unroll
-  for (int u = 0; u < kFdU; ++u) {
+  for (int u = 0; u < U; ++u) {
     const uint32_t e = min(e0 + u * kFdT, q.count - 1);  // loads stay unconditional, all in flight
     int c[3];
     fd_coords(q, e, c);
@@ -181,7 +185,7 @@ __global__ void __launch_bounds__(kFdT) k_fd_fwd_flat(const float* __restrict__ 
     }
   }
 #pragma unroll
-  for (int u = 0; u < kFdU; ++u) {
+  for (int u = 0; u < U; ++u) {
     const uint32_t e = e0 + u * kFdT;
     if (e >= q.count) break;
 #pragma unroll
@@ -194,15 +198,15 @@ __global__ void __launch_bounds__(kFdT) k_fd_fwd_flat(const float* __restrict__ 
 // ce[t] = d[t-1] - d[t] (terms off the line are 0) at the positions holding
 // x[e]; an end copied by the extension holds two, added in position order
 // (k_fd_adj below states the rule in general).
-template <int NB>
+template <int NB, int U>
 __global__ void __launch_bounds__(kFdT) k_fd_adj_flat(const float* __restrict__ d, float* __restrict__ x, const FdSame q) {
   d += (size_t)blockIdx.y * NB * q.count;
   x += (size_t)blockIdx.y * q.count;
-  const uint32_t e0 = blockIdx.x * (uint32_t)(kFdT * kFdU) + threadIdx.x;
-  float dc[kFdU][NB], dn[kFdU][NB];
+  const uint32_t e0 = blockIdx.x * (uint32_t)(kFdT * U) + threadIdx.x;
+  float dc[U][NB], dn[U][NB];
   unsigned two = 0;  // bit u*NB + k: the sample is a copied end
 #pragma unroll
-  for (int u = 0; u < kFdU; ++u) {
+  for (int u = 0; u < U; ++u) {
     const uint32_t e = min(e0 + u * kFdT, q.count - 1);  // loads stay unconditional, all in flight
     int c[3];
     fd_coords(q, e, c);
@@ -223,7 +227,7 @@ __global__ void __launch_bounds__(kFdT) k_fd_adj_flat(const float* __restrict__ 
     }
   }
 #pragma unroll
-  for (int u = 0; u < kFdU; ++u) {
+  for (int u = 0; u < U; ++u) {
     const uint32_t e = e0 + u * kFdT;
     if (e >= q.count) break;
     float acc = 0.0f;
@@ -519,11 +523,15 @@ ct_status fd_same_launch(const float* src, float* dst, const FdSame& q, int batc
     }
     return ct::launch_check("k_fd_rows");
   }
-  const dim3 g((q.count + kFdT * kFdU - 1) / (kFdT * kFdU), batch);
-  if (ADJ)
-    k_fd_adj_flat<NB><<<g, kFdT, 0, s>>>(src, dst, q);
-  else
-    k_fd_fwd_flat<NB><<<g, kFdT, 0, s>>>(src, dst, q);
+  const int u = one_each(q.count) ? 1 : kFdU;
+  const dim3 g((q.count + kFdT * u - 1) / (kFdT * u), batch);
+  if constexpr (ADJ) {
+    auto f = u == 1 ? k_fd_adj_flat<NB, 1> : k_fd_adj_flat<NB, kFdU>;
+    f<<<g, kFdT, 0, s>>>(src, dst, q);
+  } else {
+    auto f = u == 1 ? k_fd_fwd_flat<NB, 1> : k_fd_fwd_flat<NB, kFdU>;
+    f<<<g, kFdT, 0, s>>>(src, dst, q);
+  }
   return ct::launch_check(ADJ ? "k_fd_adj_flat" : "k_fd_fwd_flat");
 }
 
@@ -712,22 +720,23 @@ __device__ __forceinline__ void l21_shrink(float (&v)[NC], float lam) {
 }
 
 // The prox of up to three components (every image gradient): the components
-// are read once and kept in registers, kPxU vectors in flight per thread.
-// 3 x 192^3: 43 -> 27.7 us, the time of a copy.
+// are read once and kept in registers, U vectors in flight per thread: kPxU, or one
+// (one_each).  3 x 192^3: 43 -> 27.7 us, the time of a copy; 3 x 64 x 64 x 3 2.5 us
+// before, 3.1 with four, 2.1 with one.
 constexpr int kPxU = 4;
-template <int NC>
+template <int NC, int U>
 __global__ void __launch_bounds__(256) k_l21_prox_few(const float* __restrict__ v, float* __restrict__ out, size_t n,
                                                       float lam) {
-  const size_t e0 = (size_t)blockIdx.x * (256 * kPxU) + threadIdx.x;
-  float r[kPxU][NC];
+  const size_t e0 = (size_t)blockIdx.x * (256 * U) + threadIdx.x;
+  float r[U][NC];
 #pragma unroll
-  for (int u = 0; u < kPxU; ++u) {
+  for (int u = 0; u < U; ++u) {
     const size_t e = min(e0 + u * 256, n - 1);
 #pragma unroll
     for (int c = 0; c < NC; ++c) r[u][c] = __ldg(v + (size_t)c * n + e);
   }
 #pragma unroll
-  for (int u = 0; u < kPxU; ++u)
+  for (int u = 0; u < U; ++u)
     if (e0 + u * 256 < n) {
       l21_shrink<NC>(r[u], lam);
 #pragma unroll
@@ -988,15 +997,18 @@ ct_status ct_l21_prox(const float* v, float* out, int32_t ncomp, int64_t n, floa
   if (ncomp < 1 || n < 0)
     return ct::fail(CT_ERR_INVALID_ARG, "ct_l21_prox: ncomp=%d n=%lld", ncomp, (long long)n);
   if (n == 0) return CT_OK;
-  const size_t blocks = ((size_t)n + 256 * kPxU - 1) / (256 * kPxU);
+  const int u = one_each((size_t)n) ? 1 : kPxU;
+  const size_t blocks = ((size_t)n + 256 * u - 1) / (256 * u);
   if (ncomp <= 3 && blocks < (1ull << 31)) {
-    cudaStream_t s = ct::as_stream(stream);
+    auto launch = [&](auto one, auto four) {
+      (u == 1 ? one : four)<<<(unsigned)blocks, 256, 0, ct::as_stream(stream)>>>(v, out, (size_t)n, lam);
+    };
     if (ncomp == 1)
-      k_l21_prox_few<1><<<(unsigned)blocks, 256, 0, s>>>(v, out, (size_t)n, lam);
+      launch(k_l21_prox_few<1, 1>, k_l21_prox_few<1, kPxU>);
     else if (ncomp == 2)
-      k_l21_prox_few<2><<<(unsigned)blocks, 256, 0, s>>>(v, out, (size_t)n, lam);
+      launch(k_l21_prox_few<2, 1>, k_l21_prox_few<2, kPxU>);
     else
-      k_l21_prox_few<3><<<(unsigned)blocks, 256, 0, s>>>(v, out, (size_t)n, lam);
+      launch(k_l21_prox_few<3, 1>, k_l21_prox_few<3, kPxU>);
     return ct::launch_check("k_l21_prox_few");
   }
   k_l21_prox<<<grid_for((size_t)n, 256), 256, 0, ct::as_stream(stream)>>>(v, out, ncomp,
