@@ -1125,10 +1125,22 @@ Proj3dPlan proj3d_plan_sched(const ct_geom3d* g, Sched3d sc) {
       return ((V + k - 1) / k) * ((c / 3) * 2.3 + (part ? 0.65 + 0.55 * part : 0.0)) + split_us(k);
     };
     auto voxel_us = [&](int k) { return std::max(0.28 * ((V + k - 1) / k), 4e-6 * voxels * V) + split_us(k); };
-    int nb = 1, nv = old_ns;  // a voxel per thread: no fewer splits than a call has always had
-    for (int k = 2; k <= std::min(16, ns_max); ++k)
+    // no fewer splits than fill the SMs' three CTAs or a call has always had, at eight
+    // views or more each, so that no sum gets longer
+    int first = 1;
+    double least = 1e300;
+    for (int k = 1; k <= 16; ++k) {
+      const double rounds = std::ceil((double)bricks * k / (3.0 * sms)) / k * (1.0 + 0.02 * (k - 1));
+      if (rounds < 0.98 * least) {
+        least = rounds;
+        first = k;
+      }
+    }
+    first = std::max(old_ns, std::min(first, std::max(1, V / 8)));
+    int nb = first, nv = first;
+    for (int k = first + 1; k <= std::min(16, ns_max); ++k)
       if (brick_us(k) < 0.98 * brick_us(nb)) nb = k;
-    for (int k = old_ns + 1; k <= std::min(16, V / 4); ++k)
+    for (int k = first + 1; k <= std::min(16, V / 4); ++k)
       if (voxel_us(k) < 0.98 * voxel_us(nv)) nv = k;
     if (sc.ns > 0) nb = nv = std::min(sc.ns, ns_max);
     p.adj_voxels = voxel_us(nv) < 1.25 * brick_us(nb);
