@@ -575,24 +575,42 @@ __global__ void __launch_bounds__(kGatherWarps * 32) k_p3_gen_gather(const GenFw
 // stride is 1 or 7 modulo 8 by the sign of the two steps along axis 2, so that
 // eight neighbouring lanes walk monotonically over the eight 16-byte bank
 // groups.  Views whose tile does not fit (voxels above ~1.3 detector pixels)
-// gather from global memory.  Bound by the FP32 pipe (some 23 operations a voxel
+// gather from global memory.  Bound by the FP32 pipe (some 25 operations a voxel
 // and view).  97 x 128 x 111 voxels, 60 views: one voxel a thread with four
 // scalar gathers 238 us; bricks with the four weights formed and four multiply-adds
-// into the sum 163 us; this 157 us, and a third of the error against 64 bits less
-// (1.8e-7 -> 1.2e-7).
+// into the sum 163 us; interpolated as here 157 us, with positions times two, whose
+// edges are the weights without a further step, 147 us, in three view splits 135 us; error
+// against 64 bits 1.8e-7 -> 5.9e-8.
 // ---------------------------------------------------------------------------
 constexpr int kBrick = 16;
 
 // A voxel's value between the columns (y[r][c], y[r+1][c]), (y[r][c+1], y[r+1][c+1])
-// and then the rows, with the weights 2 min(t, 0.5) and 1 less it of each axis's first
-// and second pixel.
-__device__ __forceinline__ float gen_interp(unsigned long long y0, unsigned long long y1, float t0, float t1) {
-  const float s0 = __saturatef(fadd(t0, t0)), s1 = __saturatef(fadd(t1, t1));
-  const float o0 = __saturatef(fmaf(-2.0f, t0, 1.0f)), o1 = __saturatef(fmaf(-2.0f, t1, 1.0f));
+// and then the rows: weights s of each axis's first pixel and 1 - s of its second.
+__device__ __forceinline__ float gen_interp(unsigned long long y0, unsigned long long y1, float s0, float s1) {
+  const float o0 = fsub(1.0f, s0), o1 = fsub(1.0f, s1);
   float r0, r1;
   g_upk(g_fma(y0, g_pk(s1, s1), g_mul(y1, g_pk(o1, o1))), r0, r1);
   return fmaf(r0, s0, fmul(r1, o0));
 }
+
+// First pixel and its weight 2 min(ceil(left) - left, 0.5) on both axes, from twice
+// the rounded position (from a matrix times two: the same roundings): adding 1.5 2^24
+// rounds to an even number, so the difference of the rounding up is the weight.
+constexpr float kGMagic2 = 25165824.0f;
+constexpr int kGMagic2Bits = 0x4BC00000;
+__device__ __forceinline__ void twice_edges(unsigned long long px2, int& u0, int& u1, float& s0, float& s1) {
+  const unsigned long long magic = g_pk(kGMagic2, kGMagic2);
+  const unsigned long long left2 = g_sub(px2, g_pk(0.5f, 0.5f));
+  float f0, f1, a0, a1, l0, l1;
+  g_upk(g_add_down(left2, magic), f0, f1);
+  g_upk(g_sub(g_add_up(left2, magic), magic), a0, a1);
+  g_upk(left2, l0, l1);
+  s0 = __saturatef(fsub(a0, l0));
+  s1 = __saturatef(fsub(a1, l1));
+  u0 = __float_as_int(f0);
+  u1 = __float_as_int(f1);
+}
+
 // The same of the view `y` in global memory, zero off the detector.
 __device__ __forceinline__ float gen_gathered(const float* __restrict__ y, int R, int C, int u0, int u1, float t0,
                                               float t1) {
@@ -602,14 +620,14 @@ __device__ __forceinline__ float gen_gathered(const float* __restrict__ y, int R
   const float y10 = r1 && c0 ? __ldg(y + (size_t)(u0 + 1) * C + u1) : 0.0f;
   const float y01 = r0 && c1 ? __ldg(y + (size_t)u0 * C + u1 + 1) : 0.0f;
   const float y11 = r1 && c1 ? __ldg(y + (size_t)(u0 + 1) * C + u1 + 1) : 0.0f;
-  return gen_interp(g_pk(y00, y10), g_pk(y01, y11), t0, t1);
+  return gen_interp(g_pk(y00, y10), g_pk(y01, y11), __saturatef(fadd(t0, t0)), __saturatef(fadd(t1, t1)));
 }
 
 constexpr int kAdjSlots = 1024;  // float4 slots of a staged tile
 constexpr int kAdjChunk = 32;    // views whose tiles are laid out at once
 
 struct GenAdjView {
-  float m[8];
+  float m[8];  // the matrix times two
   int base0, base1, T0, LD;
   int ok;      // the tile fits; 2: it lies inside the detector as well
   unsigned inv;  // e / LD = (e inv) >> 16 for e < kAdjSlots
@@ -676,7 +694,7 @@ __global__ void __launch_bounds__(256, 3) k_p3_gen_adj(const float* __restrict__
       GenAdjView& t = tv[tid];
       const float* m = views + (size_t)(vc + tid) * kVT;
 #pragma unroll
-      for (int q = 0; q < 8; ++q) t.m[q] = m[q];
+      for (int q = 0; q < 8; ++q) t.m[q] = 2.0f * m[q];
       float lo[2], ext[2], mag = 0.0f;
 #pragma unroll
       for (int r = 0; r < 2; ++r) {
@@ -716,7 +734,7 @@ __global__ void __launch_bounds__(256, 3) k_p3_gen_adj(const float* __restrict__
         const unsigned long long cc = g_pk(t.m[3], t.m[7]);
         const uint32_t ld16 = 16u * (uint32_t)t.LD;
         const uint32_t origin = (uint32_t)__cvta_generic_to_shared(&sy[vi & 1][0]) -
-                                ld16 * (uint32_t)(kGMagicBits + t.base0) - 16u * (uint32_t)(kGMagicBits + t.base1);
+                                ld16 * (uint32_t)(kGMagic2Bits + t.base0) - 16u * (uint32_t)(kGMagic2Bits + t.base1);
 #pragma unroll
         for (int k = 0; k < kBrick; k += 2) {
           float v[2];
@@ -725,11 +743,11 @@ __global__ void __launch_bounds__(256, 3) k_p3_gen_adj(const float* __restrict__
             const float x0 = (float)(b0 + k + h) + 0.5f;
             const unsigned long long A = g_pk(fmul(m0, x0), fmul(m4, x0));
             int u0, u1;
-            float t0, t1;
-            foot_edges(g_add(g_add(g_add(A, P), Q), cc), u0, u1, t0, t1);
+            float s0, s1;
+            twice_edges(g_add(g_add(g_add(A, P), Q), cc), u0, u1, s0, s1);
             unsigned long long y0, y1;
             lds_pairs(origin + ld16 * (uint32_t)u0 + 16u * (uint32_t)u1, y0, y1);
-            v[h] = gen_interp(y0, y1, t0, t1);
+            v[h] = gen_interp(y0, y1, s0, s1);
           }
           g_upk(g_add(g_pk(acc[k], acc[k + 1]), g_pk(v[0], v[1])), acc[k], acc[k + 1]);
         }
@@ -740,8 +758,8 @@ __global__ void __launch_bounds__(256, 3) k_p3_gen_adj(const float* __restrict__
           const float x0 = (float)(b0 + k) + 0.5f;
           int u0, u1;
           float t0, t1;
-          edge3(px3(m0, t.m[1], t.m[2], t.m[3], x0, x1, x2), u0, t0);
-          edge3(px3(m4, t.m[5], t.m[6], t.m[7], x0, x1, x2), u1, t1);
+          edge3(0.5f * px3(m0, t.m[1], t.m[2], t.m[3], x0, x1, x2), u0, t0);
+          edge3(0.5f * px3(m4, t.m[5], t.m[6], t.m[7], x0, x1, x2), u1, t1);
           acc[k] = fadd(acc[k], gen_gathered(y, R, C, u0, u1, t0, t1));
         }
       }
