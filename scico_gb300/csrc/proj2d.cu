@@ -960,7 +960,7 @@ Proj2dPlan proj2d_plan_sched(const ct_geom2d* g, int batch, Sched2d sc) {
   // at 8; 256^2 x 180: 14.9 us at 2, 13.9 us at 4).  A larger one takes long runs of
   // even length, which stage a strip seldom, and then about one round of CTAs with
   // runs a third as long, so that the SMs end together.  Against one length and
-  // about 1824 CTAs: 512^2 x 360 60.4 -> 58.7 us, 501^2 68.5 -> 64.0 us, 640^2 x 270
+  // about 1824 CTAs (the kernels back to back; a call's other 4 us stay): 512^2 x 360 60.4 -> 58.7 us, 501^2 68.5 -> 64.0 us, 640^2 x 270
   // 78.3 -> 72.8 us, 450^2 x 300 58.8 -> 52.7 us, 16 x 256^2 x 180 112.1 -> 109.5 us.
   // Runs of 12 under 20 rounds: 384^2 x 270 33.8 us (16: 34.0), 512^2 x 129 27.0 us
   // (28.9).  Images of at most two tile columns keep even runs: their CTAs, two busy

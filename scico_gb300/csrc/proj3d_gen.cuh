@@ -578,8 +578,8 @@ __global__ void __launch_bounds__(kGatherWarps * 32) k_p3_gen_gather(const GenFw
 // gather from global memory.  Bound by the FP32 pipe (some 25 operations a voxel
 // and view).  97 x 128 x 111 voxels, 60 views: one voxel a thread with four
 // scalar gathers 238 us; bricks with the four weights formed and four multiply-adds
-// into the sum 163 us; interpolated as here 157 us, with positions times two, whose
-// edges are the weights without a further step, 147 us, in three view splits 135 us; error
+// into the sum 163 us; interpolated as here 157 us, in three view splits 141 us, with
+// positions times two, whose edges are the weights without a further step, 135 us; error
 // against 64 bits 1.8e-7 -> 5.9e-8.
 // ---------------------------------------------------------------------------
 constexpr int kBrick = 16;
