@@ -334,7 +334,7 @@ typedef struct ct_proj3d_schedule {
  * `stream` with CUDA events (one untimed call, then `reps` timed ones each), and
  * records the fastest forward and, among adjoint timings of 1, 2 and 4 within 3 %
  * of the fastest, the fewest splits, or the planner's count where that is faster by
- * more than 10 %, in a process-wide table (mutex-guarded) keyed by the
+ * more than 20 %, in a process-wide table (mutex-guarded) keyed by the
  * geometry's sizes and kind.  Later calls on that geometry (ct_proj3d_fwd /
  * adj, the fused 3D solver) use the recorded schedule; results change only
  * in summation order.  `vol` and `proj` are scratch arrays of the

@@ -9,24 +9,36 @@ namespace ct {
 // first, far enough apart that the choice does not flip between runs on noise: it sets
 // the summation order, and with it the rounding that a caller sees) the fewest within
 // kTie of the fastest, or 0, the planner's own count, which may lie between two of
-// them, where that is faster by more than kOwn.  (512^2 x 360 views: 43.2 us with 16,
+// them, where that is faster by more than `lead`.  (512^2 x 360 views: 43.2 us with 16,
 // 3.8 % above the planner's 19; 48 x 60 x 70 x 120 views: 32.0 us with 4, 22.8 us with the
-// planner's 7.)
-template <class Counts>
-int tuned_splits(const Counts& measured, float own_us, float& us) {
-  constexpr float kTie = 1.03f, kOwn = 1.10f;
+// planner's 7.)  time(count, us) measures a count, 0 the planner's: a first lead is
+// measured twice more, the fastest of each side counting, as one slow sample of a
+// few microseconds would else make it.
+template <class Counts, class Time>
+ct_status tuned_splits(const Counts& measured, float lead, bool own_fits, Time&& time, int& count, float& us) {
+  constexpr float kTie = 1.03f;
   float fastest = measured.front().second;
   for (const auto& c : measured) fastest = c.second < fastest ? c.second : fastest;
-  int count = 0;
   for (const auto& c : measured)
     if (c.second <= kTie * fastest) {
       count = c.first;
       us = c.second;
       break;
     }
-  if (kOwn * own_us >= us) return count;
-  us = own_us;
-  return 0;
+  if (!own_fits) return CT_OK;
+  float own = 0.0f, again = 0.0f;
+  ct_status st = time(0, own);
+  for (int k = 0; k < 2 && st == CT_OK && lead * own < us; ++k) {
+    st = time(count, again);
+    us = again < us ? again : us;
+    if (st == CT_OK) st = time(0, again);
+    own = again < own ? again : own;
+  }
+  if (st == CT_OK && lead * own < us) {
+    count = 0;
+    us = own;
+  }
+  return st;
 }
 
 // ---- 2D projector (proj2d.cu) ---------------------------------------------

@@ -1302,7 +1302,8 @@ ct_status ct_proj2d_autotune(const ct_geom2d* g, int32_t batch, float* img, floa
   const long ctas = (long)p0.adj_gx * p0.adj_gy * batch;
   const int ns_max = ct::max_splits(g, ctas);
   const size_t n = (size_t)batch * g->rows * g->cols;
-  auto time_adj = [&](const ct::Proj2dPlan& p, float& us) {
+  auto time_adj = [&](int ns, float& us) {
+    const ct::Proj2dPlan p = ct::proj2d_plan_sched(g, batch, ct::Sched2d{0, ns});
     return time_calls(
         [&] {
           ct_status r = ct::proj2d_adj_launch(g, p, sino, img, ws, batch, s, nullptr);
@@ -1318,14 +1319,13 @@ ct_status ct_proj2d_autotune(const ct_geom2d* g, int32_t batch, float* img, floa
     if (p.nsplit == last) continue;  // same split count as the previous candidate
     last = p.nsplit;
     float us = 0.0f;
-    st = time_adj(p, us);
+    st = time_adj(ns, us);
     if (st != CT_OK) return st;
     cand.emplace_back(p.nsplit, us);
   }
-  float own = 0.0f, best_a = 0.0f;
-  st = time_adj(p0, own);
+  float best_a = 0.0f;
+  st = ct::tuned_splits(cand, 1.10f, true, time_adj, best.ns, best_a);
   if (st != CT_OK) return st;
-  best.ns = ct::tuned_splits(cand, own, best_a);
   {
     std::lock_guard<std::mutex> lk(ct::g_sched_mu);
     ct::g_sched[ct::sched_key(g, batch)] = ct::SchedVal{best, best_f, best_a};

@@ -1619,7 +1619,8 @@ ct_status ct_proj3d_autotune(const ct_geom3d* g, float* vol, float* proj, void* 
     // 1, 2 and 4 view splits and the planner's own count, of those what the scratch
     // given holds (a call may always have had less than the counts of now need)
     const size_t scratch = workspace && aligned(workspace, 256) ? workspace_bytes : 0;
-    auto time_adj = [&](const Proj3dPlan& p, float& us) {
+    auto time_adj = [&](int ns, float& us) {
+      const Proj3dPlan p = proj3d_plan_sched(g, Sched3d{0, ns});
       return timed(
           [&] {
             ct_status r = proj3d_adj_launch(g, p, proj, vol, part, s, nullptr);
@@ -1635,14 +1636,14 @@ ct_status ct_proj3d_autotune(const ct_geom3d* g, float* vol, float* proj, void* 
       if (p.nsplit == last || p.adj_bytes > scratch) continue;
       last = p.nsplit;
       float us = 0.0f;
-      st = time_adj(p, us);
+      st = time_adj(ns, us);
       if (st != CT_OK) return st;
       cand.emplace_back(p.nsplit, us);
     }
-    float own = INFINITY;
-    if (p0.adj_bytes <= scratch) st = time_adj(p0, own);
+    // 64 x 96 x 80 x 48 views: 16.7 us with 4 splits, 15.7 us with the planner's 5, on some
+    // boxes 10 % apart in a few samples: a lead of 20 %
+    st = tuned_splits(cand, 1.20f, p0.adj_bytes <= scratch, time_adj, best.ns, best_a);
     if (st != CT_OK) return st;
-    best.ns = tuned_splits(cand, own, best_a);
   }
   {
     std::lock_guard<std::mutex> lk(g_sched3_mu);
