@@ -1142,9 +1142,9 @@ Proj3dPlan proj3d_plan_sched(const ct_geom3d* g, Sched3d sc) {
       if (brick_us(k) < 0.98 * brick_us(nb)) nb = k;
     for (int k = first + 1; k <= std::min(16, V / 4); ++k)
       if (voxel_us(k) < 0.98 * voxel_us(nv)) nv = k;
+    ns = voxel_us(nv) < 1.25 * brick_us(nb) ? nv : nb;  // also the scratch that is asked for, whatever the schedule
     if (sc.ns > 0) nb = nv = std::min(sc.ns, ns_max);
     p.adj_voxels = voxel_us(nv) < 1.25 * brick_us(nb);
-    ns = p.adj_voxels ? nv : nb;
     // forward: views per launch until the tiles of a launch pass kGenScratch (they
     // are read back from L2); the turned volume last, so that a call can go without it
     const GenTiles t = gen_tiles(g->shape, V);

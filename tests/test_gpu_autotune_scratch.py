@@ -33,3 +33,16 @@ def test_tuner_keeps_to_its_scratch(cuda, shape, det, nv, seq):
         assert bool((whole[given:] == 0x5A).all())
     finally:
         lib.ct_proj3d_schedule_clear()
+
+
+def test_query_does_not_depend_on_the_schedule(cuda):
+    """The scratch asked for after tuning is the scratch asked for before."""
+    shape, nv = (64, 64, 64), 20
+    M = X3.matrices_from_euler_angles(shape, (112, 112), "XYZ", np.stack([np.linspace(0.1, 3, nv)] * 3, 1))
+    H = X3(shape, M, (112, 112))
+    before = H.workspace_bytes()
+    try:
+        assert H.autotune()["tuned"]
+        assert X3(shape, M, (112, 112)).workspace_bytes() == before
+    finally:
+        _lib.load().ct_proj3d_schedule_clear()
