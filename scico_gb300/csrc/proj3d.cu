@@ -1640,8 +1640,8 @@ ct_status ct_proj3d_autotune(const ct_geom3d* g, float* vol, float* proj, void* 
       if (st != CT_OK) return st;
       cand.emplace_back(p.nsplit, us);
     }
-    // 64 x 96 x 80 x 48 views: 16.7 us with 4 splits, 15.7 us with the planner's 5, on some
-    // boxes 10 % apart in a few samples: a lead of 20 %
+    // 64 x 96 x 80 x 48 views: 16.7 us with 4 splits, 15.7 us with the planner's 5, in some
+    // runs 10 % apart over a few samples: a lead of 20 %
     st = tuned_splits(cand, 1.20f, p0.adj_bytes <= scratch, time_adj, best.ns, best_a);
     if (st != CT_OK) return st;
   }
